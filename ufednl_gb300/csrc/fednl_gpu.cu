@@ -108,6 +108,15 @@ int ensure_device()
 
 size_t select_smem(int k) { return select_smem_bytes(k); }
 
+// dynamic shared memory of a k-step shuffle (RandK, the FedNL-PP sampler); 0: its scratch is in global
+// memory
+size_t shuffle_smem(int k) { return shuffle_words(k) * 4 <= kShuffleSmemMax ? shuffle_words(k) * 4 : 0; }
+
+cudaError_t raise_shuffle_smem(const void* kernel, int k)
+{
+    return shuffle_smem(k) > 48 * 1024 ? fednl_raise_dyn_smem(kernel, shuffle_smem(k)) : cudaSuccess;
+}
+
 // CTAs of the cooperative Cholesky: enough threads for the first trailing update, at most one
 // resident CTA per SM
 int chol_grid(int d)
@@ -504,8 +513,8 @@ struct fednl_handle_s {
     fednl_problem_desc desc{};
     std::vector<int32_t> ns, soff;
     int d = 0, lda = 0, U = 0, ustr = 0, nc = 0, k = 0, comp = 0, W = 1, SW = 0, S = 0;
-    int binary = 0, maxn = 0, nfpart = 0, nseg = 0, hcap = 0;
-    int pp = 0, tau = 0, pp_smem_perm = 0;   // FedNL-PP: clients per round, sampler in shared memory
+    int binary = 0, maxn = 0, nfpart = 0, nseg = 0;
+    int pp = 0, tau = 0;               // FedNL-PP: clients per round
     bool data_ready = false, shifts_ready = false;
     cudaStream_t stream = nullptr;
     cudaStream_t side = nullptr;       // the round graph's second branch (k_aggregate)
@@ -630,10 +639,42 @@ int launch_round(fednl_handle h, Marks* M = nullptr, bool client_phase_only = fa
     Dev& P = h->dev;
     cudaStream_t st = h->stream;
     int S = h->S;
+    const int na = P.n_act, comp = h->comp;
+    // The master's aggregation needs only the gradients and Lk.  With TopK / TopLEK it runs in the
+    // selection kernel's idle warps; otherwise, in a graph, on a branch beside the shift update, and
+    // the compressor's draws, which read nothing of the round, run there from its start (all kept in
+    // line when the round is profiled kernel by kernel)
+    const bool agg_in_select = !h->pp && (comp == FEDNL_TOPK || comp == FEDNL_TOPLEK);
+    const bool fork = !M && h->side && !h->pp && !agg_in_select;
+    auto draw = [&](cudaStream_t s2) -> int {
+        if (comp == FEDNL_RANDK) {
+            MARK("k_randk");
+            k_randk<<<na, kShuffleThreads, shuffle_smem(h->k), s2>>>(P.rstate, h->U, h->k,
+                                                                     shuffle_smem(h->k) ? nullptr : P.shuf, P.sel,
+                                                                     h->SW, P.cnt, P.act);
+            CKL();
+        } else if (comp == FEDNL_RANDK_PHILOX) {
+            MARK("k_randk_philox");
+            k_randk_philox<<<na * kDrawCtas, 256, 0, s2>>>(P.rstate, h->U, h->k, philox_half_bits(h->U),
+                                                           h->desc.seed_base, P.sel, h->SW, P.cnt, P.act);
+            CKL();
+        } else if (comp == FEDNL_RANDSEQK) {
+            MARK("k_randseqk");
+            k_randseqk<<<na, 256, 0, s2>>>(P.rstate, h->nc, h->U, h->k, P.rseq, P.sel, h->SW, P.cnt, P.act);
+            CKL();
+        }
+        return FEDNL_OK;
+    };
+    if (fork) {
+        CK(cudaEventRecord(h->fork_ev, st));
+        CK(cudaStreamWaitEvent(h->side, h->fork_ev, 0));
+        int rc = draw(h->side);
+        if (rc) return rc;
+    }
     if (h->pp) {
         MARK("k_pp_sample");
-        k_pp_sample<<<1, kPPThreads, h->pp_smem_perm ? (size_t)h->nc * 4 : 0, st>>>(
-            h->nc, h->tau, P.sampler, P.perm, (int*)P.act, P.is_sel, P.needs, h->pp_smem_perm);
+        k_pp_sample<<<1, kPPThreads, shuffle_smem(h->tau), st>>>(
+            h->nc, h->tau, P.sampler, shuffle_smem(h->tau) ? nullptr : P.shuf, (int*)P.act, P.is_sel, P.needs);
         CKL();
     }
     if (h->binary && !P.ref) {       // the client oracle in one launch
@@ -656,7 +697,6 @@ int launch_round(fednl_handle h, Marks* M = nullptr, bool client_phase_only = fa
         else k_grad_dense<<<gg, 128, 0, st>>>(P);
         CKL();
     }
-    const int na = P.n_act;
     if (h->pp) {
         MARK("k_pp_truegrad");
         k_pp_truegrad<<<(h->d + 3) / 4, 128, 0, st>>>(P);
@@ -665,11 +705,6 @@ int launch_round(fednl_handle h, Marks* M = nullptr, bool client_phase_only = fa
         k_pp_norm<<<1, 32, 0, st>>>(P);
         CKL();
     }
-    int comp = h->comp;
-    // The master's aggregation needs only the gradients and Lk.  With TopK / TopLEK it runs in the
-    // selection kernel's idle warps; otherwise, in a graph, on a branch beside the compressor and the
-    // shift update (kept in line when the round is profiled kernel by kernel)
-    const bool agg_in_select = !h->pp && (comp == FEDNL_TOPK || comp == FEDNL_TOPLEK);
     // the master merge runs in the solve's first phase (FP64 order, not FedNL-PP, not when the
     // solve is left to a batched launch)
     const bool apply_in_solve = !h->pp && !P.ref && !client_phase_only;
@@ -689,7 +724,6 @@ int launch_round(fednl_handle h, Marks* M = nullptr, bool client_phase_only = fa
         k_frob_ref<<<na, kFrobRefThreads, (size_t)kFrobRing * h->d * 8, st>>>(P);
         CKL();
     }                             // otherwise the Hessian kernel's last block per client formed F
-    const bool fork = !M && h->side && !h->pp && !agg_in_select;
     if (fork) {
         CK(cudaEventRecord(h->fork_ev, st));
         CK(cudaStreamWaitEvent(h->side, h->fork_ev, 0));
@@ -714,19 +748,11 @@ int launch_round(fednl_handle h, Marks* M = nullptr, bool client_phase_only = fa
             P.diff, h->ustr, h->U, h->k, comp == FEDNL_TOPLEK, delta, P.F, P.sel, h->SW, P.cnt, P.needs, P.pdraw,
             P.minidx, P.status, P.act, P.ref, dr);
         CKL();
-    } else if (comp == FEDNL_RANDK) {
-        MARK("k_randk");
-        k_randk<<<na, 256, 0, st>>>(P.rstate, h->nc, h->U, h->k, P.hmap, h->hcap, P.sel, h->SW, P.cnt, P.act);
-        CKL();
-    } else if (comp == FEDNL_RANDK_PHILOX) {
-        MARK("k_randk_philox");
-        k_randk_philox<<<na, 256, 0, st>>>(P.rstate, h->U, h->k, philox_half_bits(h->U), h->desc.seed_base, P.sel,
-                                           h->SW, P.cnt, P.act);
-        CKL();
-    } else if (comp == FEDNL_RANDSEQK) {
-        MARK("k_randseqk");
-        k_randseqk<<<na, 256, 0, st>>>(P.rstate, h->nc, h->U, h->k, P.rseq, P.sel, h->SW, P.cnt, P.act);
-        CKL();
+    } else if (fork) {
+        CK(cudaStreamWaitEvent(st, h->join_ev, 0));     // the draws and the aggregation
+    } else {
+        int rc = draw(st);
+        if (rc) return rc;
     }
     if (!apply_in_solve) {
         MARK("k_apply");
@@ -749,9 +775,7 @@ int launch_round(fednl_handle h, Marks* M = nullptr, bool client_phase_only = fa
         MARK("end");
         return FEDNL_OK;
     }
-    if (fork) {
-        CK(cudaStreamWaitEvent(st, h->join_ev, 0));
-    } else if (!agg_in_select) {
+    if (!fork && !agg_in_select) {
         MARK("k_aggregate");
         k_aggregate<<<(h->d + kAggThreads - 1) / kAggThreads + 1, kAggThreads, 0, st>>>(P);   // + the block for l
         CKL();
@@ -891,10 +915,6 @@ static int create_impl(const fednl_problem_desc* desc, fednl_handle* out, int64_
     h->nseg = (h->U + 511) / 512;
     h->pp = D.clients_per_round > 0;
     h->tau = h->pp ? D.clients_per_round : h->nc;
-    h->pp_smem_perm = h->pp && (size_t)h->nc * 4 <= 48 * 1024;
-    h->hcap = 1;
-    if (h->comp == FEDNL_RANDK)
-        while (h->hcap < 4 * k) h->hcap <<= 1;
 
     Dev& P = h->dev;
     P.d = h->d;
@@ -908,7 +928,6 @@ static int create_impl(const fednl_problem_desc* desc, fednl_handle* out, int64_
     P.SW = h->SW;
     P.nfpart = h->nfpart;
     P.nseg = h->nseg;
-    P.hcap = h->hcap;
     P.lambda = D.lambda;
     P.alpha = D.alpha;
     P.inv_n = 1.0 / (double)h->nc;
@@ -946,7 +965,12 @@ static int create_impl(const fednl_problem_desc* desc, fednl_handle* out, int64_
     A.want(&P.wstate, h->W);
     A.want(&P.rstate, h->nc);
     A.want(&P.rseq, h->nc);
-    A.want(&P.hmap, (size_t)h->nc * h->hcap);
+    {   // shuffles too large for shared memory work in global memory (sampler and RandK one after another)
+        size_t sw = 0;
+        if (h->comp == FEDNL_RANDK && !shuffle_smem(k)) sw = (size_t)h->nc * shuffle_words(k);
+        if (h->pp && !shuffle_smem(h->tau)) sw = std::max(sw, shuffle_words(h->tau));
+        A.want(&P.shuf, sw);
+    }
     A.want(&P.work, fednl_chol_work_elems(h->d));
     A.want(&P.dx, h->d);
     A.want(&P.ybuf, h->d);
@@ -970,7 +994,6 @@ static int create_impl(const fednl_problem_desc* desc, fednl_handle* out, int64_
     if (h->pp) {
         A.want((int**)&P.act, h->nc);
         A.want(&P.is_sel, h->nc);
-        A.want(&P.perm, h->nc);
         A.want(&P.sampler, 1);
         A.want(&P.hbuf, ncU);
         A.want(&P.dir, (size_t)h->nc * h->d);
@@ -1015,6 +1038,11 @@ static int create_impl(const fednl_problem_desc* desc, fednl_handle* out, int64_
     }
     if (select_smem(h->k) > 48 * 1024 && h->k < h->U)
         fednl_raise_dyn_smem((const void*)k_select, select_smem(h->k));
+    if ((h->comp == FEDNL_RANDK && raise_shuffle_smem((const void*)k_randk, h->k) != cudaSuccess) ||
+        (h->pp && raise_shuffle_smem((const void*)k_pp_sample, h->tau) != cudaSuccess)) {
+        fednl_gpu_destroy(h);
+        return fail(FEDNL_ECUDA, "shared-memory attribute refused");
+    }
     h->chol_grid = chol_grid(h->d);
     if (P.ref) {
         h->ref_grid = ref_grid();
@@ -2415,23 +2443,24 @@ int rand_common(uint32_t* states, int n_gen, int d, int lda, int k, uint32_t* id
     long long U = (long long)d * (d + 1) / 2;
     if (!states || !idx || n_gen < 1 || d < 1 || lda < d || k < 1 || k > U) return fail(FEDNL_EINVAL, "bad argument");
     int SW = (int)((U + 31) / 32);
-    int hcap = 1;
-    while (hcap < 4 * k) hcap <<= 1;
     Scratch s;
     CK(cudaStreamCreateWithFlags(&s.st, cudaStreamNonBlocking));
-    unsigned *dst, *dsel;
+    unsigned *dst, *dsel, *dshuf = nullptr;
     int *dcnt, *drseq;
-    unsigned long long* dmap = nullptr;
     s.a.want(&dst, n_gen);
     s.a.want(&dsel, (size_t)n_gen * SW);
     s.a.want(&dcnt, n_gen);
     s.a.want(&drseq, n_gen);
-    if (!seq) s.a.want(&dmap, (size_t)n_gen * hcap);
+    const size_t smem = seq ? 0 : shuffle_smem(k);
+    if (!seq && !smem) s.a.want(&dshuf, (size_t)n_gen * shuffle_words(k));
     rc = s.a.commit();
     if (rc) return rc;
     CK(cudaMemcpyAsync(dst, states, n_gen * 4, cudaMemcpyHostToDevice, s.st));
     if (seq) k_randseqk<<<n_gen, 256, 0, s.st>>>(dst, n_gen, (int)U, k, drseq, dsel, SW, dcnt, nullptr);
-    else k_randk<<<n_gen, 256, 0, s.st>>>(dst, n_gen, (int)U, k, dmap, hcap, dsel, SW, dcnt, nullptr);
+    else {
+        CK(raise_shuffle_smem((const void*)k_randk, k));
+        k_randk<<<n_gen, kShuffleThreads, smem, s.st>>>(dst, (int)U, k, dshuf, dsel, SW, dcnt, nullptr);
+    }
     CKL();
     std::vector<unsigned> sel((size_t)n_gen * SW);
     std::vector<int> rseq(n_gen);

@@ -63,8 +63,7 @@ struct Dev {
     unsigned* wstate;       // [W] TopLEK generators
     unsigned* rstate;       // [nc] RandK / RandSeqK generators
     int* rseq;              // [nc] RandSeqK window start
-    unsigned long long* hmap; // [nc][hcap] RandK virtual-shuffle map
-    int hcap;
+    unsigned* shuf;         // RandK / FedNL-PP shuffle scratch when it does not fit in shared memory, else null
     double* work;           // [U] Cholesky factor
     double* dx;             // [d]
     double* ybuf;           // [d]
@@ -79,7 +78,6 @@ struct Dev {
     int pp, n_act;          // n_act: clients processed this round (tau, or nc without PP)
     const int* act;         // [n_act] processed clients in ascending order
     int* is_sel;            // [nc]
-    int* perm;              // [nc] the sampler's permutation (when it does not fit in shared memory)
     unsigned* sampler;      // [1] client sampler (RandomGenIntegerLinear)
     double* hbuf;           // [nc][ustr] the round's client Hessians (Lk after the update)
     double* dir;            // [nc][d] localGradient = x Lk + shift x - grad
@@ -1648,90 +1646,116 @@ __global__ void k_toplek_rng(int n_mat, int W, const int* worker_of, unsigned* w
 }
 
 // ---- 5. RandK / RandSeqK ---------------------------------------------------------------------
-// generateRandKItemsInUpperTriangularPart (SpecialMathRoutinesForMatrix.h:95-107): partial
-// Fisher-Yates over a copy of the upper-index list (dopt/dopt/random/include/Shuffle.h:76-93)
-// with the client's RandomGenIntegerLinear; the shuffled array is virtual: only displaced
-// positions are kept, in an open-addressing map in global scratch.  The first k entries, sorted,
-// are the selection -- set as bits of the selection bitmap, whose ascending order is the sort.
-__device__ __forceinline__ unsigned hmap_get(unsigned long long* m, int cap, unsigned key)
+// generateRandKItemsInUpperTriangularPart (SpecialMathRoutinesForMatrix.h:95-107): the first k
+// entries of a partial Fisher-Yates shuffle of the upper-index list (dopt/dopt/random/include/
+// Shuffle.h:76-93) with the client's RandomGenIntegerLinear, sorted -- set as bits of the selection
+// bitmap, whose ascending order is the sort.
+//
+// The generator's state after m steps: x -> A x + C (the step composed with itself by doubling).
+__device__ __forceinline__ void lcg_int_jump(unsigned m, unsigned& A, unsigned& C)
 {
-    unsigned hsh = (key * 2654435761u) & (unsigned)(cap - 1);
-    for (;;) {
-        unsigned long long e = m[hsh];
-        if (e == ~0ull) return key;                    // untouched: identity
-        if ((unsigned)(e >> 32) == key) return (unsigned)e;
-        hsh = (hsh + 1) & (unsigned)(cap - 1);
-    }
-}
-
-__device__ __forceinline__ void hmap_put(unsigned long long* m, int cap, unsigned key, unsigned val)
-{
-    unsigned hsh = (key * 2654435761u) & (unsigned)(cap - 1);
-    for (;;) {
-        unsigned long long e = m[hsh];
-        if (e == ~0ull || (unsigned)(e >> 32) == key) {
-            m[hsh] = ((unsigned long long)key << 32) | val;
-            return;
+    unsigned a = 214013u, c = 2531011u;
+    A = 1u;
+    C = 0u;
+    for (; m; m >>= 1) {
+        if (m & 1u) {
+            A *= a;
+            C = a * C + c;
         }
-        hsh = (hsh + 1) & (unsigned)(cap - 1);
+        c = a * c + c;
+        a *= a;
     }
 }
 
-__global__ void k_randk(unsigned* states, int n_gen, int U, int k, unsigned long long* hmap, int hcap,
-                        unsigned* sel, int SW, int* cnt, const int* act)
+// Buckets of the shuffle's position lists (a power of two, at least k) and its scratch in words:
+// the target r_i and list link of every step, and the lists' heads.
+__host__ __device__ inline int shuffle_bits(int k)
 {
-    int c = act ? act[blockIdx.x] : blockIdx.x;
-    unsigned long long* m = hmap + (size_t)c * hcap;
+    int b = 1;
+    while ((1ll << b) < k) ++b;
+    return b;
+}
+__host__ __device__ inline size_t shuffle_words(int k) { return 2 * (size_t)k + ((size_t)1 << shuffle_bits(k)); }
+
+constexpr int kShuffleThreads = 256;
+// largest shuffle scratch kept in shared memory (k = 16384 takes 192 KB); larger k uses global memory
+constexpr size_t kShuffleSmemMax = 196608;
+
+// The shuffle by one CTA, every step in parallel; calls emit(value) for the k selected values and
+// returns the generator's state after the k draws (valid in every thread).  Step i swaps places i and
+// r_i >= i.  Its draw needs only the i-th generator state, reached by jumping ahead, so all targets
+// are formed at once.  The value found at place p before step i is the one that the last earlier step
+// j with r_j = p put there, i.e. the value of place j before step j, or p itself if there is no such
+// step; the walk p, i -> j, j ends after a few links (k targets spread over n places).  The steps are
+// listed by a hash of their target.  One thread walking the swaps through a hash map in global memory
+// took 1032 us for 142 clients of k = 2408 (430 ns a step, its chain of dependent loads), this form
+// 17 us; FedNL-PP's sampler (128 of 2048 clients) 43 and 8 us.
+template <class Emit>
+__device__ __forceinline__ unsigned shuffle_block(unsigned state, unsigned n, int k, unsigned* w, Emit emit)
+{
+    const int tid = threadIdx.x, nt = blockDim.x, bits = shuffle_bits(k);
+    unsigned* r = w;
+    int* nxt = reinterpret_cast<int*>(w + k);
+    int* head = reinterpret_cast<int*>(w + 2 * (size_t)k);
+    for (int t = tid; t < (1 << bits); t += nt) head[t] = -1;
+    __syncthreads();
+    unsigned A, C, As, Cs;
+    lcg_int_jump((unsigned)tid + 1u, A, C);
+    lcg_int_jump((unsigned)nt, As, Cs);
+    unsigned st = A * state + C;
+    for (int i = tid; i < k; i += nt) {
+        const double u = __dmul_rn((double)st, 1.0 / 4294967295.0);      // lcg_int_unit
+        const unsigned p = (unsigned)i + (unsigned)round_to_nearest(__dmul_rn(u, (double)(n - 1u - (unsigned)i)));
+        r[i] = p;
+        nxt[i] = atomicExch(&head[(p * 2654435761u) >> (32 - bits)], i);
+        st = As * st + Cs;
+    }
+    __syncthreads();
+    for (int i = tid; i < k; i += nt) {
+        unsigned p = r[i];
+        int bound = i;
+        for (;;) {
+            int j = -1;          // the last step before `bound` with target p
+            for (int t = head[(p * 2654435761u) >> (32 - bits)]; t >= 0; t = nxt[t])
+                if (t < bound && t > j && r[t] == p) j = t;
+            if (j < 0) break;
+            p = (unsigned)j;
+            bound = j;
+        }
+        emit(p);
+    }
+    lcg_int_jump((unsigned)k, A, C);
+    return A * state + C;
+}
+
+// scratch: [n_gen clients][shuffle_words(k)] in global memory, or null: dynamic shared memory
+__global__ void __launch_bounds__(kShuffleThreads) k_randk(unsigned* states, int U, int k, unsigned* scratch,
+                                                           unsigned* sel, int SW, int* cnt, const int* act)
+{
+    extern __shared__ unsigned s_shuffle[];
+    const int c = act ? act[blockIdx.x] : blockIdx.x;
     unsigned* sc = sel + (size_t)c * SW;
-    for (int t = threadIdx.x; t < hcap; t += blockDim.x) m[t] = ~0ull;
     for (int w = threadIdx.x; w < SW; w += blockDim.x) sc[w] = 0u;
+    const unsigned state = states[c];
     __syncthreads();
+    const unsigned end = shuffle_block(state, (unsigned)U, k, scratch ? scratch + (size_t)c * shuffle_words(k) : s_shuffle,
+                                       [&](unsigned p) { atomicOr(&sc[p >> 5], 1u << (p & 31)); });
     if (threadIdx.x == 0) {
-        unsigned st = states[c];
-        unsigned long long n_minus_i_minus_one = (unsigned long long)U - 1;
-        for (int i = 0; i < k; ++i, --n_minus_i_minus_one) {
-            double u = lcg_int_unit(st);
-            unsigned long long r_off = round_to_nearest(__dmul_rn(u, (double)n_minus_i_minus_one));
-            if (r_off != 0) {
-                unsigned r = (unsigned)(i + r_off);
-                unsigned vi = hmap_get(m, hcap, (unsigned)i);
-                unsigned vr = hmap_get(m, hcap, r);
-                hmap_put(m, hcap, (unsigned)i, vr);
-                hmap_put(m, hcap, r, vi);
-            }
-        }
-        states[c] = st;
+        states[c] = end;
+        cnt[c] = k;
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < k; i += blockDim.x) {
-        unsigned p = hmap_get(m, hcap, (unsigned)i);
-        atomicOr(&sc[p >> 5], 1u << (p & 31));
-    }
-    if (threadIdx.x == 0) cnt[c] = k;
 }
 
 // Project-defined RandK stream (FEDNL_RANDK_PHILOX): the k positions of draw `draw` of client c are
 // the images of 0..k-1 under a six-round Feistel permutation of [0, 2^(2h)) whose round function is
 // Philox4x32-10 (Salmon et al., SC'11) keyed by (seed, c), walked back into [0, U).  Every position
 // is formed independently, one thread each; the CPU oracle computes the same stream.
-__global__ void k_randk_philox(unsigned* draws, int U, int k, int h, unsigned seed, unsigned* sel, int SW, int* cnt,
-                               const int* act)
+__global__ void __cluster_dims__(kDrawCtas, 1, 1) k_randk_philox(unsigned* draws, int U, int k, int h, unsigned seed,
+                                                                 unsigned* sel, int SW, int* cnt, const int* act)
 {
-    const int c = act ? act[blockIdx.x] : blockIdx.x;
-    unsigned* sc = sel + (size_t)c * SW;
-    for (int w = threadIdx.x; w < SW; w += blockDim.x) sc[w] = 0u;
-    const unsigned draw = draws[c];
-    __syncthreads();
-    for (int i = threadIdx.x; i < k; i += blockDim.x) {
-        uint32_t y = philox_feistel((uint32_t)i, h, seed, (uint32_t)c, draw);
-        while (y >= (uint32_t)U) y = philox_feistel(y, h, seed, (uint32_t)c, draw);   // ends: a cycle holds i < U
-        atomicOr(&sc[y >> 5], 1u << (y & 31));
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        draws[c] = draw + 1;
-        cnt[c] = k;
-    }
+    const int c = act ? act[blockIdx.x / kDrawCtas] : blockIdx.x / kDrawCtas;
+    philox_positions(draws, U, k, h, seed, sel, SW, c);
+    if (blockIdx.x % kDrawCtas == 0 && threadIdx.x == 0) cnt[c] = k;
 }
 
 // generateRandSeqKItemsInUpperTriangularPart (SpecialMathRoutinesForMatrix.h:137-169)
@@ -2867,40 +2891,25 @@ __global__ void k_ls_check(Dev P, double c, double gamma)
 // Client sampler (TrainLoop.h:1150-1157): a fresh 0..n-1 is shuffled for tau steps by the partial
 // Fisher-Yates of Shuffle.h:76-93 with the sampler's RandomGenIntegerLinear; its first tau entries
 // are this round's clients, processed and merged in ascending client order (forcesequpdate).  One
-// CTA; the permutation lives in shared memory when it fits (smem_perm), else in global scratch.
+// CTA, the steps in parallel (shuffle_block; scratch as for k_randk).
 // needs[] is cleared so that the TopLEK draw kernel skips clients that were not sampled.
-constexpr int kPPThreads = 256;
+constexpr int kPPThreads = kShuffleThreads;
 
-__global__ void __launch_bounds__(kPPThreads) k_pp_sample(int n, int tau, unsigned* sampler, int* gperm, int* act,
-                                                          int* is_sel, int* needs, int smem_perm)
+__global__ void __launch_bounds__(kPPThreads) k_pp_sample(int n, int tau, unsigned* sampler, unsigned* scratch, int* act,
+                                                          int* is_sel, int* needs)
 {
-    extern __shared__ int s_perm[];
+    extern __shared__ unsigned s_shuffle[];
     __shared__ int s_wsum[kPPThreads / 32];
-    int* perm = smem_perm ? s_perm : gperm;
     const int tid = threadIdx.x;
+    const unsigned state = *sampler;
     for (int i = tid; i < n; i += blockDim.x) {
-        perm[i] = i;
         is_sel[i] = 0;
         if (needs) needs[i] = 0;
     }
     __syncthreads();
-    if (tid == 0) {
-        unsigned st = *sampler;
-        unsigned long long n_minus_i_minus_one = (unsigned long long)n - 1;
-        for (int i = 0; i < tau; ++i, --n_minus_i_minus_one) {
-            const double u = lcg_int_unit(st);
-            const unsigned long long r_off = round_to_nearest(__dmul_rn(u, (double)n_minus_i_minus_one));
-            if (r_off != 0) {
-                const int r = i + (int)r_off;
-                const int a = perm[i], b = perm[r];
-                perm[i] = b;
-                perm[r] = a;
-            }
-        }
-        *sampler = st;
-    }
-    __syncthreads();
-    for (int t = tid; t < tau; t += blockDim.x) is_sel[perm[t]] = 1;
+    const unsigned end = shuffle_block(state, (unsigned)n, tau, scratch ? scratch : s_shuffle,
+                                       [&](unsigned c) { is_sel[c] = 1; });
+    if (tid == 0) *sampler = end;
     __syncthreads();
     // ascending compaction: thread t owns clients [t * per, (t + 1) * per)
     const int per = (n + blockDim.x - 1) / blockDim.x;

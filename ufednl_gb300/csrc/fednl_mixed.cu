@@ -292,23 +292,34 @@ int mx_launch_round(fednl_mx_handle h, cudaEvent_t* ev = nullptr, bool client_ph
         if (ev) cudaEventRecord(ev[e++], st);
     };
     mark();
+    // The client gradients and the master's aggregation read only the margins' weights and Lk, and
+    // the RandK-Philox draws read nothing of the round: in a graph they run on a branch, the draws
+    // beside the margins, the rest beside the Gram tiles, the selection and the shift update (kept in
+    // line when the round is profiled kernel by kernel)
+    const bool fork = !ev && h->side;
+    const bool randk = h->comp == FEDNL_RANDK_PHILOX;
+    auto draw = [&](cudaStream_t s2) {
+        k_mx_draw<<<h->nc * fednl::kDrawCtas, 256, 0, s2>>>(P, h->k, fednl::philox_half_bits(h->U), h->desc.seed_base);
+    };
+    if (fork && randk) {
+        CKM(cudaEventRecord(h->ev_margin, st));
+        CKM(cudaStreamWaitEvent(h->side, h->ev_margin, 0));
+        draw(h->side);
+        CKM(cudaEventRecord(h->ev_join, h->side));
+    }
     k_mx_split_x<<<(h->d + 255) / 256, 256, 0, st>>>(P);
     mark();
     k_mx_margin<<<dim3((h->L + 63) / 64, h->nc), dim3(64, 4), 0, st>>>(P);
     mark();
-    // The client gradients and the master's aggregation read only the margins' weights and Lk: in
-    // a graph they run on a branch beside the Gram tiles, the selection and the shift update (kept
-    // in line when the round is profiled kernel by kernel)
-    const bool fork = !ev && h->side;
     if (fork) {
         CKM(cudaEventRecord(h->ev_margin, st));
         CKM(cudaStreamWaitEvent(h->side, h->ev_margin, 0));
     }
     k_mx_grad<<<(h->nc * h->d + 7) / 8, 256, 0, fork ? h->side : st>>>(P);
     mark();
-    const bool randk = h->comp == FEDNL_RANDK_PHILOX;
     if (randk) {
-        k_mx_draw<<<h->nc, 256, 0, st>>>(P, h->k, fednl::philox_half_bits(h->U), h->desc.seed_base);
+        if (fork) CKM(cudaStreamWaitEvent(st, h->ev_join, 0));
+        else draw(st);
         mark();
     }
     GramJob J{h->dp, h->nc, h->L, h->dp / kBM, h->tiles, h->ns_dev, nullptr, P.Dw, h->err};

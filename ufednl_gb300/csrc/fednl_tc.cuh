@@ -564,20 +564,9 @@ __global__ void __launch_bounds__(256) k_mx_grad(MxDev P)
 }
 
 // RandK-Philox draw of every client (the FP64 engine's stream)
-__global__ void k_mx_draw(MxDev P, int k, int h, unsigned seed)
+__global__ void __cluster_dims__(fednl::kDrawCtas, 1, 1) k_mx_draw(MxDev P, int k, int h, unsigned seed)
 {
-    const int c = blockIdx.x;
-    unsigned* sc = P.sel + (size_t)c * P.SW;
-    for (int w = threadIdx.x; w < P.SW; w += blockDim.x) sc[w] = 0u;
-    const unsigned draw = P.draws[c];
-    __syncthreads();
-    for (int i = threadIdx.x; i < k; i += blockDim.x) {
-        uint32_t y = fednl::philox_feistel((uint32_t)i, h, seed, (uint32_t)c, draw);
-        while (y >= (uint32_t)P.U) y = fednl::philox_feistel(y, h, seed, (uint32_t)c, draw);
-        atomicOr(&sc[y >> 5], 1u << (y & 31));
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) P.draws[c] = draw + 1;
+    fednl::philox_positions(P.draws, P.U, k, h, seed, P.sel, P.SW, blockIdx.x / fednl::kDrawCtas);
 }
 
 // ---- TopK / TopLEK of the mixed-precision form -----------------------------------------------
