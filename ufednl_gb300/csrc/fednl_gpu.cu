@@ -616,6 +616,12 @@ cudaError_t launch_hess_binary(fednl_handle h, const Dev& Q, int nclients, int m
     return launch_hess_binary_t<false>(Q, h->nseg, h->hess_smem_gl, nclients, mode, st, nt);
 }
 
+cudaError_t launch_hess_dense(const Dev& Q, int nclients, int mode, cudaStream_t st)
+{
+    k_hess_dense<<<dim3((Q.U + kDenseThreads - 1) / kDenseThreads, nclients), kDenseThreads, 0, st>>>(Q, mode);
+    return cudaGetLastError();
+}
+
 cudaError_t raise_hess_smem(fednl_handle h)
 {
     cudaError_t e = cudaSuccess;
@@ -716,8 +722,12 @@ int launch_round(fednl_handle h, Marks* M = nullptr, bool client_phase_only = fa
     if (h->binary) {
         CK(launch_hess_binary(h, P, na, hmode, st, h->hess_kind, h->hess_nt));
     } else {
-        k_hess_dense<<<dim3(h->nfpart, na), kHessThreads, 0, st>>>(P, hmode);
-        CKL();
+        CK(launch_hess_dense(P, na, hmode, st));
+        if (hmode != 3 && !P.ref) {
+            MARK("k_diff_norms");
+            k_diff_norms<<<dim3(h->nfpart, na), kHessThreads, 0, st>>>(P);
+            CKL();
+        }
     }
     if (P.ref) {
         MARK("k_frob_ref");
@@ -1669,8 +1679,7 @@ int fednl_gpu_init_shifts(fednl_handle h, const double* x0)
     if (h->binary) {
         CK(launch_hess_binary(h, Pall, h->nc, 1, st, h->hess_kind, h->hess_nt));
     } else {
-        k_hess_dense<<<dim3(h->nfpart, h->nc), kHessThreads, 0, st>>>(Pall, 1);
-        CKL();
+        CK(launch_hess_dense(Pall, h->nc, 1, st));
     }
     k_h_init<<<(h->U + 255) / 256, 256, 0, st>>>(P);
     CKL();

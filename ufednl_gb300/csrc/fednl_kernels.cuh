@@ -674,48 +674,103 @@ __global__ void __launch_bounds__(NT) k_hess_binary(Dev P, int mode)
     if ((mode == 0 || mode == 2) && !P.ref) client_fsum_last_block(P, c);
 }
 
-// dense FP64: the reference's per-entry order u_i (D_s u_j), samples in order
-__global__ void __launch_bounds__(kHessThreads) k_hess_dense(Dev P, int mode)
+// Dense features: the reference's per-entry order, sum over the samples of u_i (D_s u_j), u = b_s a_s.
+// The label drops out of a term exactly ((-a)(D (-b)) = a (D b), rounding being symmetric), so a term is
+// one product and one add, the least this order allows: the kernel is bound by the FP64 pipe, and
+// everything else is kept off it.  A CTA owns 128 consecutive upper positions of one client, one a
+// thread; these lie in few columns (at most 16, one or two at d of some hundreds), whose D_s a_sj the
+// CTA forms once per sample, kDenseT samples at a time and one batch ahead in shared memory.  Each
+// thread loads its a_si from global memory (consecutive lanes, consecutive i) four samples ahead of
+// their use; the clients' rows stay in L2.  d = 512, 24 clients of 300-900 samples: 29.9 ms with two
+// row loads, a column product and two label products per term, 7.5 ms now (7.2 ms is the pipe's time
+// for two operations a term).  Four positions a thread took the same time there and 876 against 653 us
+// at d = 256, 10 clients of 500 (few CTAs, a last wave of a third).
+// mode as for k_hess_binary; the norms of modes 0 and 2 are k_diff_norms's.
+constexpr int kDenseThreads = 128;
+constexpr int kDenseT = 16;
+constexpr int kDenseCols = 16;      // columns that 128 consecutive upper positions can touch
+
+__global__ void __launch_bounds__(kDenseThreads) k_hess_dense(Dev P, int mode)
+{
+    __shared__ double s_w[2][kDenseT][kDenseCols];
+    const int c = P.act ? P.act[blockIdx.y] : blockIdx.y;
+    const int n = P.ns[c], off = P.soff[c], d = P.d;
+    const int tid = threadIdx.x, p0 = blockIdx.x * kDenseThreads, p = p0 + tid;
+    const double* A = P.A + (size_t)off * d;
+    const double* Dv = P.Dv + off;
+    int it, j_lo, j_hi, i, j;
+    upper_ij(p0, it, j_lo);
+    upper_ij(min(p0 + kDenseThreads, P.U) - 1, it, j_hi);
+    upper_ij(min(p, P.U - 1), i, j);
+    const int ncols = j_hi - j_lo + 1, jc = j - j_lo;
+    const bool live = p0 + (tid & ~31) < P.U;              // the warp has positions
+    auto form_w = [&](int s0, int buf) {
+        for (int t = tid; t < kDenseT * ncols; t += kDenseThreads) {
+            const int r = t / ncols, col = t - r * ncols;
+            if (s0 + r < n) s_w[buf][r][col] = __dmul_rn(Dv[s0 + r], A[(size_t)(s0 + r) * d + j_lo + col]);
+        }
+    };
+    double h = 0.0, a[4], an[4];
+    auto load4 = [&](double (&v)[4], int s) {     // samples s .. s+3 (past the last one: the last again)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = __ldg(A + (size_t)min(s + u, n - 1) * d + i);
+    };
+    form_w(0, 0);
+    load4(a, 0);
+    __syncthreads();
+    for (int s0 = 0, buf = 0; s0 < n; s0 += kDenseT, buf ^= 1) {
+        if (s0 + kDenseT < n) form_w(s0 + kDenseT, buf ^ 1);
+        const int cnt = min(kDenseT, n - s0);
+        if (live)
+            for (int r0 = 0; r0 < cnt; r0 += 4) {
+                load4(an, s0 + r0 + 4);
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (r0 + u < cnt) h = __dadd_rn(h, __dmul_rn(a[u], s_w[buf][r0 + u][jc]));
+#pragma unroll
+                for (int u = 0; u < 4; ++u) a[u] = an[u];
+            }
+        __syncthreads();
+    }
+    if (p >= P.U) return;
+    const size_t q = (size_t)c * P.ustr + p;
+    if (i == j) h = __dadd_rn(h, P.lambda);
+    if (mode == 1) {
+        P.shift[q] = h;
+    } else {
+        if (mode == 2) P.hbuf[q] = h;
+        P.diff[q] = __dsub_rn(h, P.shift[q]);
+    }
+}
+
+// ||diff||_F^2 and Lk of the processed clients from their differences, in k_hess_binary's segments
+__global__ void __launch_bounds__(kHessThreads) k_diff_norms(Dev P)
 {
     const int c = P.act ? P.act[blockIdx.y] : blockIdx.y;
-    const int n = P.ns[c], off = P.soff[c];
     const size_t base = (size_t)c * P.ustr;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int seg = blockIdx.x * (kHessThreads / 32) + warp;
     const int p_seg = seg * 512;
-    double fa = 0.0, fb2 = 0.0;
-    for (int q = 0; q < 16; ++q) {
-        const int p = p_seg + 32 * q + lane;
-        if (p >= P.U) break;
-        int i, j;
-        upper_ij(p, i, j);
-        double h = 0.0;
-        for (int s = 0; s < n; ++s) {
-            const double* a = P.A + (size_t)(off + s) * P.d;
-            const bool pos = P.lab[off + s] == 1.0;
-            const double ui = pos ? a[i] : __dmul_rn(a[i], -1.0);
-            const double uj = pos ? a[j] : __dmul_rn(a[j], -1.0);
-            h = __dadd_rn(h, __dmul_rn(ui, __dmul_rn(P.Dv[off + s], uj)));
+    if (p_seg < P.U) {
+        double v[16], fa = 0.0, fb2 = 0.0;
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+            const int p = p_seg + 32 * q + lane;
+            v[q] = p < P.U ? P.diff[base + p] : 0.0;
         }
-        if (i == j) h = __dadd_rn(h, P.lambda);
-        if (mode == 1) {
-            P.shift[base + p] = h;
-        } else {
-            if (mode == 2) P.hbuf[base + p] = h;
-            const double df = __dsub_rn(h, P.shift[base + p]);
-            P.diff[base + p] = df;
-            if (mode != 3) {
-                const double r = fma(df, df, i == j ? fa : fb2);     // one FP64 instruction per warp
-                if (i == j) fa = r;
-                else fb2 = r;
-            }
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+            const int p = p_seg + 32 * q + lane;
+            if (p >= P.U) break;
+            const bool dg = upper_is_diag(p);
+            const double r = fma(v[q], v[q], dg ? fa : fb2);     // one FP64 instruction per warp
+            if (dg) fa = r;
+            else fb2 = r;
         }
-    }
-    if ((mode == 0 || mode == 2) && p_seg < P.U) {
         const double cs = chunk_tree(segment_value(fa, fb2));
         if (lane == 0) P.Fpart[(size_t)c * P.nseg + seg] = cs;
     }
-    if ((mode == 0 || mode == 2) && !P.ref) client_fsum_last_block(P, c);
+    client_fsum_last_block(P, c);
 }
 
 // master H = mean_i shift_i after the initial shifts (TrainLoop.h:639-643, :732-735)
