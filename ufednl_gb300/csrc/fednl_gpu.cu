@@ -755,7 +755,7 @@ int launch_round(fednl_handle h, Marks* M = nullptr, bool client_phase_only = fa
             dr.lk = P.lk;
         }
         k_select<<<na, kSelThreads, h->k < h->U ? select_smem(h->k) : 0, st>>>(
-            P.diff, h->ustr, h->U, h->k, comp == FEDNL_TOPLEK, delta, P.F, P.sel, h->SW, P.cnt, P.needs, P.pdraw,
+            P.diff, P.gmax, P.gstr, h->ustr, h->U, h->k, comp == FEDNL_TOPLEK, delta, P.F, P.sel, h->SW, P.cnt, P.needs, P.pdraw,
             P.minidx, P.status, P.act, P.ref, dr);
         CKL();
     } else if (fork) {
@@ -968,6 +968,9 @@ static int create_impl(const fednl_problem_desc* desc, fednl_handle* out, int64_
     A.want(&h->drawctr, 1);
     A.want(&P.lk, h->nc);
     A.want(&P.sel, (size_t)h->nc * h->SW);
+    P.gstr = (h->SW + 3) / 4 * 4;
+    const bool topk = (h->comp == FEDNL_TOPK || h->comp == FEDNL_TOPLEK) && h->k < h->U;
+    A.want(&P.gmax, topk ? (size_t)h->nc * P.gstr : 0);
     A.want(&P.cnt, h->nc);
     A.want(&P.needs, h->nc);
     A.want(&P.pdraw, h->nc);
@@ -2378,8 +2381,9 @@ int select_common(const double* mats, int n_mat, int d, int lda, int k, bool lek
     Scratch s;
     CK(cudaStreamCreateWithFlags(&s.st, cudaStreamNonBlocking));
     double *dfull, *dpack, *dF, *dp, *dcs;
-    unsigned *dsel, *dws = nullptr;
+    unsigned *dsel, *dws = nullptr, *dgm;
     int *dcnt, *dneeds, *dmi, *dwo = nullptr, *derr;
+    const int gstr = (SW + 3) / 4 * 4;
     size_t full = (size_t)d * lda;
     s.a.want(&dfull, (size_t)n_mat * full);
     s.a.want(&dpack, (size_t)n_mat * ustr);
@@ -2387,6 +2391,7 @@ int select_common(const double* mats, int n_mat, int d, int lda, int k, bool lek
     s.a.want(&dp, n_mat);
     s.a.want(&dcs, (size_t)n_mat * ((full + 31) / 32));
     s.a.want(&dsel, (size_t)n_mat * SW);
+    s.a.want(&dgm, (size_t)n_mat * gstr);
     s.a.want(&dcnt, n_mat);
     s.a.want(&dneeds, n_mat);
     s.a.want(&dmi, n_mat);
@@ -2400,14 +2405,14 @@ int select_common(const double* mats, int n_mat, int d, int lda, int k, bool lek
     CK(cudaMemcpyAsync(dfull, mats, (size_t)n_mat * full * 8, cudaMemcpyHostToDevice, s.st));
     CK(cudaMemsetAsync(derr, 0, 4, s.st));
     k_pack_upper<<<dim3((unsigned)std::min<long long>(1024, (U + 255) / 256), n_mat), 256, 0, s.st>>>(dfull, d, lda, (int)U,
-                                                                                                     (int)ustr, dpack);
+                                                                                                     (int)ustr, dpack, dgm, gstr);
     CKL();
     k_l2sq_full<<<n_mat, 256, 0, s.st>>>(dfull, (long long)full, dcs, dF);
     CKL();
     if (select_smem(k) > 48 * 1024 && k < U)
         CK(fednl_raise_dyn_smem((const void*)k_select, select_smem(k)));
     double delta = (double)k * (1.0 / (double)U);
-    k_select<<<n_mat, kSelThreads, k < U ? select_smem(k) : 0, s.st>>>(dpack, (int)ustr, (int)U, k, lek ? 1 : 0, delta,
+    k_select<<<n_mat, kSelThreads, k < U ? select_smem(k) : 0, s.st>>>(dpack, dgm, gstr, (int)ustr, (int)U, k, lek ? 1 : 0, delta,
                                                                       dF, dsel, SW, dcnt, dneeds, dp, dmi, derr, nullptr, 0,
                                                                       SelectDraws{nullptr, 0, 0, nullptr, MasterAgg{}});
     CKL();
@@ -2747,7 +2752,7 @@ int fednl_gpu_optionb_solve(const double* H, int32_t d, int32_t lda, double l, c
     CK(cudaMemcpyAsync(dg, g, d * 8, cudaMemcpyHostToDevice, s.st));
     CK(cudaMemsetAsync(P.status, 0, 4, s.st));
     k_pack_upper<<<dim3((unsigned)std::min<long long>(1024, (U + 255) / 256), 1), 256, 0, s.st>>>(dfull, d, lda, (int)U,
-                                                                                                (int)U, dpack);
+                                                                                                (int)U, dpack, nullptr, 0);
     CKL();
     CK(launch_chol(P, chol_grid(d), s.st, dpack, 0, nullptr, l, dg, P.dx, nullptr, 0));
     int status = 0;
@@ -2807,7 +2812,7 @@ int fednl_gpu_optionb_solve32(const double* H, int32_t d, int32_t lda, double l,
     CK(cudaMemcpyAsync(dg, g, d * 8, cudaMemcpyHostToDevice, s.st));
     CK(cudaMemcpyAsync(dl, &l, 8, cudaMemcpyHostToDevice, s.st));
     k_pack_upper<<<dim3((unsigned)std::min<long long>(1024, (U + 255) / 256), 1), 256, 0, s.st>>>(dfull, d, lda, (int)U,
-                                                                                                (int)U, dpack);
+                                                                                                (int)U, dpack, nullptr, 0);
     k_split_pairs<<<(unsigned)((U + 255) / 256), 256, 0, s.st>>>(dpack, d, phh, phl, prh, prl);
     CKL();
     E.hh = phh;

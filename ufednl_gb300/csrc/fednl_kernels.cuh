@@ -56,6 +56,8 @@ struct Dev {
     double* F;              // [nc] ||diff||_F^2
     double* lk;             // [nc]
     unsigned* sel;          // [nc][SW] selection bitmaps over p
+    unsigned* gmax;         // [nc][gstr] bounds of |diff| over 32 positions (key_bound), TopK / TopLEK, else null
+    int gstr;
     int* cnt;               // [nc]
     int* needs;             // [nc] TopLEK: rounding draw needed
     double* pdraw;          // [nc]
@@ -114,6 +116,22 @@ __device__ __forceinline__ void upper_ij(int p, int& i, int& j)
     while ((long long)(jj + 1) * (jj + 2) / 2 <= p) ++jj;
     j = jj;
     i = p - (int)((long long)jj * (jj + 1) / 2);
+}
+
+// A 32-bit bound of |v|: its upper word, one more if any lower bit is set.  |v| > |r| implies
+// key_bound(v) > the upper word of |r|, so the selection's scan skips 32 entries at a time on it.
+__device__ __forceinline__ unsigned key_bound(double v)
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+    return (unsigned)(b >> 32) + ((unsigned)b != 0u ? 1u : 0u);
+}
+
+// word <- the bound of a warp's row of 32 upper positions, of which `left` lanes are inside U (the others
+// are not here)
+__device__ __forceinline__ void row_bound(unsigned* word, int left, int lane, double df)
+{
+    const unsigned m = __reduce_max_sync(left >= 32 ? 0xffffffffu : (1u << left) - 1u, key_bound(df));
+    if (lane == 0) *word = m;
 }
 
 __device__ __forceinline__ bool upper_is_diag(int p)
@@ -660,6 +678,7 @@ __global__ void __launch_bounds__(NT) k_hess_binary(Dev P, int mode)
             if (mode == 2) P.hbuf[base + p] = h;
             const double df = __dsub_rn(h, P.shift[base + p]);
             P.diff[base + p] = df;
+            if (P.gmax) row_bound(P.gmax + (size_t)c * P.gstr + (p >> 5), P.U - (p - lane), lane, df);
             if (mode != 3) {
                 const double r = fma(df, df, i == j ? fa : fb2);     // one FP64 instruction per warp
                 if (i == j) fa = r;
@@ -739,7 +758,9 @@ __global__ void __launch_bounds__(kDenseThreads) k_hess_dense(Dev P, int mode)
         P.shift[q] = h;
     } else {
         if (mode == 2) P.hbuf[q] = h;
-        P.diff[q] = __dsub_rn(h, P.shift[q]);
+        const double df = __dsub_rn(h, P.shift[q]);
+        P.diff[q] = df;
+        if (P.gmax) row_bound(P.gmax + (size_t)c * P.gstr + (p >> 5), P.U - (p & ~31), tid & 31, df);
     }
 }
 
@@ -795,16 +816,22 @@ __global__ void k_h_init(Dev P)
 // * buildMinHeap runs level by level in parallel: sifts of nodes on one level touch disjoint
 //   subtrees, so the result equals the reference's descending-index order.
 // * The scanned entries stream into shared memory by bulk asynchronous copies (cp.async.bulk with
-//   an mbarrier per buffer, double-buffered); one warp tests them 256 at a time, each lane its
-//   first entry above the root, one warp-wide minimum per replacement.  The heap's top two levels
-//   live in registers during the scan, the same in every lane, and the warp replaces the root in
-//   step: most root replacements stop within the top three levels (the carried comparison value
-//   ends the walk early), so a replacement is a few compares and at most one shared-memory load.
+//   an mbarrier per buffer, double-buffered), with a 32-bit bound per 32 entries that the kernel which
+//   wrote the differences left (row_bound): one warp skips the rows whose bound is not above the root.
+//   The heap's top lives in registers during the scan, the same in every lane, and the warp replaces the
+//   root in step: most root replacements stop within the top three levels (the carried comparison value
+//   ends the walk early).
 // * TopLEK extracts in chunks of 32 recording the order in place (extracFromMinHeap leaves the
 //   extracted element at the array's end, MinHeap.h:133-140) and stops after the chunk that opens
-//   the rounding window; the top two heap levels live in registers during the extraction.  The
-//   window numerator uses the fixed parallel order of the CPU oracle (chunked tree for the heap's
-//   terms, chunked doubling scan plus in-order carries for the extracted terms).
+//   the rounding window, whose numerators a second warp forms a chunk behind.  The window numerator uses
+//   the fixed parallel order of the CPU oracle (chunked tree for the heap's terms, chunked doubling scan
+//   plus in-order carries for the extracted terms), or the reference's, one term at a time.
+// Bound by latency: a chain of dependent comparisons per replacement and per extraction, one CTA per
+// client, the launch as long as its slowest client.  Cycles of that client (w8a-like, d = 301, k = 2408):
+// first rounds 855 k, of which extraction 510 k, to 440 k (2387 extractions at 208 -> 100 cycles, windows
+// beside them); settled rounds 580 k to 377 k (713 replacements at 650 -> 440 cycles with their
+// searches, 1387 rows without an entry above the root at 37 -> 2).  k_select 376 -> 207 us; a9a-like
+// (d = 124, k = 992) 139 -> 95 us, dense d = 512, k = 4096 239 -> 137 us, reference order at w8a 696 -> 299.
 struct HeapS {
     unsigned long long* key;   // bits of |value|
     unsigned* hid;             // packed upper position p
@@ -877,7 +904,7 @@ __device__ __forceinline__ void heap_sift(HeapS& h, int i, int heap_size)
     heap_descend(h, i, heap_size, kv, kv, h.hid[i]);
 }
 
-constexpr int kSelThreads = 128;
+constexpr int kSelThreads = 256;
 constexpr int kSelStage = 2048;                    // doubles per staging buffer (16 KB)
 constexpr long long kSelWaitCycles = 2000000000ll; // bounded mbarrier wait (~1 s)
 
@@ -915,47 +942,155 @@ __device__ __forceinline__ unsigned long long heap_replace_root(HeapS& h, int k,
     return m;
 }
 
-// heap_replace_root with the heap's levels 0 and 1 in registers (K0..K4, I0..I4; k >= 21, so levels
-// 0-2 are complete): the same comparisons and moves, level 2 and below in shared memory
-__device__ __forceinline__ unsigned long long heap_replace_root_r(HeapS& h, int k, unsigned long long cand, unsigned p,
-                                                                  unsigned long long& K0, unsigned long long& K1,
-                                                                  unsigned long long& K2, unsigned long long& K3,
-                                                                  unsigned long long& K4, unsigned& I0, unsigned& I1,
-                                                                  unsigned& I2, unsigned& I3, unsigned& I4)
+// The heap's top in registers (at least 21 entries, so levels 0-2 are complete): the root's key and id
+// (K0, I0) and the four level-1 keys sorted, s1 <= .. <= s4, equal keys by node (t: node 1..4, and bit 3
+// set if the key is above the least of the node's children).  An entry that enters at the root is
+// compared with all of them at once: against s1 it decides the new root, against s2..s4 the place of
+// the value that replaces s1 (a tree over unsorted keys makes three dependent comparisons, and the
+// chain of comparisons is what a step costs).  The level-1 ids and the least child keys (mn, by node)
+// and positions stay in shared memory, those of the node of s1 loaded ahead (i1, m1, g1).
+struct HeapMins {
+    unsigned long long mn[5];   // least child's key, by node
+    int gp[5];                  // its position
+};
+
+struct HeapTop {
+    unsigned long long K0, s1, s2, s3, s4, m1;
+    unsigned I0, i1, t1, t2, t3, t4;
+    int g1;
+    HeapMins* mins;             // shared
+
+    // the least child of level-1 node s (the leftmost one): its key
+    __device__ __forceinline__ unsigned long long children(const HeapS& h, unsigned s)
+    {
+        const int f = 4 * (int)s + 1;
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(h.key + f);
+        const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(h.key + f + 2);
+        const bool s01 = a.y < a.x, s23 = b.y < b.x;
+        const unsigned long long n01 = s01 ? a.y : a.x, n23 = s23 ? b.y : b.x;
+        const bool sr = n23 < n01;
+        const unsigned long long m = sr ? n23 : n01;
+        mins->gp[s] = f + (sr ? (s23 ? 3 : 2) : (s01 ? 1 : 0));
+        mins->mn[s] = m;
+        return m;
+    }
+    __device__ __forceinline__ void ahead(const HeapS& h)
+    {
+        i1 = h.hid[t1 & 7];
+        m1 = mins->mn[t1 & 7];
+        g1 = mins->gp[t1 & 7];
+    }
+    __device__ __forceinline__ void load(const HeapS& h, HeapMins* m)
+    {
+        mins = m;
+        K0 = h.key[0];
+        I0 = h.hid[0];
+        s1 = h.key[1]; s2 = h.key[2]; s3 = h.key[3]; s4 = h.key[4];
+        t1 = 1u | (s1 > children(h, 1u) ? 8u : 0u);
+        t2 = 2u | (s2 > children(h, 2u) ? 8u : 0u);
+        t3 = 3u | (s3 > children(h, 3u) ? 8u : 0u);
+        t4 = 4u | (s4 > children(h, 4u) ? 8u : 0u);
+        auto order = [](unsigned long long& a, unsigned& ta, unsigned long long& b, unsigned& tb) {
+            if (b < a || (b == a && (tb & 7u) < (ta & 7u))) {
+                const unsigned long long x = a;
+                a = b;
+                b = x;
+                const unsigned y = ta;
+                ta = tb;
+                tb = y;
+            }
+        };
+        order(s1, t1, s2, t2);
+        order(s3, t3, s4, t4);
+        order(s1, t1, s3, t3);
+        order(s2, t2, s4, t4);
+        order(s2, t2, s3, t3);
+        ahead(h);
+    }
+    __device__ __forceinline__ void store(HeapS& h) const
+    {
+        h.key[0] = K0;
+        h.hid[0] = I0;
+        h.key[t1 & 7] = s1; h.key[t2 & 7] = s2; h.key[t3 & 7] = s3; h.key[t4 & 7] = s4;
+    }
+    // The entry (ck, ci) enters at the root of a heap of n >= 21 entries with its own key as the
+    // comparison value (MinHeap.h:78-85 and :125-141: heap_descend(h, 0, n, ck, ck, ci)), in two steps:
+    // the new root, true if the entry goes below it; then its place below.  below() returns true if
+    // entries in shared memory moved.
+    __device__ __forceinline__ bool root(unsigned long long ck, unsigned ci)
+    {
+        const bool gt = ck > s1;
+        K0 = gt ? s1 : ck;
+        I0 = gt ? i1 : ci;
+        return gt;
+    }
+    __device__ __forceinline__ bool below(HeapS& h, int n, unsigned long long ck, unsigned ci)
+    {
+        const unsigned nd = t1 & 7u;
+        const bool deeper = (t1 & 8u) != 0u;
+        unsigned long long x = ck, xm = m1;
+        unsigned xi = ci;
+        if (deeper) {       // level 2: the least child of the node is below the value that moved up
+            x = m1;
+            xi = h.hid[g1];
+            heap_descend(h, g1, n, m1, ck, ci);
+            xm = children(h, nd);
+        }
+        h.hid[nd] = xi;
+        const unsigned tx = nd | (x > xm ? 8u : 0u);
+        // x after s_k: above it, or equal with the later node
+        const bool a2 = x >= s2 + ((t2 & 7u) > nd ? 1u : 0u);
+        const bool a3 = x >= s3 + ((t3 & 7u) > nd ? 1u : 0u);
+        const bool a4 = x >= s4 + ((t4 & 7u) > nd ? 1u : 0u);
+        s1 = a2 ? s2 : x;
+        t1 = a2 ? t2 : tx;
+        s2 = a2 ? (a3 ? s3 : x) : s2;
+        t2 = a2 ? (a3 ? t3 : tx) : t2;
+        s3 = a3 ? (a4 ? s4 : x) : s3;
+        t3 = a3 ? (a4 ? t4 : tx) : t3;
+        s4 = a4 ? x : s4;
+        t4 = a4 ? tx : t4;
+        ahead(h);
+        return deeper;
+    }
+};
+
+// Extractions (extracFromMinHeap, MinHeap.h:125-141) that bring the heap from `size` to `target` entries,
+// by one thread: the last entry leaves for the root and the root for the last place.  While the heap has
+// more than 21 entries its top is in `top` (live), and the next last entry is loaded a step ahead; the
+// answer is whether it still is.  100 cycles a step; 208 with a tree of comparisons over unsorted keys
+// (and the windows between the chunks), 290 with a warp-wide minimum over lanes holding the nodes (its
+// votes, and ties that need the keys' lower words), 165 on 32-bit ranks after 116 k cycles of sorting.
+__device__ __forceinline__ bool extract_chunk(HeapS& h, HeapTop& top, bool live, int size, int target)
 {
-    const bool r12 = K2 < K1, r34 = K4 < K3;
-    const unsigned long long m12 = r12 ? K2 : K1, m34 = r34 ? K4 : K3;
-    const bool r = m34 < m12;
-    const unsigned long long m = r ? m34 : m12;
-    if (!(cand > m)) {
-        K0 = cand;
-        I0 = p;
-        return cand;
+    if (live) {
+        const int stop = max(target, 21);
+        if (size > stop) {
+            unsigned long long LK = h.key[size - 1];
+            unsigned LI = h.hid[size - 1];
+            for (; size > stop; --size) {
+                const int n = size - 1;                  // heap size after the swap
+                const unsigned long long nk = h.key[n - 1];
+                const unsigned ni = h.hid[n - 1];
+                h.key[n] = top.K0;
+                h.hid[n] = top.I0;
+                const bool moved = top.root(LK, LI) && top.below(h, n, LK, LI);
+                LK = moved ? h.key[n - 1] : nk;
+                LI = moved ? h.hid[n - 1] : ni;
+            }
+        }
+        if (size > 21) return true;
+        top.store(h);
     }
-    const int lo = r ? (r34 ? 4 : 3) : (r12 ? 2 : 1);
-    K0 = m;
-    I0 = lo == 1 ? I1 : lo == 2 ? I2 : lo == 3 ? I3 : I4;
-    // the children of lo (level 2) against the value that moved up
-    const int f = 4 * lo + 1;
-    const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(h.key + f);
-    const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(h.key + f + 2);
-    const bool s01 = a.y < a.x, s23 = b.y < b.x;
-    const unsigned long long n01 = s01 ? a.y : a.x, n23 = s23 ? b.y : b.x;
-    const bool sr = n23 < n01;
-    const unsigned long long m2 = sr ? n23 : n01;
-    unsigned long long nk = cand;
-    unsigned ni = p;
-    if (m > m2) {
-        const int gp = f + (sr ? (s23 ? 3 : 2) : (s01 ? 1 : 0));
-        nk = m2;
-        ni = h.hid[gp];
-        heap_descend(h, gp, k, m2, cand, p);
+    for (; size > target; --size) {
+        const int n = size - 1;
+        const unsigned long long LK = h.key[n];
+        const unsigned LI = h.hid[n];
+        h.key[n] = h.key[0];
+        h.hid[n] = h.hid[0];
+        heap_descend(h, 0, n, LK, LK, LI);
     }
-    if (lo == 1) { K1 = nk; I1 = ni; }
-    else if (lo == 2) { K2 = nk; I2 = ni; }
-    else if (lo == 3) { K3 = nk; I3 = ni; }
-    else { K4 = nk; I4 = ni; }
-    return m;
+    return false;
 }
 
 // dynamic shared memory of k_select: two staging buffers, key[k] (three slots ahead and 32 bytes
@@ -977,15 +1112,6 @@ __device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)
 __device__ __forceinline__ void mbar_init(unsigned long long* bar)
 {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bar)));
-}
-
-__device__ __forceinline__ void tma_load_1d(void* dst, const void* src, unsigned bytes, unsigned long long* bar)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_addr(dst)),
-                 "l"(src), "r"(bytes), "r"(smem_addr(bar))
-                 : "memory");
 }
 
 // bounded wait for the given phase parity; false if it did not complete in time
@@ -1128,6 +1254,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_hess_hits(Dev P, int mode, in
                     if (mode == 2) P.hbuf[base + p] = h;
                     const double df = __dsub_rn(h, s_sh[t]);
                     P.diff[base + p] = df;
+                    if (P.gmax) row_bound(P.gmax + (size_t)c * P.gstr + seg * 16 + q, cnt - 32 * q, lane, df);
                     if (mode != 3) {
                         const double r = fma(df, df, diag ? fa : fb2);     // one FP64 instruction per warp
                         if (diag) fa = r;
@@ -1252,15 +1379,18 @@ struct SelectDraws {
 };
 
 // The difference's squared Frobenius norm in the fixed segment order (k_hess_binary's, the CPU
-// oracle's orc_frob_sym) and Lk = sqrt of it (TopK.h:74-78), formed by warps 1-3 of the selection
-// kernel while warp 0 walks the heap: segment seg holds 512 upper positions, lane l squares
-// positions 32 q + l into fused multiply-adds (diagonal and off-diagonal apart, loaded ahead) and
-// gives a + 2 b to the segment's halving tree; warp 1 then adds the segment sums in order.
+// oracle's orc_frob_sym) and Lk = sqrt of it (TopK.h:74-78), formed by six of the selection kernel's
+// warps, two on each SM sub-partition that the heap's warp 0 is not on, while that walks the heap:
+// segment seg holds 512 upper positions, lane l squares positions 32 q + l into fused multiply-adds
+// (diagonal and off-diagonal apart, loaded ahead) and gives a + 2 b to the segment's halving tree; warp 1
+// then adds the segment sums in order.
+constexpr int kNormWarps = 6;
+
 __device__ __forceinline__ void select_norms(const SelectDraws& dr, const double* __restrict__ v, int U, int c,
                                           double* F, int warp, int lane)
 {
     double* fp = dr.fpart + (size_t)c * dr.nseg;
-    for (int seg = warp - 1; seg < dr.nseg; seg += 3) {
+    for (int seg = warp < 4 ? warp - 1 : warp - 2; seg < dr.nseg; seg += kNormWarps) {
         const int p_seg = seg * 512;
         double x[16];
 #pragma unroll
@@ -1288,12 +1418,13 @@ __device__ __forceinline__ void select_norms(const SelectDraws& dr, const double
         const double cs = chunk_tree(segment_value(fa, fb2));
         if (lane == 0) fp[seg] = cs;
     }
-    asm volatile("bar.sync 1, 96;" ::: "memory");
+    asm volatile("bar.sync 1, 192;" ::: "memory");
     if (warp == 1) {
         double f = 0.0;
         for (int q0 = 0; q0 < dr.nseg; q0 += 32) {
             const double t = (q0 + lane < dr.nseg) ? fp[q0 + lane] : 0.0;
             const int cnt = min(32, dr.nseg - q0);
+#pragma unroll 8
             for (int u = 0; u < cnt; ++u) f = __dadd_rn(f, __shfl_sync(0xffffffffu, t, u));
         }
         if (lane == 0) {
@@ -1319,10 +1450,86 @@ __device__ __forceinline__ void select_finish(const SelectDraws& dr, const int* 
     if (threadIdx.x == 0) *dr.ctr = 0u;
 }
 
+// Chunk q of the scanned entries (from st, a multiple of 128) and its groups' bounds into buffer b
+__device__ __forceinline__ void select_load(double* stage, unsigned* s_gm, const double* v, const unsigned* gm, int ustr,
+                                            int st, int b, unsigned long long* bar)
+{
+    const unsigned len = (unsigned)min(kSelStage, ustr - st), words = (len / 32 + 3) & ~3u;   // within gstr
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(len * 8 + words * 4)
+                 : "memory");
+    bulk_copy_1d(stage + b * kSelStage, v + st, len * 8, bar);
+    bulk_copy_1d(s_gm + b * (kSelStage / 32), gm + st / 32, words * 4, bar);
+}
+
+// The scan of SpecialMathRoutinesForMatrix.h:300-318 over the entries [k, U) by one warp, chunks of
+// kSelStage entries and their groups' bounds streamed through two shared-memory buffers.  The heap's top
+// lives in registers (REGS: k >= 21), the same in every lane: the warp replaces the root in step, without
+// a divergent branch or a broadcast.  A lane holds the bound of 32 consecutive entries; a minimum over
+// the lanes gives the next group that can hold an entry above the root, another one its first such entry,
+// and each further one takes a comparison, a minimum over the lanes and a shuffle, started from the new
+// root before the replaced entry goes on below it.  The root of this heap can also decrease (a deeper
+// entry may move up), so every search compares with the current root.  Returns false if a copy never
+// completed.
+template <bool REGS>
+__device__ __forceinline__ bool select_scan(HeapS& h, int k, const double* v, const unsigned* gm, int U, int ustr, int s0,
+                                            int n_chunks, double* stage, unsigned* s_gm, unsigned long long* s_bar,
+                                            HeapMins* mins, int lane)
+{
+    unsigned long long root = h.key[0];
+    HeapTop top;
+    if (REGS) top.load(h, mins);
+    for (int q = 0; q < n_chunks; ++q) {
+        const int b = q & 1;
+        if (!mbar_wait(&s_bar[b], (unsigned)(q >> 1) & 1u)) return false;
+        const int st = s0 + q * kSelStage;
+        const int len = min(kSelStage, U - st);
+        const double* buf = stage + b * kSelStage;
+        const int lo = max(0, k - st);         // entries of the chunk before k are the heap's first
+        for (int o = 0; o < len; o += 1024) {
+            const unsigned bound = o + 32 * lane < len ? s_gm[b * (kSelStage / 32) + (o >> 5) + lane] : 0u;
+            int g = -1;
+            for (;;) {
+                g = (int)__reduce_min_sync(0xffffffffu,
+                                           (bound > (unsigned)(root >> 32) && lane > g) ? (unsigned)lane : 32u);
+                if (g == 32) break;
+                const int e0 = o + 32 * g, idx = e0 + lane;
+                // outside [k, U) an entry reads as 0, which never exceeds the root
+                const unsigned long long mine = (idx < len && idx >= lo) ? abs_bits(buf[idx]) : 0ull;
+                int l = (int)__reduce_min_sync(0xffffffffu, mine > root ? (unsigned)lane : 32u);
+                unsigned long long cand = __shfl_sync(0xffffffffu, mine, l & 31);
+                while (l < 32) {
+                    const unsigned p = (unsigned)(st + e0 + l);
+                    bool gt = false;
+                    if (REGS) {
+                        gt = top.root(cand, p);
+                        root = top.K0;
+                    } else {
+                        unsigned long long nr = 0ull;
+                        if (lane == 0) nr = heap_replace_root(h, k, cand, p);
+                        root = __shfl_sync(0xffffffffu, nr, 0);
+                    }
+                    l = (int)__reduce_min_sync(0xffffffffu, (mine > root && lane > l) ? (unsigned)lane : 32u);
+                    const unsigned long long nc = __shfl_sync(0xffffffffu, mine, l & 31);
+                    if (REGS && gt) top.below(h, k, cand, p);
+                    cand = nc;
+                }
+            }
+        }
+        __syncwarp();
+        if (lane == 0 && q + 2 < n_chunks) {       // refill this buffer with chunk q + 2
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            select_load(stage, s_gm, v, gm, ustr, s0 + (q + 2) * kSelStage, b, &s_bar[b]);
+        }
+    }
+    if (REGS && lane == 0) top.store(h);
+    return true;
+}
+
 // vals: [n_mat][ustr] packed upper values (signed), rows 16-byte aligned (ustr even); F: [n_mat]
 // squared Frobenius norms.  Output: sel bitmap per matrix, cnt (entries kept before the rounding
 // draw), TopLEK draw request.  err: set to 1 if a bounded wait ran out.
-__global__ void __maxnreg__(192) k_select(const double* __restrict__ vals, int ustr, int U, int k,
+__global__ void __launch_bounds__(kSelThreads, 1) k_select(const double* __restrict__ vals,
+                                                        const unsigned* __restrict__ gmax, int gstr, int ustr, int U, int k,
                                                         int lek, double delta, double* F,
                                                         unsigned* sel, int SW, int* cnt, int* needs,
                                                         double* pdraw, int* minidx, int* err, const int* act,
@@ -1330,7 +1537,10 @@ __global__ void __maxnreg__(192) k_select(const double* __restrict__ vals, int u
 {
     extern __shared__ __align__(16) unsigned long long s_dyn[];
     __shared__ __align__(8) unsigned long long s_bar[2];
-    __shared__ int s_keep, s_fail;
+    __shared__ __align__(16) unsigned s_gm[2 * (kSelStage / 32)];
+    __shared__ HeapMins s_mins;
+    __shared__ int s_keep, s_fail, s_more, s_hit;
+    __shared__ double s_win[5];
     const int c = act ? act[blockIdx.x] : blockIdx.x;
     const double* v = vals + (size_t)c * ustr;
     unsigned* sc = sel + (size_t)c * SW;
@@ -1347,7 +1557,7 @@ __global__ void __maxnreg__(192) k_select(const double* __restrict__ vals, int u
             cnt[c] = U;
             if (needs) needs[c] = 0;
         }
-        if (dr.norms && warp != 0) select_norms(dr, v, U, c, F, warp, lane);
+        if (dr.norms && warp != 0 && warp != 4) select_norms(dr, v, U, c, F, warp, lane);
         if (dr.agg.gc && blockIdx.x == 0 && warp != 0) {
             if (warp == 1) {
                 if (dr.agg.lk) master_l(dr.agg, lane);
@@ -1359,29 +1569,37 @@ __global__ void __maxnreg__(192) k_select(const double* __restrict__ vals, int u
         return;
     }
     double* stage = (double*)s_dyn;                                          // [2][kSelStage]
+    HeapMins* mins = &s_mins;
     HeapS h;
     h.key = align_up_ptr<unsigned long long>(s_dyn + 2 * kSelStage, 32) + 3;  // [k], key+1 32-byte aligned
     double* terms = (double*)(h.key + k);                                    // [k]
     h.hid = align_up_ptr<unsigned>(terms + k, 16) + 3;                       // [k], hid+1 16-byte aligned
     double* csum = align_up_ptr<double>(h.hid + k, 8);                       // [ceil(k/32)]
 
-    // scanned region [k, U) streamed in chunks starting at an even element (16-byte aligned)
-    const int s0 = k & ~1;
+    // scanned region [k, U) streamed in chunks from a multiple of 128 (four groups: 16 bytes of bounds)
+    const unsigned* gm = gmax + (size_t)c * gstr;
+    const int s0 = k & ~127;
     const int n_chunks = (U - s0 + kSelStage - 1) / kSelStage;
     if (tid == 0) {
         s_fail = 0;
         mbar_init(&s_bar[0]);
         mbar_init(&s_bar[1]);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        for (int q = 0; q < 2 && q < n_chunks; ++q) {
-            const int st = s0 + q * kSelStage;
-            const int len = min(kSelStage, ustr - st);
-            tma_load_1d(stage + q * kSelStage, v + st, (unsigned)len * 8u, &s_bar[q]);
-        }
+        for (int q = 0; q < 2 && q < n_chunks; ++q)
+            select_load(stage, s_gm, v, gm, ustr, s0 + q * kSelStage, q, &s_bar[q]);
     }
-    for (int t = tid; t < k; t += blockDim.x) {
-        h.key[t] = abs_bits(v[t]);
-        h.hid[t] = (unsigned)t;
+    for (int t0 = tid; t0 < k; t0 += 8 * blockDim.x) {      // eight loads in flight a thread
+        double x[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) x[u] = t0 + u * (int)blockDim.x < k ? v[t0 + u * blockDim.x] : 0.0;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int t = t0 + u * blockDim.x;
+            if (t < k) {
+                h.key[t] = abs_bits(x[u]);
+                h.hid[t] = (unsigned)t;
+            }
+        }
     }
     __syncthreads();
     // buildMinHeap (MinHeap.h:147-191) level by level, deepest first
@@ -1401,7 +1619,7 @@ __global__ void __maxnreg__(192) k_select(const double* __restrict__ vals, int u
     }
     // scan, SpecialMathRoutinesForMatrix.h:300-318
     if (warp != 0) {
-        if (dr.norms) select_norms(dr, v, U, c, F, warp, lane);
+        if (dr.norms && warp != 4) select_norms(dr, v, U, c, F, warp, lane);
         if (dr.agg.gc && blockIdx.x == 0) {      // the master's aggregation beside the heap walk
             if (warp == 1) {
                 if (dr.agg.lk) master_l(dr.agg, lane);
@@ -1410,75 +1628,9 @@ __global__ void __maxnreg__(192) k_select(const double* __restrict__ vals, int u
             }
         }
     } else {
-        unsigned long long root = h.key[0];
-        // levels 0 and 1 of the heap live in registers during the scan (k >= 21), the same in every
-        // lane: the warp replaces the root in step, without a divergent branch or a broadcast
-        const bool regs = k >= 21;
-        unsigned long long K0 = 0, K1 = 0, K2 = 0, K3 = 0, K4 = 0;
-        unsigned I0 = 0, I1 = 0, I2 = 0, I3 = 0, I4 = 0;
-        if (regs) {
-            K0 = h.key[0]; K1 = h.key[1]; K2 = h.key[2]; K3 = h.key[3]; K4 = h.key[4];
-            I0 = h.hid[0]; I1 = h.hid[1]; I2 = h.hid[2]; I3 = h.hid[3]; I4 = h.hid[4];
-        }
-        for (int q = 0; q < n_chunks; ++q) {
-            const int b = q & 1;
-            if (!mbar_wait(&s_bar[b], (unsigned)(q >> 1) & 1u)) {
-                if (lane == 0) s_fail = 1;
-                break;
-            }
-            const int st = s0 + q * kSelStage;
-            const int len = min(kSelStage, U - st);
-            const double* buf = stage + b * kSelStage;
-            // 256 entries per step, 8 per lane in lane-contiguous groups of 32 (entry e = 32 j + lane
-            // of the step).  Each pass finds the first entry above the root that comes after the last
-            // one taken (each lane its own first, then the warp minimum) and replaces the root with
-            // it.  The root of this heap can also decrease (a deeper element may move up), so every
-            // remaining entry is tested again after each replacement.  Entries outside [k, U) read as
-            // 0, which never exceeds the root.
-            for (int o = 0; o < len; o += 256) {
-                unsigned long long v[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const int idx = o + j * 32 + lane;
-                    v[j] = (idx < len && st + idx >= k) ? abs_bits(buf[idx]) : 0ull;
-                }
-                int done = -1;                           // last entry taken in this step
-                for (;;) {
-                    unsigned e = 0xffffffffu;
-                    unsigned long long mine = 0ull;
-#pragma unroll
-                    for (int j = 7; j >= 0; --j)
-                        if (v[j] > root && j * 32 + lane > done) {
-                            e = (unsigned)(j * 32 + lane);
-                            mine = v[j];
-                        }
-                    e = __reduce_min_sync(0xffffffffu, e);
-                    if (e == 0xffffffffu) break;
-                    const unsigned long long cand = __shfl_sync(0xffffffffu, mine, (int)(e & 31u));
-                    done = (int)e;
-                    if (regs) {
-                        root = heap_replace_root_r(h, k, cand, (unsigned)(st + o + done), K0, K1, K2, K3, K4, I0, I1,
-                                                   I2, I3, I4);
-                        __syncwarp();
-                    } else {
-                        unsigned long long nr = 0ull;
-                        if (lane == 0) nr = heap_replace_root(h, k, cand, (unsigned)(st + o + done));
-                        root = __shfl_sync(0xffffffffu, nr, 0);
-                    }
-                }
-            }
-            __syncwarp();
-            if (lane == 0 && q + 2 < n_chunks) {       // refill this buffer with chunk q + 2
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                const int nst = s0 + (q + 2) * kSelStage;
-                const int nlen = min(kSelStage, ustr - nst);
-                tma_load_1d(stage + b * kSelStage, v + nst, (unsigned)nlen * 8u, &s_bar[b]);
-            }
-        }
-        if (regs && lane == 0) {
-            h.key[0] = K0; h.key[1] = K1; h.key[2] = K2; h.key[3] = K3; h.key[4] = K4;
-            h.hid[0] = I0; h.hid[1] = I1; h.hid[2] = I2; h.hid[3] = I3; h.hid[4] = I4;
-        }
+        const bool ok = k >= 21 ? select_scan<true>(h, k, v, gm, U, ustr, s0, n_chunks, stage, s_gm, s_bar, mins, lane)
+                                : select_scan<false>(h, k, v, gm, U, ustr, s0, n_chunks, stage, s_gm, s_bar, mins, lane);
+        if (!ok && lane == 0) s_fail = 1;
     }
     __syncthreads();
     if (s_fail) {   // a copy never completed: give the copies in flight a bounded chance, report
@@ -1505,9 +1657,49 @@ __global__ void __maxnreg__(192) k_select(const double* __restrict__ vals, int u
             }
         }
         __syncthreads();
+        double num0 = 0.0, omd = 0.0, eps = 0.0, hi = 0.0, carry = 0.0, prev_last = 0.0;
+        double prev_hit = 0.0, next_hit = 0.0;
+        int first = k;
+        // Chunk q's numerators from its extractions' terms (lane t: extraction 32 q + t) and the window test
+        // of SpecialMathRoutinesForMatrix.h:475-476 on the numerators before (prev) and after (next) each:
+        // hi > prev and omd < next + eps.  True at the first chunk holding a hit.
+        auto window = [&](int q, double x) {
+            const int nq = min(32, k - q * 32);
+            double prv, nxt;
+            if (ref) {   // one extraction at a time: every lane walks the chain of adds and lane t keeps
+                         // numerator t; the tests then run side by side
+                double run = carry;
+                prv = nxt = carry;
+#pragma unroll 4
+                for (int t = 0; t < nq; ++t) {
+                    const double tt = __shfl_sync(0xffffffffu, x, t);
+                    if (lane == t) prv = run;
+                    run = __dadd_rn(run, tt);
+                    if (lane == t) nxt = run;
+                }
+                carry = run;
+            } else {     // doubling scan of the terms, plus the carry of the chunks before
+                for (int hh = 1; hh < 32; hh <<= 1) {
+                    const double y = __shfl_up_sync(0xffffffffu, x, hh);
+                    if (lane >= hh) x = __dadd_rn(x, y);
+                }
+                const double tot = __shfl_sync(0xffffffffu, x, nq - 1);
+                nxt = __dadd_rn(carry, x);
+                prv = __shfl_up_sync(0xffffffffu, nxt, 1);
+                if (lane == 0) prv = prev_last;
+                prev_last = __shfl_sync(0xffffffffu, nxt, 31);
+                carry = __dadd_rn(carry, tot);
+            }
+            const unsigned hits = __ballot_sync(0xffffffffu, lane < nq && hi > prv && omd < __dadd_rn(nxt, eps));
+            if (!hits) return false;
+            const int l = __ffs(hits) - 1;
+            first = q * 32 + l;
+            prev_hit = __shfl_sync(0xffffffffu, prv, l);
+            next_hit = __shfl_sync(0xffffffffu, nxt, l);
+            return true;
+        };
         if (warp == 0) {
             const double fr = __ldcg(F + c);     // formed by warp 1 when the norms are formed here
-            double num0;
             if (ref) {   // the reference's order: ||M||^2 minus each heap term in heap-array order
                 double nm = fr;
                 if (lane == 0)
@@ -1519,171 +1711,99 @@ __global__ void __maxnreg__(192) k_select(const double* __restrict__ vals, int u
                     for (int q = 0; q < nch; ++q) sh = __dadd_rn(sh, csum[q]);
                 num0 = __dsub_rn(fr, __shfl_sync(0xffffffffu, sh, 0));
             }
-            // window test of SpecialMathRoutinesForMatrix.h:475-476 on the numerators before (prev) and
-            // after (next) extraction m: hi > prev and omd < next + eps
-            const double omd = __dmul_rn(__dsub_rn(1.0, delta), fr);
-            const double eps = __dmul_rn(1e-1, fr);
-            const double hi = __dadd_rn(omd, eps);
-            int first = k;
-            double prev_hit = 0.0, next_hit = 0.0;
+            omd = __dmul_rn(__dsub_rn(1.0, delta), fr);
+            eps = __dmul_rn(1e-1, fr);
+            hi = __dadd_rn(omd, eps);
+            carry = prev_last = num0;
+            bool more = false;
             // Each numerator is num0 plus non-negative terms, added with monotone rounding, so none is
             // below num0: if hi > num0 fails no extraction opens the window, and none is made.
             if (hi > num0) {
                 // Extraction (extracFromMinHeap, MinHeap.h:125-141) in chunks of 32: element m lands at
-                // position k-1-m.  After each chunk the warp forms the chunk's numerators (doubling
-                // scan of its terms, plus the carry of the chunks before it) and stops at the first
-                // chunk holding a window hit.  Extractions after the hit only reorder positions
-                // [0, k-1-first), whose set is what is kept.  While the heap has more than 21
-                // entries, positions 0..4 live in lane 0's registers.
-                unsigned long long K0 = 0, K1 = 0, K2 = 0, K3 = 0, K4 = 0;
-                unsigned I0 = 0, I1 = 0, I2 = 0, I3 = 0, I4 = 0;
-                int size = k;
-                bool live = false;
-                if (lane == 0 && k > 21) {
-                    K0 = h.key[0]; K1 = h.key[1]; K2 = h.key[2]; K3 = h.key[3]; K4 = h.key[4];
-                    I0 = h.hid[0]; I1 = h.hid[1]; I2 = h.hid[2]; I3 = h.hid[3]; I4 = h.hid[4];
-                    live = true;
-                }
-                double carry = num0, prev_last = num0;
-                for (int q = 0; q < nch; ++q) {
-                    if (lane == 0) {
-                        const int target = max(k - 32 * (q + 1), 1);     // heap size after this chunk
-                        for (; live && size > max(target, 21); --size) {
-                            const int n = size - 1;                      // heap size after the swap
-                            const unsigned long long LK = h.key[n];
-                            const unsigned LI = h.hid[n];
-                            // level-2 keys (positions 5..20), loaded ahead of the level-1 decision
-                            unsigned long long G[16];
-#pragma unroll
-                            for (int t = 0; t < 8; ++t) {
-                                const ulonglong2 g2 = *reinterpret_cast<const ulonglong2*>(h.key + 5 + 2 * t);
-                                G[2 * t] = g2.x;
-                                G[2 * t + 1] = g2.y;
-                            }
-                            h.key[n] = K0;
-                            h.hid[n] = I0;
-                            // level 1, leftmost minimum of the children, moved up if strictly below L
-                            const bool r12 = K2 < K1, r34 = K4 < K3;
-                            const unsigned long long m12 = r12 ? K2 : K1, m34 = r34 ? K4 : K3;
-                            const bool r = m34 < m12;
-                            const unsigned long long lv = r ? m34 : m12;
-                            const int lo = r ? (r34 ? 4 : 3) : (r12 ? 2 : 1);
-                            if (!(LK > lv)) {
-                                K0 = LK;
-                                I0 = LI;
-                                continue;
-                            }
-                            // root takes the child, the child's slot takes L (still in registers)
-                            if (lo == 1) { K0 = K1; I0 = I1; K1 = LK; I1 = LI; }
-                            else if (lo == 2) { K0 = K2; I0 = I2; K2 = LK; I2 = LI; }
-                            else if (lo == 3) { K0 = K3; I0 = I3; K3 = LK; I3 = LI; }
-                            else { K0 = K4; I0 = I4; K4 = LK; I4 = LI; }
-                            // level 2: children of `lo` against the value that moved up (lv)
-                            const int gb = 4 * (lo - 1);
-                            const unsigned long long g0 = lo == 1 ? G[0] : lo == 2 ? G[4] : lo == 3 ? G[8] : G[12];
-                            const unsigned long long g1 = lo == 1 ? G[1] : lo == 2 ? G[5] : lo == 3 ? G[9] : G[13];
-                            const unsigned long long g2 = lo == 1 ? G[2] : lo == 2 ? G[6] : lo == 3 ? G[10] : G[14];
-                            const unsigned long long g3 = lo == 1 ? G[3] : lo == 2 ? G[7] : lo == 3 ? G[11] : G[15];
-                            const bool s01 = g1 < g0, s23 = g3 < g2;
-                            const unsigned long long n01 = s01 ? g1 : g0, n23 = s23 ? g3 : g2;
-                            const bool sr = n23 < n01;
-                            const unsigned long long lv2 = sr ? n23 : n01;
-                            if (!(lv > lv2)) continue;
-                            const int gp = 5 + gb + (sr ? (s23 ? 3 : 2) : (s01 ? 1 : 0));
-                            const unsigned GI = h.hid[gp];
-                            if (lo == 1) { K1 = lv2; I1 = GI; }
-                            else if (lo == 2) { K2 = lv2; I2 = GI; }
-                            else if (lo == 3) { K3 = lv2; I3 = GI; }
-                            else { K4 = lv2; I4 = GI; }
-                            // L enters at gp; deeper levels carry the value that moved up, as the reference
-                            heap_descend(h, gp, n, lv2, LK, LI);
-                        }
-                        if (live && size <= 21) {
-                            h.key[0] = K0; h.key[1] = K1; h.key[2] = K2; h.key[3] = K3; h.key[4] = K4;
-                            h.hid[0] = I0; h.hid[1] = I1; h.hid[2] = I2; h.hid[3] = I3; h.hid[4] = I4;
-                            live = false;
-                        }
-                        for (; size > target; --size) {
-                            const int n = size - 1;
-                            const unsigned long long LK = h.key[n];
-                            const unsigned LI = h.hid[n];
-                            h.key[n] = h.key[0];
-                            h.hid[n] = h.hid[0];
-                            heap_descend(h, 0, n, LK, LK, LI);
-                        }
-                    }
-                    __syncwarp();
-                    const int m = q * 32 + lane;
-                    double x = (m < k) ? term_of(h.key[k - 1 - m], h.hid[k - 1 - m]) : 0.0;
-                    if (ref) {   // numerators one extraction at a time (every lane walks the same chain)
-                        int hit = -1;
-                        double run = carry, ph = 0.0, nh = 0.0;
-                        const int nq = min(32, k - q * 32);
-                        for (int t = 0; t < nq; ++t) {
-                            const double tt = __shfl_sync(0xffffffffu, x, t);
-                            const double nx = __dadd_rn(run, tt);
-                            if (hi > run && omd < __dadd_rn(nx, eps)) {
-                                hit = t;
-                                ph = run;
-                                nh = nx;
-                                break;
-                            }
-                            run = nx;
-                        }
-                        if (hit >= 0) {
-                            first = q * 32 + hit;
-                            prev_hit = ph;
-                            next_hit = nh;
-                            break;
-                        }
-                        carry = run;
-                        continue;
-                    }
-                    for (int hh = 1; hh < 32; hh <<= 1) {
-                        const double y = __shfl_up_sync(0xffffffffu, x, hh);
-                        if (lane >= hh) x = __dadd_rn(x, y);
-                    }
-                    const double tot = __shfl_sync(0xffffffffu, x, min(31, k - 1 - q * 32));
-                    const double nxt = __dadd_rn(carry, x);
-                    double prv = __shfl_up_sync(0xffffffffu, nxt, 1);
-                    if (lane == 0) prv = prev_last;
-                    const unsigned hits = __ballot_sync(0xffffffffu, m < k && hi > prv && omd < __dadd_rn(nxt, eps));
-                    if (hits) {
-                        const int l = __ffs(hits) - 1;
-                        first = q * 32 + l;
-                        prev_hit = __shfl_sync(0xffffffffu, prv, l);
-                        next_hit = __shfl_sync(0xffffffffu, nxt, l);
-                        break;
-                    }
-                    prev_last = __shfl_sync(0xffffffffu, nxt, 31);
-                    carry = __dadd_rn(carry, tot);
-                }
-                if (lane == 0 && live) {
-                    h.key[0] = K0; h.key[1] = K1; h.key[2] = K2; h.key[3] = K3; h.key[4] = K4;
-                    h.hid[0] = I0; h.hid[1] = I1; h.hid[2] = I2; h.hid[3] = I3; h.hid[4] = I4;
+                // position k-1-m.  After each chunk the warp forms the chunk's numerators and stops at the
+                // first chunk holding a window hit.  Extractions after the hit only reorder positions
+                // [0, k-1-first), whose set is what is kept.  Once a run has settled the window opens in the
+                // first chunk.
+                if (lane == 0) {
+                    HeapTop top;
+                    const bool live = k > 21;
+                    if (live) top.load(h, mins);
+                    if (extract_chunk(h, top, live, k, max(k - 32, 1))) top.store(h);
                 }
                 __syncwarp();
+                more = !window(0, lane < k ? term_of(h.key[k - 1 - lane], h.hid[k - 1 - lane]) : 0.0) && nch > 1;
             }
             if (lane == 0) {
-                if (first < k) {
-                    pdraw[c] = __dadd_rn(__dsub_rn(omd, prev_hit), eps) / __dadd_rn(__dsub_rn(next_hit, prev_hit), eps);
-                    needs[c] = 1;
-                    minidx[c] = (int)h.hid[k - 1 - first];
-                    s_keep = k - 1 - first;      // positions [0, k-1-first) stay in the heap
-                } else {
-                    needs[c] = 0;
-                    pdraw[c] = 0.0;
-                    minidx[c] = 0;
-                    s_keep = 0;
+                s_more = more;
+                s_hit = 0;
+                s_win[0] = omd;
+                s_win[1] = eps;
+                s_win[2] = hi;
+                s_win[3] = carry;
+                s_win[4] = prev_last;
+            }
+        }
+        __syncthreads();
+        if (s_more) {
+            // Warp 0 extracts chunk q while warp 1 forms the window of chunk q - 1, whose places no longer
+            // change; a hit is seen a chunk late, which only reorders the places below it.
+            if (warp == 0) {
+                HeapTop top;
+                bool live = k - 32 > 21;
+                if (lane == 0 && live) top.load(h, mins);
+                for (int q = 1;; ++q) {
+                    if (q < nch && lane == 0) live = extract_chunk(h, top, live, k - 32 * q, max(k - 32 * (q + 1), 1));
+                    asm volatile("bar.sync 2, 64;" ::: "memory");
+                    if (s_hit || q == nch) break;
                 }
+                if (lane == 0 && live) top.store(h);
+            } else if (warp == 1) {
+                omd = s_win[0];
+                eps = s_win[1];
+                hi = s_win[2];
+                carry = s_win[3];
+                prev_last = s_win[4];
+                for (int q = 1;; ++q) {
+                    if (q > 1) {
+                        const int m = (q - 1) * 32 + lane;
+                        const bool hit = window(q - 1, m < k ? term_of(h.key[k - 1 - m], h.hid[k - 1 - m]) : 0.0);
+                        if (lane == 0) s_hit = hit;
+                    }
+                    asm volatile("bar.sync 2, 64;" ::: "memory");
+                    if (s_hit || q == nch) break;
+                }
+            }
+        }
+        if (warp == (s_more ? 1 : 0) && lane == 0) {
+            if (first < k) {
+                pdraw[c] = __dadd_rn(__dsub_rn(omd, prev_hit), eps) / __dadd_rn(__dsub_rn(next_hit, prev_hit), eps);
+                needs[c] = 1;
+                minidx[c] = (int)h.hid[k - 1 - first];
+                s_keep = k - 1 - first;      // positions [0, k-1-first) stay in the heap
+            } else {
+                needs[c] = 0;
+                pdraw[c] = 0.0;
+                minidx[c] = 0;
+                s_keep = 0;
             }
         }
         __syncthreads();
         keep = s_keep;
     }
+    // the kept entries' bits, collected in the staging buffers where the bitmap fits there (U <= 262144)
+    unsigned* bits = reinterpret_cast<unsigned*>(stage);
+    const bool local = SW <= 4 * kSelStage;
+    if (local) {
+        for (int w = tid; w < SW; w += blockDim.x) bits[w] = 0u;
+        __syncthreads();
+    }
     for (int t = tid; t < keep; t += blockDim.x) {
         const unsigned p = h.hid[t];
-        atomicOr(&sc[p >> 5], 1u << (p & 31));
+        atomicOr(local ? &bits[p >> 5] : &sc[p >> 5], 1u << (p & 31));
+    }
+    if (local) {
+        __syncthreads();
+        for (int w = tid; w < SW; w += blockDim.x) sc[w] = bits[w];
     }
     if (tid == 0) cnt[c] = keep;
     select_finish(dr, needs, pdraw, minidx, sel, SW, cnt);
@@ -2747,10 +2867,10 @@ __global__ void k_op_identity(const double* diffs, double* shifts, int n_mat, in
         }
     }
 }
-// pack the upper triangle of n column-major d x lda matrices and their full squared norms
-__global__ void k_pack_upper(const double* full, int d, int lda, int U, int ustr, double* packed)
+// pack the upper triangle of n column-major d x lda matrices, with the bounds of their rows of 32 (gmax)
+__global__ void k_pack_upper(const double* full, int d, int lda, int U, int ustr, double* packed, unsigned* gmax, int gstr)
 {
-    int t = blockIdx.y;
+    int t = blockIdx.y;       // with gmax, ustr is a multiple of 32: a warp's positions are one row
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < ustr; p += gridDim.x * blockDim.x) {
         double v = 0.0;
         if (p < U) {
@@ -2759,6 +2879,8 @@ __global__ void k_pack_upper(const double* full, int d, int lda, int U, int ustr
             v = full[(size_t)t * d * lda + (size_t)j * lda + i];
         }
         packed[(size_t)t * ustr + p] = v;
+        const int lane = threadIdx.x & 31;
+        if (gmax) row_bound(gmax + (size_t)t * gstr + (p >> 5), 32, lane, v);
     }
 }
 
