@@ -155,7 +155,7 @@ cudaError_t launch_chol_ref(const Dev& P, int grid, cudaStream_t st, const doubl
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kRefCholThreads);
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = ref_chol_smem(P.d, grid);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
@@ -166,15 +166,15 @@ cudaError_t launch_chol_ref(const Dev& P, int grid, cudaStream_t st, const doubl
                               record);
 }
 
-// CTAs of the reference-order solve: its trailing updates are light, its cost is the per-block
-// barriers and the pivot rows, so a modest grid
-int ref_grid()
+// CTAs of the reference-order solve: one for every 256 entries of the first trailing update, at most one
+// an SM (each holds up to 32 panel columns and the panel's block in shared memory)
+int ref_grid(int d)
 {
-    int dev = 0, sms = 1, bps = 1;
+    int dev = 0, sms = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_chol_ref, kRefCholThreads, 0);
-    return std::max(1, std::min(32, sms * std::max(1, bps)));
+    const long long m = std::max(1, d + 1 - kRefNB);
+    return (int)std::max<long long>(1, std::min<long long>(sms, (m * (m + 1) / 2 + kRefCholThreads - 1) / kRefCholThreads));
 }
 
 }  // namespace
@@ -996,7 +996,7 @@ static int create_impl(const fednl_problem_desc* desc, fednl_handle* out, int64_
     if (P.ref) {
         const size_t ua = (size_t)(h->d + 1) * (h->d + 2) / 2;
         A.want(&P.rref, ua);
-        A.want(&P.racc, 9 * ua);
+        A.want(&P.racc, 8 * ua);
     }
     if (P.fmode) {
         A.want(&P.fterm, h->S);
@@ -1058,7 +1058,11 @@ static int create_impl(const fednl_problem_desc* desc, fednl_handle* out, int64_
     }
     h->chol_grid = chol_grid(h->d);
     if (P.ref) {
-        h->ref_grid = ref_grid();
+        h->ref_grid = ref_grid(h->d);
+        if (fednl_raise_dyn_smem((const void*)k_chol_ref, ref_chol_smem(h->d, h->ref_grid)) != cudaSuccess) {
+            fednl_gpu_destroy(h);
+            return fail(FEDNL_ECUDA, "shared-memory attribute refused");
+        }
         if ((size_t)kFrobRing * h->d * 8 > 48 * 1024)
             fednl_raise_dyn_smem((const void*)k_frob_ref, (size_t)kFrobRing * h->d * 8);
     }

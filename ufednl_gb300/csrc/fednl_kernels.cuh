@@ -103,7 +103,7 @@ struct Dev {
     // the reference's arithmetic order (fednl_refmode.cuh)
     int ref;                // 1: FEDNL_ORDER_REFERENCE
     double* rref;           // [(d+1)(d+2)/2] Cholesky factor with y as column d
-    double* racc;           // [9][(d+1)(d+2)/2] lane and tail accumulators of its dot products
+    double* racc;           // [8][(d+1)(d+2)/2] lane accumulators of its dot products
 };
 
 // ---- helpers -------------------------------------------------------------------------------
@@ -2152,14 +2152,18 @@ __device__ __forceinline__ double rcp_rn_int(double r)
     return __longlong_as_double((long long)(((unsigned long long)(2045u - E) << 52) + (Q - (1ull << 52))));
 }
 
-// r = RN(sqrt(a)) and inv = RN(1 / r) together, as the Cholesky's pivot needs them.  The square root
-// runs as in sqrt_rn_int.  The reciprocal's float-float estimate Q0 ~ 2^105 / T1 is formed from the
-// square root's first Newton value T1 (within 53 of the root S), independently of the square root's
-// second step, so only its exact integer correction waits for S: Q0 is within 361 of 2^105 / T1 and
-// 2^105 / T1 within 2 |T1 - S| + 1 of 2^105 / S, so the residual 2^105 - S Q0 stays below 2^62 and
-// one correction step lands within 1/2 (the FP32 reciprocal of T1 differs from that of S by
-// 2^-46 relative); the remainder test then rounds as in rcp_rn_int.  S = 2^53 (the root rounds up
-// to the next power of two) gives r and 1 / r as exact powers of two.
+// r = RN(sqrt(a)) and inv = RN(1 / r) together, as the reference order's pivot needs them.  As in
+// sqrt_rn_int, with one reciprocal square root y (the hardware's estimate and a Newton step, within
+// 2^-23 relative of 1 / sqrt(M)) in place of the square root and the divisions: ri comes from fm y and its
+// residual (within 12 of sqrt(M)), so the first Newton value T1 is within 190 of the root S and
+// |N - T1^2| < 2^62; the second step's quotient is off by 190 2^-22 and lands within 1/2, and the exact
+// test rounds.  The reciprocal's float-float estimate Q0 ~ 2^105 / T1 starts from y 2^-26 and one Newton
+// step (within 450), independently of the square root's second step, so only its exact integer
+// correction waits for S: 2^105 / T1 is within 2 |T1 - S| + 1 of 2^105 / S, so the residual 2^105 - S Q0
+// stays below 2^63 and one correction step lands within 1/2; the remainder test then rounds as in
+// rcp_rn_int.  S = 2^53 (the root rounds up to the next power of two) gives r and 1 / r as exact powers
+// of two.  With correctly rounded float square root, divisions and reciprocal a row of the reference
+// order's solve took 1500 cycles, now 1260.
 __device__ __forceinline__ double sqrt_rcp_rn_int(double a, double& inv)
 {
     const unsigned long long ia = (unsigned long long)__double_as_longlong(a);
@@ -2173,25 +2177,30 @@ __device__ __forceinline__ double sqrt_rcp_rn_int(double a, double& inv)
     const unsigned long long M = ((ia & 0xFFFFFFFFFFFFFull) | (1ull << 52)) << odd;
     const int eh = ((int)E - 1023 - odd) / 2;
     const float fm = __fmul_rn(__uint2float_rn((unsigned)(M >> 22)), 4194304.0f);
-    const unsigned ri = __float2uint_rn(__fsqrt_rn(fm));
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(fm));
+    y = __fmaf_rn(__fmul_rn(0.5f, y), __fmaf_rn(-__fmul_rn(fm, y), y, 1.0f), y);
+    const float g0 = __fmul_rn(fm, y);
+    const float g = __fmaf_rn(__fmul_rn(0.5f, y), __fmaf_rn(-g0, g0, fm), g0);
+    const unsigned ri = __float2uint_rn(g);
     const long long D0 = (long long)(M - (unsigned long long)ri * ri);
-    const float d1 = __fdiv_rn(__fmul_rn(__int2float_rn((int)(D0 >> 3)), 268435456.0f), __uint2float_rn(ri));
+    const float d1 = __fmul_rn(__int2float_rn((int)(D0 >> 3)), __fmul_rn(y, 268435456.0f));   // D0 2^25 / ri
     unsigned long long T = ((unsigned long long)ri << 26) + (unsigned long long)(long long)__float2int_rn(d1);
     // reciprocal estimate from T1 (= T here), clamped to [2^52, 2^53) so that mh is exact and
     // y0 2^76 an integer; the clamp moves it no further from S < 2^53
     const unsigned long long T1 = min(max(T, 1ull << 52), (1ull << 53) - 1ull);
     const float mh = __fmul_rn(__uint2float_rn((unsigned)(T1 >> 29)), 536870912.0f);
     const float ml = __uint2float_rn((unsigned)(T1 & 0x1FFFFFFFull));
-    const float y0 = __frcp_rn(mh);
+    const float yr = __fmul_rn(y, 0x1p-26f);
+    const float y0 = fminf(__fmaf_rn(yr, __fmaf_rn(-mh, yr, 1.0f), yr), 0x1p-52f);
     const float e = __fsub_rn(fmaf(-mh, y0, 1.0f), __fmul_rn(ml, y0));
     unsigned long long Q = ((unsigned long long)__float2uint_rn(__fmul_rn(y0, 0x1p76f)) << 29) +
                            (unsigned long long)(long long)__float2int_rn(__fmul_rn(__fmul_rn(y0, e), 0x1p105f));
     // square root, second step and rounding
     const unsigned long long Nlo = M << 52;
     long long Rm = (long long)(Nlo - T * T);
-    const float rf = __fmul_rn(__int2float_rn((int)(Rm >> 32)), 4294967296.0f);
-    const float tf = __fmul_rn(__uint2float_rn((unsigned)(T >> 29)), 536870912.0f);
-    T += (unsigned long long)(long long)__float2int_rn(__fdiv_rn(rf, __fmul_rn(tf, 2.0f)));
+    T += (unsigned long long)(long long)__float2int_rn(
+        __fmul_rn(__fmul_rn(__int2float_rn((int)(Rm >> 32)), 32.0f), y));      // (Rm / 2^32) 2^32 y 2^-27
     Rm = (long long)(Nlo - T * T);
     if (Rm > (long long)T) ++T;
     else if (Rm <= -(long long)T) --T;

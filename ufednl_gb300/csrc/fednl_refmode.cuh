@@ -413,130 +413,494 @@ __global__ void k_ls_check_ref(Dev P, double c, double gamma)
 // in the two-Vec4d order.  In the dot of entry (j, i) over k < j, row k goes to lane k mod 8 when
 // k < 8 floor(j/8) and to the in-order tail otherwise; the terms of each lane and of the tail are
 // added in increasing k, which is the order in which the rows of R are finished.  So the kernel runs
-// right-looking over blocks of 8 rows with nine accumulators per entry of the augmented matrix
-// [H | g] (g as column d, whose entries become y):
-//   1. CTA 0 finishes the block's rows one by one (pivot, then the row's entries from their
-//      accumulators with the reference's expression; the block's later rows collect the row in
-//      their tails);
-//   2. grid barrier; every CTA adds the block's 8 rows to lane l of the entries below the block
-//      (row 8b + l into lane l: one product and one add per lane and entry); grid barrier.
-// The backward substitution runs in one warp of CTA 0: for each row from the bottom, lanes 0-7 form
-// the Vec4d lanes of its dot product and lane 8 the tail.  Every value equals the reference's.
+// right-looking with eight lane accumulators per entry of the augmented matrix [H | g] (g as column d,
+// whose entries become y), in panels of 32 rows:
+//   1. every CTA finishes the panel's 32 x 32 block redundantly (no barrier) and, behind it, its own
+//      share of the columns to the right, all in shared memory, 8 rows at a time: the rows' lane sums are
+//      reduced (L); warp 0 runs the pivots' chain one row ahead (tail, square root and reciprocal by
+//      integer arithmetic); warp 1 forms the 8 x 8 block's rows, a lane per entry; warp 3 the block's
+//      columns right of it and warps 2 and 5-7 the own columns follow warp 1 row by row; then all warps
+//      add the 8 rows to the lanes of the panel's later rows;
+//   2. grid barrier; the CTAs add the panel's rows to the lanes of the trailing entries in tiles, four rows
+//      a lane; grid barrier.
+// The backward substitution runs in CTA 0.  Row i's lane q starts with x[i + 1 + q], the value found q
+// rows earlier, so when x[t] is known, lane q of warp 0 forms lane q of row t - 1 - q, all from x[t],
+// x[t + 8], ...; lane 0 completes row t - 1.  Other warps form the next step's products and the row's
+// finished partial sums, so warp 0 issues one dependent add per product and the row's last operations.
+// Every value equals the reference's.
+// Bound by these chains (a dependent FP64 add takes 64 cycles): 1260 cycles a row of the factorisation
+// and 1440 + 8 (d - i) a row of the substitution.  d = 301: 2735 -> 783 us (before: one CTA finishing 8
+// rows at a time from lanes in global memory, a substitution whose products waited for their loads).
 constexpr int kRefCholThreads = 256;
+constexpr int kRefNB = 32;                                       // panel rows
+constexpr int kRefSlab = 16;                                     // panel columns of a CTA per pass
+constexpr int kRefBlock = kRefNB * (kRefNB + 1) / 2;             // block entries (j, i), j <= i
+constexpr int kRefSmemD = 8192;
 
 __device__ __forceinline__ size_t apos(int j, int i) { return (size_t)i * (i + 1) / 2 + j; }
 
-__global__ void __launch_bounds__(kRefCholThreads) k_chol_ref(Dev P, const double* __restrict__ Hin,
-                                                              const double* lptr, double lval,
-                                                              const double* __restrict__ gin, double* dxout,
-                                                              double* xupd, int record)
+// columns a CTA holds at once, and its dynamic shared memory: lanes [8][E], H [E], L [8][64], the rows
+// [32][65] (block columns 0..31, own columns 32..63); the substitution reuses it: products
+// [2][8 ceil(d / 8)] and x [d] (larger d keeps them in global memory)
+__host__ __device__ inline int ref_slab(int d, int G) { return d / G + 1 < kRefSlab ? d / G + 1 : kRefSlab; }
+__host__ __device__ inline size_t ref_chol_smem(int d, int G)
 {
+    const size_t E = kRefBlock + (size_t)kRefNB * ref_slab(d, G);
+    const size_t fac = (9 * E + 8 * 64 + kRefNB * 65) * 8;
+    const size_t sub = d <= kRefSmemD ? (2 * (size_t)((d + 7) & ~7) + d) * 8 : 0;
+    return fac > sub ? fac : sub;
+}
+
+__device__ __forceinline__ double plus_zero(double v)        // 0.0 + v without the FP64 pipe
+{
+    return __double_as_longlong(v) == (long long)0x8000000000000000ull ? 0.0 : v;
+}
+
+// RN(a / b) from inv = RN(1 / b): two Markstein steps (P. W. Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000", 1990): the first leaves a faithful quotient, the second, its
+// remainder exact, rounds it correctly.  Five operations, about half the cycles of the division; operands
+// and quotients near the ends of the exponent range (tested beside the operations) take the division.
+__device__ __forceinline__ double div_by(double a, double b, double inv)
+{
+    double q = __dmul_rn(a, inv);
+    q = __fma_rn(__fma_rn(-q, b, a), inv, q);
+    q = __fma_rn(__fma_rn(-q, b, a), inv, q);
+    const int ea = (int)((unsigned long long)__double_as_longlong(a) >> 52) & 0x7ff;
+    const int eb = (int)((unsigned long long)__double_as_longlong(b) >> 52) & 0x7ff;
+    if ((unsigned)(ea - 200) > 1600u || (unsigned)(eb - 200) > 1600u || (unsigned)(ea - eb + 800) > 1600u)
+        q = __ddiv_rn(a, b);
+    return q;
+}
+
+__global__ void __launch_bounds__(kRefCholThreads, 1) k_chol_ref(Dev P, const double* __restrict__ Hin,
+                                                                 const double* lptr, double lval,
+                                                                 const double* __restrict__ gin, double* dxout,
+                                                                 double* xupd, int record)
+{
+    extern __shared__ double s_ref[];
     GridSync gs(P.bar, gridDim.x);
-    __shared__ double s_r, s_inv;
-    __shared__ int s_bad;
-    const int d = P.d, tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31;
-    const size_t Ua = (size_t)(d + 1) * (d + 2) / 2;
+    __shared__ double s_r[kRefNB], s_inv[kRefNB], s_num1[8], s_tl[8], s_ls[16][8], s_part[2][2], s_last[80], s_ent[4][12];
+    __shared__ int s_bad, s_neg[8];       // a pivot of the factorisation / row k of the 8 was negative
+    const int d = P.d, D = d + 1, tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5;
+    const int G = gridDim.x, bid = blockIdx.x;
+    const size_t Ua = (size_t)D * (d + 2) / 2;
     double* R = P.rref;                       // [Ua] R, column d = y
-    double* acc = P.racc;                     // [9][Ua]: lanes 0..7, then the tail
-    volatile unsigned* badflag = P.bar + 3;   // not positive definite, set by CTA 0 before a barrier
+    double* acc = P.racc;                     // [8][Ua] lanes of the entries right of and below the panel
+    double* rinv = P.work;                    // [d] 1 / R_kk
     const double l = lptr ? *lptr : lval;
-    if (P.ls && blockIdx.x == 0 && tid == 0) P.ls[4] = 0.0;
-    if (blockIdx.x == 0 && tid == 0) *badflag = 0u;
-    {
-        const size_t gtid = (size_t)blockIdx.x * nthr + tid, gthr = (size_t)gridDim.x * nthr;
-        for (size_t p = gtid; p < 9 * Ua; p += gthr) acc[p] = 0.0;
+    const int slab = ref_slab(d, G), E = kRefBlock + kRefNB * slab;
+    double* AL = s_ref;                       // [8][E]
+    double* HV = AL + 8 * (size_t)E;          // [E]
+    double(*Lr)[64] = reinterpret_cast<double(*)[64]>(HV + E);
+    double(*RB)[65] = reinterpret_cast<double(*)[65]>(HV + E + 8 * 64);
+    if (P.ls && bid == 0 && tid == 0) P.ls[4] = 0.0;
+    if (record && bid == G - 1 && warp == 7) {      // ||g||, for the round's statistics
+        const double gsq = refo::dot8_warp(gin, gin, d);
+        if (lane == 0) P.stats[0] = sqrt(gsq);
     }
-    if (!gs.sync()) goto timeout;
-    for (int k0 = 0; k0 < d; k0 += 8) {
-        const int k1 = min(k0 + 8, d);
-        if (blockIdx.x == 0) {
-            for (int k = k0; k < k1; ++k) {
-                if (tid == 0) {
+    if (tid == 0) s_bad = 0;
+    for (int c0 = 0; c0 < d; c0 += kRefNB) {
+        const int nb = min(kRefNB, d - c0), c1 = c0 + nb;
+        const int ntot = D - c1 > bid ? (D - c1 - bid + G - 1) / G : 0;     // own columns c1 + bid + s G
+        // own columns in passes of `slab` (one pass unless d > 32 G); the block is redone in each
+        for (int base = 0; base == 0 || base < ntot; base += slab) {
+            const int ns = max(0, min(slab, ntot - base));
+            const int col0 = c1 + bid + base * G;                            // global column of own column 0
+            __syncthreads();
+            // entries of the panel: block (j, i) at i (i + 1) / 2 + j, own column s at kRefBlock + 32 s + j
+            for (int e = tid; e < kRefBlock + kRefNB * ns; e += nthr) {
+                int j, i;
+                if (e < kRefBlock) {
+                    upper_ij(e, j, i);
+                    if (i >= nb) continue;
+                    i += c0;
+                } else {
+                    j = (e - kRefBlock) & (kRefNB - 1);
+                    if (j >= nb) continue;
+                    i = col0 + ((e - kRefBlock) / kRefNB) * G;
+                }
+                j += c0;
+                double v[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) v[q] = c0 ? acc[q * Ua + apos(j, i)] : 0.0;
+                const double h = i < d ? Hin[up_pos(j, i)] : gin[j];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) AL[q * (size_t)E + e] = v[q];
+                HV[e] = i == j ? __dadd_rn(h, l) : h;
+            }
+            __syncthreads();
+            for (int r0 = 0; r0 < nb; r0 += 8) {
+                const int nr = min(8, nb - r0), r1 = r0 + 8, m = nb - r1;     // rows of the panel after them
+                // L of the 8 rows: a warp per block row, then the own columns' entries
+                for (int t = tid; t < 8 * kRefNB + 8 * ns; t += nthr) {
+                    const bool blk = t < 8 * kRefNB;
+                    const int q = blk ? t >> 5 : (t - 8 * kRefNB) / ns, j = r0 + q;
+                    const int s = blk ? t & 31 : (t - 8 * kRefNB) - q * ns;
+                    if (q >= nr || (blk && (s < j || s >= nb))) continue;
+                    const int e = blk ? s * (s + 1) / 2 + j : kRefBlock + kRefNB * s + j;
                     double c8[8];
 #pragma unroll
-                    for (int q = 0; q < 8; ++q) c8[q] = acc[q * Ua + apos(k, k)];
-                    const double sq = __dadd_rn(refo::lanes8(c8), acc[8 * Ua + apos(k, k)]);
-                    const double a = __dsub_rn(__dadd_rn(Hin[up_pos(k, k)], l), sq);
-                    s_bad = (a < 0.0) ? 1 : 0;
-                    double inv;
-                    const double r = sqrt_rcp_rn_int(a, inv);
-                    s_r = r;
-                    s_inv = inv;
-                    R[apos(k, k)] = r;
+                    for (int u = 0; u < 8; ++u) c8[u] = AL[u * (size_t)E + e];
+                    Lr[q][blk ? s : 32 + s] = refo::lanes8(c8);
+                }
+                __syncthreads();
+                if (warp == 0) {
+                    // the pivots: sq = L + tail, a = (H + l) - sq, r = sqrt(a), 1 / r
+                    const auto pivot = [&](int k, double sq) {
+                        const int j = r0 + k;
+                        const double a = __dsub_rn(HV[j * (j + 1) / 2 + j], sq);
+                        double inv;
+                        const double r = sqrt_rcp_rn_int(a, inv);
+                        if (lane == 0) {
+                            s_r[j] = r;
+                            s_inv[j] = inv;
+                            s_neg[k] = a < 0.0 ? 1 : 0;
+                            if (a < 0.0) s_bad = 1;
+                        }
+                        return inv;
+                    };
+                    double inv = pivot(0, Lr[0][r0]);
+                    for (int k = 0; k < nr; ++k) {
+                        asm volatile("bar.sync 1, 64;" ::: "memory");      // row k's pivot, warp 1's exports
+                        if (s_neg[k]) break;
+                        if (k + 1 < nr) {
+                            const double rk = __dmul_rn(inv, s_num1[k]);
+                            const double tl = __dadd_rn(s_tl[k], __dmul_rn(rk, rk));
+                            inv = pivot(k + 1, __dadd_rn(Lr[k + 1][r0 + k + 1], tl));
+                        }
+                    }
+                } else if (warp == 1) {
+                    // the 8 x 8 block's entries (j, i), 1 <= j <= i < 8, a lane each, in the order of j; row k
+                    // is formed by the lanes of row k (lanes 28.. those of row 0)
+                    int j = 1, i = 1;
+                    {
+                        int e = lane < 28 ? lane : 0;
+                        while (e >= 8 - j) {
+                            e -= 8 - j;
+                            ++j;
+                        }
+                        i = j + e;
+                    }
+                    const bool on = lane < 28 && i < nr;
+                    double tail = 0.0, h = 0.0, L = 0.0;
+                    if (on) {
+                        const int bi = r0 + i;
+                        h = HV[bi * (bi + 1) / 2 + r0 + j];
+                        L = Lr[j][bi];
+                    }
+                    double num0 = 0.0;       // row 0: lane i holds column i (1..7)
+                    if (lane >= 1 && lane < nr) {
+                        const int bi = r0 + lane;
+                        num0 = __dsub_rn(HV[bi * (bi + 1) / 2 + r0], Lr[0][bi]);
+                    }
+                    if (lane == 1) {
+                        s_num1[0] = num0;
+                        s_tl[0] = 0.0;
+                    }
+                    for (int k = 0; k < nr; ++k) {
+                        asm volatile("bar.sync 1, 64;" ::: "memory");      // row k's pivot
+                        if (s_neg[k]) {
+                            asm volatile("bar.arrive %0, 192;" ::"r"(3 + k) : "memory");
+                            break;
+                        }
+                        const double inv = s_inv[r0 + k];
+                        if (k == 0) {
+                            const double r = __dmul_rn(inv, num0);
+                            if (lane < nr) RB[r0][r0 + lane] = lane == 0 ? s_r[r0] : r;
+                        } else {
+                            const double r = __dmul_rn(inv, num0);
+                            if (on && j == k) RB[r0 + k][r0 + i] = i == k ? s_r[r0 + k] : r;
+                        }
+                        __threadfence_block();
+                        __syncwarp();
+                        asm volatile("bar.arrive %0, 192;" ::"r"(3 + k) : "memory");
+                        if (k + 1 < nr) {
+                            const bool later = on && j > k;
+                            const double rj = later ? RB[r0 + k][r0 + j] : 0.0, ri = later ? RB[r0 + k][r0 + i] : 0.0;
+                            const double nt = __dadd_rn(tail, __dmul_rn(rj, ri));
+                            tail = later ? nt : tail;
+                            num0 = __dsub_rn(h, __dadd_rn(L, tail));       // of use for row k + 1
+                            if (on && j == k + 1 && i == k + 2) s_num1[k + 1] = num0;
+                            if (on && j == k + 2 && i == k + 2) s_tl[k + 1] = tail;      // for pivot k + 2
+                        }
+                    }
+                } else if (warp == 3) {
+                    // the block's columns right of the 8, a lane each, row by row behind warp 1
+                    const int i = r0 + 8 + lane;
+                    const bool on = i < nb;
+                    double tail[8], h[8];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        tail[q] = 0.0;
+                        h[q] = on ? HV[i * (i + 1) / 2 + r0 + q] : 0.0;
+                    }
+                    double num = on ? __dsub_rn(h[0], Lr[0][i]) : 0.0;
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        if (k >= nr) break;
+                        asm volatile("bar.sync %0, 192;" ::"r"(3 + k) : "memory");
+                        if (s_neg[k]) break;
+                        if (m <= 0) continue;
+                        const double r = __dmul_rn(s_inv[r0 + k], num);
+                        if (on) RB[r0 + k][i] = r;
+#pragma unroll
+                        for (int q = k + 1; q < 8; ++q) {        // the row joins the tails of the 8 rows after it
+                            tail[q] = __dadd_rn(tail[q], __dmul_rn(RB[r0 + k][r0 + q], r));
+                            if (q == k + 1) num = __dsub_rn(h[q], __dadd_rn(on ? Lr[q][i] : 0.0, tail[q]));
+                        }
+                    }
+                } else if (warp != 4) {
+                    // own columns, four a warp, a lane per column and row: lane 8 c + q holds row q's tail
+                    const int s = (warp == 2 ? 0 : warp - 4) * 4 + (lane >> 3), q = lane & 7;
+                    const bool on = s < ns && q < nr, isd = col0 + s * G == d;
+                    const double h = on ? HV[kRefBlock + kRefNB * s + r0 + q] : 0.0, L = on ? Lr[q][32 + s] : 0.0;
+                    const bool any = (s & ~3) < ns;              // the warp has columns
+                    double tail = 0.0, num = __dsub_rn(h, L);
+                    for (int k = 0; k < nr; ++k) {
+                        asm volatile("bar.sync %0, 192;" ::"r"(3 + k) : "memory");
+                        if (s_neg[k]) break;
+                        if (!any) continue;
+                        double r = __dmul_rn(s_inv[r0 + k], num);
+                        if (isd && q == k && on) r = div_by(num, s_r[r0 + k], s_inv[r0 + k]);
+                        r = __shfl_sync(0xffffffffu, r, (lane & ~7) + k);
+                        if (on && q == k) RB[r0 + k][32 + s] = r;
+                        if (k + 1 < nr) {
+                            const double rj = q > k && q < nr ? RB[r0 + k][r0 + q] : 0.0;
+                            const double nt = __dadd_rn(tail, __dmul_rn(rj, r));
+                            tail = q > k ? nt : tail;
+                            num = __dsub_rn(h, __dadd_rn(L, tail));        // of use for row k + 1
+                        }
+                    }
                 }
                 __syncthreads();
                 if (s_bad) break;
-                const double r = s_r, inv = s_inv;
-                for (int i = k + 1 + tid; i <= d; i += nthr) {
-                    double c8[8];
+                // the 8 rows join the lanes of the panel's later rows
+                if (m > 0) {
+                    const int tb = m * (m + 1) / 2;
+                    for (int t = tid; t < tb + m * ns; t += nthr) {
+                        int j, i, e;
+                        if (t < tb) {
+                            upper_ij(t, j, i);
+                            j += r1;
+                            i += r1;
+                            e = i * (i + 1) / 2 + j;
+                        } else {
+                            const int s = (t - tb) / m;
+                            j = r1 + (t - tb) - s * m;
+                            i = 32 + s;
+                            e = kRefBlock + kRefNB * s + j;
+                        }
+                        double v[8], u[8], w[8];      // loaded before the first store
 #pragma unroll
-                    for (int q = 0; q < 8; ++q) c8[q] = acc[q * Ua + apos(k, i)];
-                    const double dot = __dadd_rn(refo::lanes8(c8), acc[8 * Ua + apos(k, i)]);
-                    R[apos(k, i)] = (i < d) ? __dmul_rn(inv, __dsub_rn(Hin[up_pos(k, i)], dot))
-                                            : __ddiv_rn(__dsub_rn(gin[k], dot), r);
-                }
-                __syncthreads();
-                // the block's later rows j collect row k in their tails: entries (j, i), j <= i <= d
-                for (int j = k + 1; j < k1; ++j) {
-                    const double rkj = R[apos(k, j)];
-                    for (int i = j + tid; i <= d; i += nthr)
-                        acc[8 * Ua + apos(j, i)] = __dadd_rn(acc[8 * Ua + apos(j, i)], __dmul_rn(rkj, R[apos(k, i)]));
+                        for (int q = 0; q < 8; ++q) {
+                            v[q] = AL[q * (size_t)E + e];
+                            u[q] = RB[r0 + q][j];
+                            w[q] = RB[r0 + q][i];
+                        }
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) AL[q * (size_t)E + e] = __dadd_rn(v[q], __dmul_rn(u[q], w[q]));
+                    }
                 }
                 __syncthreads();
             }
-            if (tid == 0 && s_bad) *badflag = 1u;
+            if (s_bad) break;
+            if (bid == 0 && base == 0 && tid < nb) rinv[c0 + tid] = s_inv[tid];
+            if (bid == 0 && base == 0)
+                for (int e = tid; e < kRefBlock; e += nthr) {
+                    int j, i;
+                    upper_ij(e, j, i);
+                    if (i < nb) R[apos(c0 + j, c0 + i)] = RB[j][i];
+                }
+            for (int t = tid; t < nb * ns; t += nthr) {
+                const int s = t / nb, j = t - s * nb;
+                R[apos(c0 + j, col0 + s * G)] = RB[j][32 + s];
+            }
         }
-        if (!gs.sync()) goto timeout;
-        if (*badflag) {
-            if (blockIdx.x == 0 && tid == 0) {
+        if (s_bad) {      // the same decision in every CTA
+            if (bid == 0 && tid == 0) {
                 *P.status = -4;
                 if (record) *P.round_ctr += 1;
             }
             gs.finish();
             return;
         }
-        if (k1 - k0 == 8 && k1 < d) {
-            // lane l of every entry (j, i), k1 <= j <= min(i, d - 1), k1 <= i <= d, adds row k0 + l
-            for (int i = k1 + (int)blockIdx.x; i <= d; i += (int)gridDim.x) {
-                double ri[8];
+        if (!gs.sync()) goto timeout;
+        if (c1 < d) {     // then nb = 32: four rows join each lane of the trailing entries
+            // tiles of TS x TS entries, their 2 TS columns of the panel's rows in shared memory; a thread
+            // forms (entry, lane) pairs, so a small trailing triangle still fills the warps.  A tile of 16
+            // takes about three times as long as one of 8 (FP64 pipe against latency): the size whose
+            // rounds over the CTAs are shorter
+            const int m = D - c1, n16 = (m + 15) / 16, n8 = (m + 7) / 8;
+            const int rounds16 = (n16 * (n16 + 1) / 2 + G - 1) / G, rounds8 = (n8 * (n8 + 1) / 2 + G - 1) / G;
+            const int TS = 3 * rounds16 <= rounds8 ? 16 : 8, nt = TS == 16 ? n16 : n8, sh = TS == 16 ? 4 : 3;
+            double* A = s_ref;                        // [32][TS + 1] columns j
+            double* B = A + kRefNB * (TS + 1);        // [32][TS + 1] columns i
+            for (int tile = bid; tile < nt * (nt + 1) / 2; tile += G) {
+                int tj, ti;
+                upper_ij(tile, tj, ti);
+                const int j0 = c1 + tj * TS, i0 = c1 + ti * TS;
+                __syncthreads();
+                for (int t = tid; t < kRefNB * TS; t += nthr) {
+                    const int k = t & (kRefNB - 1), u = t / kRefNB;
+                    A[k * (TS + 1) + u] = j0 + u <= d ? R[apos(c0 + k, j0 + u)] : 0.0;
+                    B[k * (TS + 1) + u] = i0 + u <= d ? R[apos(c0 + k, i0 + u)] : 0.0;
+                }
+                __syncthreads();
+                for (int t = tid; t < 8 * TS * TS; t += nthr) {
+                    const int ju = t & (TS - 1), iu = (t >> sh) & (TS - 1), q = t >> (2 * sh);
+                    const int j = j0 + ju, i = i0 + iu;
+                    if (j > i || i > d) continue;
+                    double* ap = acc + q * Ua + apos(j, i);
+                    double a = c0 ? *ap : 0.0;
 #pragma unroll
-                for (int q = 0; q < 8; ++q) ri[q] = R[apos(k0 + q, i)];
-                const int jmax = min(i, d - 1);
-                for (int j = k1 + tid; j <= jmax; j += nthr) {
-                    const size_t pe = apos(j, i);
-#pragma unroll
-                    for (int q = 0; q < 8; ++q)
-                        acc[q * Ua + pe] = __dadd_rn(acc[q * Ua + pe], __dmul_rn(R[apos(k0 + q, j)], ri[q]));
+                    for (int k = 0; k < kRefNB; k += 8)
+                        a = __dadd_rn(a, __dmul_rn(A[(k + q) * (TS + 1) + ju], B[(k + q) * (TS + 1) + iu]));
+                    *ap = a;
                 }
             }
             if (!gs.sync()) goto timeout;
         }
     }
-    if (blockIdx.x != 0) {
+    if (bid != 0) {
         gs.finish();
         return;
     }
     {
-        double* x = P.ybuf;                  // [d]
-        if (tid < 32) {
-            for (int i = d - 1; i >= 0; --i) {
-                const int len = d - 1 - i, items = len & ~7;
-                double a = 0.0;
-                if (lane < 8) {
-                    for (int q = lane; q < items; q += 8) a = __dadd_rn(a, __dmul_rn(R[apos(i, i + 1 + q)], x[i + 1 + q]));
-                } else if (lane == 8) {
-                    for (int q = items; q < len; ++q) a = __dadd_rn(a, __dmul_rn(R[apos(i, i + 1 + q)], x[i + 1 + q]));
-                }
-                double c8[8];
-#pragma unroll
-                for (int q = 0; q < 8; ++q) c8[q] = __shfl_sync(0xffffffffu, a, q);
-                const double rest = __shfl_sync(0xffffffffu, a, 8);
-                if (lane == 0) x[i] = __ddiv_rn(__dsub_rn(R[apos(i, d)], __dadd_rn(refo::lanes8(c8), rest)), R[apos(i, i)]);
+        // Backward substitution.  Step t: x[t] is known; lane q of warp 0 forms lane q of row t - 1 - q.
+        const int pst = (d + 7) & ~7;                     // products per buffer: [m][q], element t + 8 m
+        double* prod = d <= kRefSmemD ? s_ref : acc;      // [2][pst]; the lanes are no longer needed
+        double* x = d <= kRefSmemD ? s_ref + 2 * (size_t)pst : P.ybuf;
+        double* rest = P.rinv;                            // [d] the rows' tails
+        auto elems = [&](int i) { return (d - 1 - i) >> 3; };      // of each of row i's lanes
+        const int first = max(0, d - 8);                  // rows first .. d-1: fewer than 8 elements, all tail
+        __syncthreads();
+        // the first rows' entries, y and diagonal in shared memory
+        if (tid < 80) {
+            const int i = first + tid / 10, c = tid % 10;
+            if (i < d) s_last[tid] = c < 8 ? (first + c < d && first + c >= i ? R[apos(i, first + c)] : 0.0)
+                                           : c == 8 ? R[apos(i, d)] : rinv[i];
+        }
+        __syncthreads();
+        if (warp == 0) {
+            for (int i = d - 1; i >= first; --i) {
+                const double* ri = s_last + (i - first) * 10;
+                double sum = 0.0;
+                for (int t = i + 1; t < d; ++t) sum = __dadd_rn(sum, __dmul_rn(ri[t - first], x[t]));
+                const double v = div_by(__dsub_rn(ri[8], __dadd_rn(0.0, sum)), ri[i - first], ri[9]);
+                if (lane == 0) x[i] = v;
                 __syncwarp();
             }
-            if (record) {
-                const double gsq = refo::dot8_warp(gin, gin, d);
-                if (lane == 0) P.stats[0] = sqrt(gsq);
+        }
+        __syncthreads();
+        for (int i = tid; i < first; i += nthr) {         // tails: at most seven elements, of the rows known now
+            const int u0 = i + 1 + 8 * elems(i);
+            double v[7], sum = 0.0;
+#pragma unroll
+            for (int u = 0; u < 7; ++u) v[u] = u0 + u < d ? R[apos(i, u0 + u)] : 0.0;
+#pragma unroll
+            for (int u = 0; u < 7; ++u)
+                if (u0 + u < d) sum = __dadd_rn(sum, __dmul_rn(v[u], x[u0 + u]));
+            rest[i] = sum;
+        }
+        // The products of a step, elements m >= 1: u = 8 m + q, row t - 1 - q, column t + 8 m, by warps 2, 3
+        // and 5-7 (warp 4 shares warp 0's sub-partition, whose FP64 pipe the chain needs).
+        // R is loaded two steps ahead of the products' use (four a thread; more at large d in line).
+        constexpr int kAhead = 4;
+        double rv[kAhead];
+        const int pt = warp < 4 ? tid - 64 : tid - 96, pn = nthr - 96;
+        auto entry = [&](int t, int u, int& c) {
+            const int q = u & 7, mm = u >> 3, i = t - 1 - q;
+            c = t + 8 * mm;
+            return t >= 1 && mm >= 1 && i >= 0 && mm < elems(i) ? (long long)apos(i, c) : -1ll;
+        };
+        auto fetch = [&](int t) {
+#pragma unroll
+            for (int v = 0; v < kAhead; ++v) {
+                int c;
+                const long long at = entry(t, pt + v * pn, c);
+                rv[v] = at >= 0 ? R[at] : 0.0;
+            }
+        };
+        auto products = [&](int t) {
+            double* pr = prod + (size_t)(t & 1) * pst;
+#pragma unroll
+            for (int v = 0; v < kAhead; ++v) {
+                int c;
+                if (entry(t, pt + v * pn, c) >= 0) pr[pt + v * pn] = __dmul_rn(rv[v], x[c]);
+            }
+            for (int u = pt + kAhead * pn; u < pst; u += pn) {
+                int c;
+                const long long at = entry(t, u, c);
+                if (at >= 0) pr[u] = __dmul_rn(R[at], x[c]);
+            }
+        };
+        if (warp >= 2 && warp != 4) fetch(d - 2);       // step d - 1 has no element m >= 1
+        // warp 0's entries of a step, brought to shared memory by warp 1 a step ahead: R of the newest element
+        // (lane q < 8), the row's y (8), diagonal (9), its reciprocal (10) and the row's tail (11)
+        auto ahead = [&](int t) {
+            const int i = t - 1 - lane;
+            double v = 0.0;
+            if (t >= 1) {
+                if (lane < 8 && i >= 0) v = R[apos(i, t)];
+                else if (lane == 8) v = R[apos(t - 1, d)];
+                else if (lane == 9) v = R[apos(t - 1, t - 1)];
+                else if (lane == 10) v = rinv[t - 1];
+                else if (lane == 11 && t - 1 < first) v = rest[t - 1];
+            }
+            return v;
+        };
+        if (warp == 1 && lane < 12) s_ent[(d - 1) & 3][lane] = ahead(d - 1);
+        __syncthreads();
+        // One barrier a step, after the chain: it hands warp 0 the row's partial sums and the next step's
+        // products, and the others the lanes' sums.  The newest x goes on in warp 0's registers; the others
+        // use an x seven barriers after it is stored at the earliest.
+        double xt = x[d - 1], en = warp == 0 ? s_ent[(d - 1) & 3][lane & 7] : 0.0;
+        for (int t = d - 1; t >= 1; --t) {
+            const int row = t - 1;
+            const bool finish = row < first;               // the step completes row t - 1
+            if (warp == 0) {
+                const int i = t - 1 - lane;
+                const bool on = lane < 8 && i >= 0 && i < first;
+                const double* pr = prod + (size_t)(t & 1) * pst + (lane & 7);
+                const int M = on ? elems(i) : 0;
+                const int M0 = (d - t) >> 3;               // lane 0's elements; the others have as many or one more
+                double c = plus_zero(__dmul_rn(en, xt));
+#pragma unroll 8
+                for (int m = 1; m < M0; ++m) c = __dadd_rn(c, pr[8 * m]);
+                if (M0 >= 1 && M > M0) c = __dadd_rn(c, pr[8 * M0]);
+                if (on && M > 0 && lane > 0) s_ls[i & 15][lane] = c;
+                __syncthreads();
+                const double* et = s_ent[t & 3];
+                en = s_ent[(t - 1) & 3][lane & 7];
+                if (finish) {
+                    const double* pa = s_part[t & 1];
+                    double v = __dadd_rn(__dadd_rn(c, s_ls[row & 15][2]), pa[0]);
+                    v = __dadd_rn(plus_zero(v), pa[1]);
+                    v = __dadd_rn(v, et[11]);
+                    v = div_by(__dsub_rn(et[8], v), et[9], et[10]);
+                    if (lane == 0) x[row] = v;
+                    xt = __shfl_sync(0xffffffffu, v, 0);
+                } else {
+                    xt = x[row];
+                }
+            } else {
+                if (warp == 1) {
+                    const double nx = ahead(t - 1);
+                    if (finish) {
+                        const double* c = s_ls[row & 15];
+                        const double p0 = __dadd_rn(c[1], c[3]);
+                        const double p1 = __dadd_rn(__dadd_rn(c[4], c[6]), __dadd_rn(c[5], c[7]));
+                        if (lane == 0) {
+                            s_part[t & 1][0] = p0;
+                            s_part[t & 1][1] = p1;
+                        }
+                    }
+                    if (lane < 12) s_ent[(t - 1) & 3][lane] = nx;
+                } else if (warp != 4) {
+                    products(t - 1);
+                    fetch(t - 2);
+                }
+                __syncthreads();
             }
         }
         __syncthreads();
@@ -555,7 +919,7 @@ __global__ void __launch_bounds__(kRefCholThreads) k_chol_ref(Dev P, const doubl
     gs.finish();
     return;
 timeout:
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (bid == 0 && threadIdx.x == 0) {
         *P.status = -5;
         if (record) *P.round_ctr += 1;
     }
