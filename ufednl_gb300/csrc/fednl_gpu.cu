@@ -595,6 +595,10 @@ int round_hess_mode(fednl_handle h)
     return sel && !h->dev.ref && !h->desc.option_a ? 3 : 0;
 }
 
+// the reference order's ||diff||_F^2 beside the heap walk, while the ring of columns fits next to the heap
+size_t frob_smem(int d) { return (size_t)2 * kFrobCols * d * 8 + 16; }
+bool select_frob_fits(fednl_handle h) { return h->k < h->U && select_smem(h->k) + frob_smem(h->d) <= 225 * 1024; }
+
 size_t hits_smem(fednl_handle h, int nt)
 {
     return hits_stage_bytes(nt) + ((size_t)h->maxn + 2 * h->d + (size_t)(nt / 32) * h->hits_maxrec) * 8;
@@ -729,7 +733,8 @@ int launch_round(fednl_handle h, Marks* M = nullptr, bool client_phase_only = fa
             CKL();
         }
     }
-    if (P.ref) {
+    const bool frob_in_select = P.ref && agg_in_select && select_frob_fits(h);
+    if (P.ref && !frob_in_select) {
         MARK("k_frob_ref");
         k_frob_ref<<<na, kFrobRefThreads, (size_t)kFrobRing * h->d * 8, st>>>(P);
         CKL();
@@ -754,7 +759,13 @@ int launch_round(fednl_handle h, Marks* M = nullptr, bool client_phase_only = fa
             dr.fpart = P.Fpart;
             dr.lk = P.lk;
         }
-        k_select<<<na, kSelThreads, h->k < h->U ? select_smem(h->k) : 0, st>>>(
+        if (frob_in_select) {
+            dr.agg.lk = nullptr;          // l is formed by k_apply
+            dr.frob = h->d;
+            dr.lk = P.lk;
+        }
+        const size_t smem = h->k < h->U ? select_smem(h->k) + (frob_in_select ? frob_smem(h->d) : 0) : 0;
+        k_select<<<na, kSelThreads, smem, st>>>(
             P.diff, P.gmax, P.gstr, h->ustr, h->U, h->k, comp == FEDNL_TOPLEK, delta, P.F, P.sel, h->SW, P.cnt, P.needs, P.pdraw,
             P.minidx, P.status, P.act, P.ref, dr);
         CKL();
@@ -766,7 +777,7 @@ int launch_round(fednl_handle h, Marks* M = nullptr, bool client_phase_only = fa
     }
     if (!apply_in_solve) {
         MARK("k_apply");
-        k_apply<<<(h->U + 127) / 128, 128, 0, st>>>(P);
+        k_apply<<<(h->U + 127) / 128 + (frob_in_select ? 1 : 0), 128, 0, st>>>(P, frob_in_select);
         CKL();
     }
     if (h->pp) {
@@ -1049,8 +1060,10 @@ static int create_impl(const fednl_problem_desc* desc, fednl_handle* out, int64_
         fednl_gpu_destroy(h);
         return fail(FEDNL_ECUDA, "initial copies failed");
     }
-    if (select_smem(h->k) > 48 * 1024 && h->k < h->U)
-        fednl_raise_dyn_smem((const void*)k_select, select_smem(h->k));
+    {
+        const size_t smem = select_smem(h->k) + (P.ref && select_frob_fits(h) ? frob_smem(h->d) : 0);
+        if (smem > 48 * 1024 && h->k < h->U) fednl_raise_dyn_smem((const void*)k_select, smem);
+    }
     if ((h->comp == FEDNL_RANDK && raise_shuffle_smem((const void*)k_randk, h->k) != cudaSuccess) ||
         (h->pp && raise_shuffle_smem((const void*)k_pp_sample, h->tau) != cudaSuccess)) {
         fednl_gpu_destroy(h);

@@ -1376,6 +1376,9 @@ struct SelectDraws {
     int norms, nseg;
     double* fpart;     // [n_mat][nseg]
     double* lk;        // [n_mat]
+    // frob != 0: these warps form the reference order's ||diff||_F^2 and Lk instead (select_frob_ref), in
+    // a ring of 2 kFrobCols columns of `frob` = d entries at the end of the dynamic shared memory
+    int frob;
 };
 
 // The difference's squared Frobenius norm in the fixed segment order (k_hess_binary's, the CPU
@@ -1430,6 +1433,98 @@ __device__ __forceinline__ void select_norms(const SelectDraws& dr, const double
         if (lane == 0) {
             F[c] = f;
             dr.lk[c] = sqrt(f);
+        }
+    }
+}
+
+// ||diff||_F^2 and Lk in the reference's order (MatrixNMD_SIMD_double.h:1068-1253), by the selection
+// kernel's warps beside the heap walk.  The ten running sums of the reference's loop are chains of
+// dependent FP64 adds (eight lane accumulators shared by all columns: column j, rows i < 8 floor(j/8) with
+// i mod 8 = lane; one scalar for rows 8 floor(j/8) .. j-1; one for the diagonal), and a dependent FP64 add
+// costs 64 cycles (320 while another warp issues FP64 instructions on the sub-partition), so everything
+// else is taken off them: warps 3, 6 and 7 square the coming columns into a ring (kFrobCols columns a
+// step, contiguous in the packed order, their loads a step ahead); warp 1, alone on its sub-partition, adds
+// the eight lanes; warp 2 the two scalars.  d = 301: 5681 dependent adds at 86 cycles, 237 us beside the
+// walk, against 346 us for a kernel of its own before it (the round 1617 -> 1453 us).
+constexpr int kFrobCols = 4;
+constexpr int kFrobAhead = 13;       // loads of a staging thread kept a step ahead (4 d entries over 96 threads)
+constexpr int kFrobStagers = 96;
+
+__device__ __forceinline__ void select_frob_ref(double* ring, const double* __restrict__ v, int d, int c, double* F,
+                                                double* lk, double* s_two, int warp, int lane)
+{
+    auto start = [](int j) { return (size_t)j * (j + 1) / 2; };
+    const int steps = (d + kFrobCols - 1) / kFrobCols;
+    double acc = 0.0;
+    // step s: columns kFrobCols s .. are staged, those of step s - 1 added from the other buffer
+    if (warp == 1 || warp == 2) {
+        for (int s = 0; s <= steps; ++s) {
+            if (s > 0) {
+                const int ja = (s - 1) * kFrobCols, jb = min(d, ja + kFrobCols);
+                const double* buf = ring + (size_t)((s - 1) & 1) * kFrobCols * d;
+                for (int j = ja; j < jb; ++j) {
+                    const int items = j & ~7;
+                    if (warp == 1) {           // element m of lane l: m 8 + l
+                        const double* p = buf + (lane & 7);
+                        int m = 0;
+                        for (; m + 8 <= items >> 3; m += 8) {
+                            double w[8];
+#pragma unroll
+                            for (int u = 0; u < 8; ++u) w[u] = p[8 * (m + u)];
+#pragma unroll
+                            for (int u = 0; u < 8; ++u) acc = __dadd_rn(acc, w[u]);
+                        }
+#pragma unroll 4
+                        for (; m < items >> 3; ++m) acc = __dadd_rn(acc, p[8 * m]);
+                    } else if (lane == 0) {
+                        for (int i = items; i < j; ++i) acc = __dadd_rn(acc, buf[i]);
+                    } else if (lane == 1) {
+                        acc = __dadd_rn(acc, buf[j]);
+                    }
+                    buf += j + 1;
+                }
+            }
+            asm volatile("bar.sync 3, 160;" ::: "memory");
+        }
+    } else {
+        const int st = (warp == 3 ? 0 : warp - 5) * 32 + lane;
+        double pre[kFrobAhead];
+        auto fetch = [&](int s) {
+            const size_t o = start(s * kFrobCols);
+            const int len = s < steps ? (int)(start(min(d, (s + 1) * kFrobCols)) - o) : 0;
+#pragma unroll
+            for (int u = 0; u < kFrobAhead; ++u)
+                pre[u] = st + kFrobStagers * u < len ? v[o + st + kFrobStagers * u] : 0.0;
+        };
+        fetch(0);
+        for (int s = 0; s <= steps; ++s) {
+            if (s < steps) {
+                double* buf = ring + (size_t)(s & 1) * kFrobCols * d;
+                const size_t o = start(s * kFrobCols);
+                const int len = (int)(start(min(d, (s + 1) * kFrobCols)) - o);
+#pragma unroll
+                for (int u = 0; u < kFrobAhead; ++u)
+                    if (st + kFrobStagers * u < len) buf[st + kFrobStagers * u] = __dmul_rn(pre[u], pre[u]);
+                for (int i = st + kFrobStagers * kFrobAhead; i < len; i += kFrobStagers)
+                    buf[i] = __dmul_rn(v[o + i], v[o + i]);
+                fetch(s + 1);
+            }
+            asm volatile("bar.sync 3, 160;" ::: "memory");
+        }
+    }
+    if (warp == 2 && lane < 2) s_two[lane] = acc;
+    asm volatile("bar.sync 3, 160;" ::: "memory");
+    if (warp == 1) {
+        double c8[8];
+#pragma unroll
+        for (int l = 0; l < 8; ++l) c8[l] = __shfl_sync(0xffffffffu, acc, l);
+        if (lane == 0) {       // (0 + h(c0..c3)) + h(c4..c7), the tail added last, both triangles, the diagonal
+            double out = __dadd_rn(0.0, __dadd_rn(__dadd_rn(c8[0], c8[2]), __dadd_rn(c8[1], c8[3])));
+            out = __dadd_rn(out, __dadd_rn(__dadd_rn(c8[4], c8[6]), __dadd_rn(c8[5], c8[7])));
+            out = __dadd_rn(out, s_two[0]);
+            const double f = __dadd_rn(__dadd_rn(out, out), s_two[1]);
+            F[c] = f;
+            lk[c] = sqrt(f);
         }
     }
 }
@@ -1620,6 +1715,9 @@ __global__ void __launch_bounds__(kSelThreads, 1) k_select(const double* __restr
     // scan, SpecialMathRoutinesForMatrix.h:300-318
     if (warp != 0) {
         if (dr.norms && warp != 4) select_norms(dr, v, U, c, F, warp, lane);
+        if (dr.frob && warp != 4 && warp != 5)
+            select_frob_ref(align_up_ptr<double>((char*)s_dyn + select_smem_bytes(k), 16), v, dr.frob, c, F, dr.lk,
+                            s_win, warp, lane);
         if (dr.agg.gc && blockIdx.x == 0) {      // the master's aggregation beside the heap walk
             if (warp == 1) {
                 if (dr.agg.lk) master_l(dr.agg, lane);
@@ -2034,8 +2132,13 @@ __device__ __forceinline__ double apply_word(const Dev& P, int p, int lane)
 
 // A warp covers the 32 positions of one selection word.  In the FP64 round the same work runs in
 // the Option-B solve's first phase (chol_body, apply_first).
-__global__ void __launch_bounds__(128) k_apply(Dev P)
+// form_l: the launch has one more block, which forms l (the reference order's Lk come from k_select).
+__global__ void __launch_bounds__(128) k_apply(Dev P, int form_l)
 {
+    if (form_l && blockIdx.x == gridDim.x - 1) {
+        if (threadIdx.x < 32) master_l(MasterAgg{P.gc, P.lk, P.g, P.stats, P.d, P.nc, P.inv_n}, threadIdx.x);
+        return;
+    }
     const int p = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
     const double h = apply_word(P, p, lane);      // blockDim % 32 == 0: the warp covers one word
     if (p < P.U) P.H[p] = h;

@@ -283,6 +283,7 @@ __global__ void k_ls_margin_ref(Dev P, int S)
 }
 
 // ---- 3r. ||diff||_F^2 from the packed upper part, per processed client ----------------------
+// For the compressors without a selection kernel (TopK / TopLEK: select_frob_ref, in k_select).
 // One CTA per client.  The ten running sums of the reference's loop are chains of dependent FP64
 // adds (eight lane accumulators shared by all columns: column j, rows i < 8 floor(j/8) with
 // i mod 8 = lane; one scalar for rows 8 floor(j/8) .. j-1; one for the diagonal), and a dependent
