@@ -22,6 +22,7 @@
 #include <exception>
 #include <functional>
 #include <map>
+#include <queue>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -117,8 +118,9 @@ cudaError_t raise_shuffle_smem(const void* kernel, int k)
     return shuffle_smem(k) > 48 * 1024 ? fednl_raise_dyn_smem(kernel, shuffle_smem(k)) : cudaSuccess;
 }
 
-// CTAs of the cooperative Cholesky: enough threads for the first trailing update, at most one
-// resident CTA per SM
+// CTAs of the cooperative Cholesky, at most one per SM: two warps of the first trailing update each (its
+// entries' chains of 32 fused multiply-adds then run on sub-partitions of their own), which also leaves a
+// CTA few panel columns (d = 69: 3 CTAs of 13 columns 66 us, 12 of 3 60 us)
 int chol_grid(int d)
 {
     int dev = 0, sms = 1, bps = 1;
@@ -126,7 +128,7 @@ int chol_grid(int d)
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_chol_coop, kCoopThreads, 0);
     long long m = d + 1 > kCholNB ? d + 1 - kCholNB : 1;
-    long long want = (m * (m + 1) / 2 + kCoopThreads - 1) / kCoopThreads;
+    long long want = (m * (m + 1) / 2 + 63) / 64;
     long long g = std::min<long long>(want, (long long)sms * std::max(bps, 1));
     g = std::min<long long>(g, sms);
     return (int)std::max<long long>(1, g);
@@ -179,9 +181,23 @@ int ref_grid(int d)
 
 }  // namespace
 
-// One cooperative launch solving several problems' systems: job j gets a contiguous group of CTAs
-// (its share of the SMs, at least one) and its own barrier words.  More jobs than resident CTAs
-// are solved in successive launches.
+// Modelled cycles of one problem's solve on g CTAs: the pivot pairs' chain and the panels' barriers and
+// loads, which no CTA count shortens; the updates' warp operations at the SM's FP64 rate (19 cycles each);
+// and the panel columns beyond a CTA's slab, one a warp.  Measured at g = 1 .. 152 it is within a third of
+// the kernel's time, and only the order of the problems by it matters here.
+static double solve_cycles(int d, int g)
+{
+    const double panels = (d + kCholNB - 1) / kCholNB;
+    const double beyond = std::max(0.0, std::ceil((double)d / g / 2 - kCholSlab));
+    return 725.0 * d + 10e3 * panels + (double)d * d * d / 6 / 32 * 19 / g +
+           panels * std::ceil(beyond / (kCoopThreads / 32)) * 9e3;
+}
+
+// One cooperative launch solving several problems' systems: job j gets a contiguous group of CTAs and its
+// own barrier words.  Every job starts with one CTA, and each further one goes to the job that would
+// finish last, while it still gains from it: the launch lasts as long as its slowest job (shares in
+// proportion to the jobs' own grids gave two problems of d = 1024 beside six smaller ones 35 of 152 CTAs
+// each and a serving tick of 3.79 ms, so 3.24).  More jobs than resident CTAs are solved in successive launches.
 int fednl_solve_batch_launch(const FednlSolveDesc* descs, int n, void* stream)
 {
     if (n <= 0) return FEDNL_OK;
@@ -201,17 +217,23 @@ int fednl_solve_batch_launch(const FednlSolveDesc* descs, int n, void* stream)
     for (int first = 0; first < n; first += cap) {
         const int m = std::min(cap, n - first);
         std::vector<CholJob> jobs(m);
-        std::vector<long long> want(m);
-        long long tot = 0;
+        std::vector<int> share(m, 1), most(m);
+        using Last = std::pair<double, int>;        // (modelled cycles, job)
+        std::priority_queue<Last> last;
         for (int j = 0; j < m; ++j) {
-            want[j] = chol_grid(descs[first + j].d);
-            tot += want[j];
+            most[j] = chol_grid(descs[first + j].d);
+            last.push({solve_cycles(descs[first + j].d, 1), j});
+        }
+        for (int left = cap - m; left > 0 && !last.empty(); --left) {
+            const int j = last.top().second;
+            if (share[j] >= most[j]) break;         // the slowest job has all it can use
+            last.pop();
+            last.push({solve_cycles(descs[first + j].d, ++share[j]), j});
         }
         int cta = 0;
         for (int j = 0; j < m; ++j) {
             const FednlSolveDesc& S = descs[first + j];
-            int g = tot <= cap ? (int)want[j] : (int)std::max<long long>(1, want[j] * (cap - m) / tot + 1);
-            g = std::min(g, cap - cta - (m - 1 - j));
+            const int g = share[j];
             CholJob& J = jobs[j];
             J = CholJob{};
             J.P.d = S.d;

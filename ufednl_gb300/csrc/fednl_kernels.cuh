@@ -75,7 +75,7 @@ struct Dev {
     int* status;            // [1]
     double* stats;          // [2] ||g||, l
     int hist_cap;
-    unsigned* bar;          // [4] grid barrier: arrival count, generation, error flag
+    unsigned* bar;          // [4] grid barrier: arrival count with error flag, finished CTAs (two spare)
     // FedNL-PP (bin_fednl_local_pp); act == nullptr: every client takes part (plain FedNL)
     int pp, n_act;          // n_act: clients processed this round (tau, or nc without PP)
     const int* act;         // [n_act] processed clients in ascending order
@@ -1352,6 +1352,7 @@ __device__ __forceinline__ double lk_mean(const double* lk, int nc, double inv_n
     for (int c0 = 0; c0 < nc; c0 += 32) {
         const double v = (c0 + lane < nc) ? lk[c0 + lane] : 0.0;
         const int cnt = min(32, nc - c0);
+#pragma unroll 8
         for (int t = 0; t < cnt; ++t) l = __dadd_rn(l, __shfl_sync(0xffffffffu, v, t));
     }
     return __dmul_rn(l, inv_n);
@@ -2065,7 +2066,10 @@ __global__ void k_randseqk(unsigned* states, int n_gen, int U, int k, int* rseq,
 // walks its own mask in client order, four clients at a time with their loads issued together (the
 // same operations as one position at a time).  Updates the selecting clients' shifts; returns the
 // new H[p].
-__device__ __forceinline__ double apply_word(const Dev& P, int p, int lane)
+// KIND: 0 the difference itself is sent, 1 the difference times mult (RandK, RandSeqK), 2 its sign and
+// exponent (Natural).
+template <int KIND>
+__device__ __forceinline__ double apply_word_kind(const Dev& P, int p, int lane)
 {
     const bool in = p < P.U;
     const int word = p >> 5;                      // the same for the whole warp
@@ -2090,44 +2094,65 @@ __device__ __forceinline__ double apply_word(const Dev& P, int p, int lane)
             mine |= ((w >> lane) & 1u) << t;
         }
         if (!in) mine = 0u;
-        // each lane walks its own selecting clients, four at a time with their loads issued ahead:
-        // the warp's FP64 instructions then serve the lanes' events side by side, not one client of
-        // the batch at a time (most clients select one or two of a word's 32 positions)
-        while (__any_sync(0xffffffffu, mine != 0u)) {
-            int tt[4];
+        // each lane walks its own selecting clients, four at a time with the next four's loads issued
+        // ahead: the warp's FP64 instructions then serve the lanes' events side by side, not one client of
+        // the batch at a time (most clients select one or two of a word's 32 positions).  No branch parts
+        // the events, so that only the additions into H wait for one another.
+        constexpr int kEv = 4;
+        double dv[kEv], sv[kEv];
+        int cc[kEv];
+        auto gather = [&]() {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                tt[e] = mine ? __ffs(mine) - 1 : -1;
+            for (int e = 0; e < kEv; ++e) {
+                const int t = mine ? __ffs(mine) - 1 : -1;
+                const int c = __shfl_sync(0xffffffffu, cl, t & 31);
                 mine &= mine - 1u;
+                cc[e] = t < 0 ? -1 : c;
+                const size_t q = (size_t)c * P.ustr + p;
+                dv[e] = t >= 0 ? P.diff[q] : 0.0;
+                sv[e] = t >= 0 ? P.shift[q] : 0.0;
             }
-            double dv[4], sv[4];
-            size_t qq[4];
+        };
+        bool any = __any_sync(0xffffffffu, mine != 0u);
+        if (any) gather();
+        while (any) {
+            double item[kEv], v0[kEv], sent[kEv];
+            int c0_[kEv];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int c = __shfl_sync(0xffffffffu, cl, tt[e] < 0 ? 0 : tt[e]);
-                qq[e] = (size_t)c * P.ustr + p;
-                if (tt[e] >= 0) {
-                    dv[e] = P.diff[qq[e]];
-                    sv[e] = P.shift[qq[e]];
-                }
+            for (int e = 0; e < kEv; ++e) {
+                item[e] = KIND == 1 ? __dmul_rn(dv[e], P.mult) : KIND == 2 ? natural_trunc(dv[e]) : dv[e];
+                v0[e] = sv[e];
+                c0_[e] = cc[e];
+            }
+            any = __any_sync(0xffffffffu, mine != 0u);
+            if (any) gather();
+#pragma unroll
+            for (int e = 0; e < kEv; ++e) sent[e] = __dmul_rn(item[e], P.prescale);
+#pragma unroll
+            for (int e = 0; e < kEv; ++e) {
+                const double hn = __dadd_rn(h, sent[e]);
+                h = c0_[e] >= 0 ? hn : h;
+            }
+            const double alpha = P.alpha;
+            if (alpha != 1.0) {      // 1.0 multiplies exactly: no operation then
+#pragma unroll
+                for (int e = 0; e < kEv; ++e) item[e] = __dmul_rn(alpha, item[e]);
             }
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-                if (tt[e] >= 0) {
-                    double item, sent;
-                    if (P.comp == 5) {                 // Natural: master adds preScale * trunc(diff)
-                        item = natural_trunc(dv[e]);
-                        sent = __dmul_rn(P.prescale, item);
-                    } else {
-                        item = (P.comp == 1 || P.comp == 3 || P.comp == 6) ? __dmul_rn(dv[e], P.mult) : dv[e];
-                        sent = __dmul_rn(item, P.prescale);
-                    }
-                    P.shift[qq[e]] = __dadd_rn(sv[e], __dmul_rn(P.alpha, item));
-                    h = __dadd_rn(h, sent);
-                }
+            for (int e = 0; e < kEv; ++e) v0[e] = __dadd_rn(v0[e], item[e]);
+#pragma unroll
+            for (int e = 0; e < kEv; ++e)
+                if (c0_[e] >= 0) P.shift[(size_t)c0_[e] * P.ustr + p] = v0[e];
         }
     }
     return h;
+}
+
+__device__ __forceinline__ double apply_word(const Dev& P, int p, int lane)
+{
+    if (P.comp == 5) return apply_word_kind<2>(P, p, lane);
+    if (P.comp == 1 || P.comp == 3 || P.comp == 6) return apply_word_kind<1>(P, p, lane);
+    return apply_word_kind<0>(P, p, lane);
 }
 
 // A warp covers the 32 positions of one selection word.  In the FP64 round the same work runs in
@@ -2188,6 +2213,7 @@ __device__ __forceinline__ size_t up_pos(int i, int j) { return (size_t)j * (j +
 constexpr int kCholNB = 32;
 constexpr int kCholSlab = 8;                          // panel columns per CTA kept in shared memory
 constexpr int kCoopThreads = 256;
+static_assert(kCholSlab == kCoopThreads / 32, "a warp loads one own column");
 constexpr long long kBarrierCycles = 4000000000ll;   // ~2 s at 2 GHz, then ETIMEOUT
 
 // ---- correctly rounded square root and reciprocal without the FP64 pipe ----------------------
@@ -2323,15 +2349,20 @@ __device__ __forceinline__ double sqrt_rcp_rn_int(double a, double& inv)
     return r;
 }
 
-// Bounded grid barrier of n cooperating CTAs on three words: bar[0] counts arrivals since the
-// launch began (the e-th barrier completes when it reaches e n), bar[1] counts CTAs that have
-// finished, bar[2] is the error flag.  One fence and one reduction per CTA, then a poll with acquire
-// loads: no counter is reset between barriers.  Every CTA calls finish() once after its last
-// barrier; the last one to do so returns both counters to zero for the next launch.  sync() returns
-// false (error flag set) when the other CTAs did not arrive in time.
+// Bounded grid barrier of n cooperating CTAs on two words: bar[0] counts arrivals since the launch began
+// (the e-th barrier completes when it reaches e n) and carries the error flag in its top bit, bar[1]
+// counts CTAs that have finished.  One release reduction per CTA, then a poll with acquire loads of that
+// one word (flag and count in one trip to L2), and the CTA's barrier hands the acquired view to its other
+// threads: no counter is reset between barriers and no further fence is taken.  Every CTA calls finish()
+// once after its last barrier; the last one to do so returns both words to zero for the next launch.
+// sync() returns false (error flag set) when the other CTAs did not arrive in time.  With the flag in a
+// word of its own, read in turn with the count, and a fence behind the poll a barrier of 152 CTAs took
+// 4.2 k cycles, now 2.5 k.
 // A launch that is one thread-block cluster uses the cluster's hardware barrier instead (every
 // thread of every CTA arrives with release and waits with acquire semantics; the callers' control
 // flow is the same in every CTA, so every barrier is reached by all of them).
+constexpr unsigned kBarrierError = 0x80000000u;
+
 struct GridSync {
     unsigned* bar;
     unsigned n;
@@ -2354,25 +2385,22 @@ struct GridSync {
             // arrival with release semantics: after the CTA barrier it publishes every thread's writes
             // of this CTA (the acquire load below makes the other CTAs' writes visible to this one)
             asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
-            volatile unsigned* verr = bar + 2;
             int ok = 1;
             const long long t0 = clock64();
             for (;;) {
                 unsigned v;
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
-                if ((int)(v - target) >= 0) break;
-                if (*verr) {
+                if (v & kBarrierError) {
                     ok = 0;
                     break;
                 }
+                if (v >= target) break;
                 if (clock64() - t0 > kBarrierCycles) {
-                    atomicExch(bar + 2, 1u);
+                    atomicOr(bar, kBarrierError);
                     ok = 0;
                     break;
                 }
             }
-            asm volatile("fence.acq_rel.gpu;" ::: "memory");      // the other CTAs' writes, for this CTA
-            if (*verr) ok = 0;
             s_ok = ok;
         }
         __syncthreads();
@@ -2409,7 +2437,7 @@ __device__ __forceinline__ void chol_body(const Dev& P, const double* __restrict
     __shared__ double s_inv[kCholNB];     // 1 / pivot (single column), p and r (pair)
     __shared__ double s_q[kCholNB];       // q of the pair starting at k
     __shared__ unsigned short s_ent[kCholNB * (kCholNB + 1) / 2];
-    __shared__ int s_fail;
+    __shared__ int s_neg[kCholNB / 2];    // the block's a or det was negative
     __shared__ double s_yb[2][32];
     __shared__ double s_l;
     int ent_nb = -1;
@@ -2434,8 +2462,11 @@ __device__ __forceinline__ void chol_body(const Dev& P, const double* __restrict
                 if (bid == 0) P.stats[1] = lm;
             }
         } else {
-            for (int wd = (int)bid * nmw + (own_l ? warp - 1 : warp); wd < (U + 31) >> 5; wd += NMW) {
-                const int p = wd * 32 + lane;
+            // a word per warp, spread over the CTAs first: a word that most clients selected takes long, and
+            // the SM's FP64 unit serves three to four warps before each waits longer
+            const int words = (U + 31) >> 5;
+            for (int t = (own_l ? warp - 1 : warp) * (int)G + (int)bid; t < words; t += NMW) {
+                const int p = t * 32 + lane;
                 const double hv = apply_word(P, p, lane);
                 if (p < U) {
                     P.H[p] = hv;
@@ -2451,7 +2482,7 @@ __device__ __forceinline__ void chol_body(const Dev& P, const double* __restrict
             l = s_l;
             for (int jj = tid; jj < d; jj += blockDim.x) {
                 const int p = jj * (jj + 1) / 2 + jj;
-                if (((p >> 5) % NMW) / nmw == (int)bid) A[p] = __dadd_rn(P.H[p], l);
+                if ((p >> 5) % (int)G == (int)bid) A[p] = __dadd_rn(P.H[p], l);
             }
         }
     } else {
@@ -2473,13 +2504,23 @@ __device__ __forceinline__ void chol_body(const Dev& P, const double* __restrict
         // shared memory, at most kCholSlab; any further ones are finished after the column loop)
         const int ntot = D > c1 ? (D - c1 - (int)bid + (int)G - 1) / (int)G : 0;
         const int ns = max(0, min(ntot, kCholSlab));
-        for (int t = tid; t < nb * nb; t += blockDim.x) {
-            int i = t % nb, j = t / nb;
-            if (i <= j) Db[i][j] = A[up_pos(c0 + i, c0 + j)];
-        }
-        for (int t = tid; t < nb * ns; t += blockDim.x) {
-            const int i = t % nb, sl = t / nb;
-            Sb[i][sl] = A[up_pos(c0 + i, c1 + (int)bid + sl * (int)G)];
+        {   // all the panel's loads issued before the first is stored: block entries by column (warp w the
+            // columns w, w + 8, ...; lane = row), own columns likewise
+            constexpr int kW = kCoopThreads / 32;
+            double bv[kCholNB / kW], sv;
+            const int sl = warp;                 // kCholSlab = kW columns, one a warp
+#pragma unroll
+            for (int q = 0; q < kCholNB / kW; ++q) {
+                const int j = warp + q * kW;
+                bv[q] = j < nb && lane <= j ? A[up_pos(c0 + lane, c0 + j)] : 0.0;
+            }
+            sv = sl < ns && lane < nb ? A[up_pos(c0 + lane, c1 + (int)bid + sl * (int)G)] : 0.0;
+#pragma unroll
+            for (int q = 0; q < kCholNB / kW; ++q) {
+                const int j = warp + q * kW;
+                if (j < nb && lane <= j) Db[lane][j] = bv[q];
+            }
+            if (sl < ns && lane < nb) Sb[lane][sl] = sv;
         }
         // block entries (i, j), i <= j, listed by descending i: those with i > k are a prefix
         if (nb != ent_nb) {
@@ -2493,7 +2534,6 @@ __device__ __forceinline__ void chol_body(const Dev& P, const double* __restrict
             }
             ent_nb = nb;
         }
-        if (tid == 0) s_fail = 0;
         __syncthreads();
         // Column loop over the panel's pivot blocks: the pairs (k, k+1), k even (2x2 blocks of D),
         // and a single column last when nb is odd.  Warp 0 runs only the pivot chain, one block
@@ -2502,23 +2542,26 @@ __device__ __forceinline__ void chol_body(const Dev& P, const double* __restrict
         // correctly rounded reciprocal and D^{-1} = [[p, q], [q, r]] (a lane per entry).  Six other
         // warps form the multipliers of rows k and k+1 (l1 = fma(p, w1, q w2), l2 = fma(q, w1, r w2)
         // into Rb / SR, a thread per row and column) and apply block k (two fused multiply-adds) to
-        // every other entry below row k+1.  Each of their threads owns fixed entries for the whole panel and keeps them in
-        // registers: block entries e = ut + 192 q of the descending-row list (rows 1..nb-1) and slab
-        // entries (row nb-1 - e / ns, slab column e mod ns) likewise, so the entries still active at
-        // block k (row > k+1) fill the lowest slots of consecutive threads.  An entry is written to
-        // Db / Sb when its row becomes one of the next pivot rows (the entries of the block after
-        // the next one block earlier, for the chain).  Warp 4 stays idle: it shares warp 0's SM
-        // sub-partition, whose FP64 pipe the chain needs.
-        constexpr int kSlotsB = (kCholNB * (kCholNB - 1) / 2 + kCoopThreads - 65) / (kCoopThreads - 64);
-        constexpr int kSlotsS = ((kCholNB - 1) * kCholSlab + kCoopThreads - 65) / (kCoopThreads - 64);
+        // every other entry below row k+1.  Each of their threads owns fixed entries for the whole panel
+        // and keeps them in registers: block entries e = ut + 192 q of the descending-row list (rows
+        // 1..nb-1) and slab entries (row nb-1 - e / ns, slab column e mod ns) likewise, so the entries
+        // still active at block k (row > k+1) fill the lowest slots of consecutive threads.  An entry is
+        // written to Db / Sb when its row becomes one of the next pivot rows (the entries of the block
+        // after the next one block earlier, for the chain).  A warp has one FP64 operation in flight (64
+        // cycles) and the SM's unit takes one every 19, so six update warps finish sooner than fewer with
+        // more entries each: three 25.6 k cycles a panel, four 23.9 k, five 23.7 k, six 22.9 k.
+        constexpr int kUpd = 192;
+        constexpr int kSlotsB = (kCholNB * (kCholNB - 1) / 2 + kUpd - 1) / kUpd;
+        constexpr int kSlotsS = ((kCholNB - 1) * kCholSlab + kUpd - 1) / kUpd;
         const int ut = (warp < 4 ? warp - 1 : warp - 2) * 32 + lane;    // 0..191 for the update warps
+        const bool upd = warp != 0 && warp != 4;
         double vb[kSlotsB], vs[kSlotsS];
         int ib[kSlotsB], jb[kSlotsB], is_[kSlotsS], ss[kSlotsS];
-        if (warp != 0 && warp != 4) {
+        if (upd) {
             const int nbe = nb * (nb - 1) / 2;     // block entries below row 0
 #pragma unroll
             for (int q = 0; q < kSlotsB; ++q) {
-                const int e = ut + q * (kCoopThreads - 64);
+                const int e = ut + q * kUpd;
                 ib[q] = -1;
                 jb[q] = 0;
                 vb[q] = 0.0;
@@ -2531,7 +2574,7 @@ __device__ __forceinline__ void chol_body(const Dev& P, const double* __restrict
             }
 #pragma unroll
             for (int q = 0; q < kSlotsS; ++q) {     // the first slab entries on warps 5-7, one per sub-partition
-                const int e = (ut + 96) % (kCoopThreads - 64) + q * (kCoopThreads - 64);
+                const int e = (ut + kUpd / 2) % kUpd + q * kUpd;
                 is_[q] = -1;
                 ss[q] = 0;
                 vs[q] = 0.0;
@@ -2544,7 +2587,8 @@ __device__ __forceinline__ void chol_body(const Dev& P, const double* __restrict
         }
         // Warp 0: the parameters of the block at k2 from its (updated) entries a, b, c (b, c unused
         // for a single column): the pivot block goes to Rb (0 between the rows of a pair), D^{-1} to
-        // s_inv / s_q, and a negative a or det (not NaN, not -0) fails the factorisation.
+        // s_inv / s_q, and a negative a or det (not NaN, not -0) fails the factorisation (the block's own
+        // flag, read by all after the barrier that ends this step).
         auto block_params = [&](int k2, bool pair2, double a, double b, double c) {
             const auto neg = [](double v) {
                 const long long vb_ = __double_as_longlong(v), mag = vb_ & 0x7fffffffffffffffll;
@@ -2563,21 +2607,25 @@ __device__ __forceinline__ void chol_body(const Dev& P, const double* __restrict
                     Rb[k2][k2] = a;
                     Rb[k2][k2 + 1] = 0.0;
                     Rb[k2 + 1][k2 + 1] = c;
-                    if (neg(a) || neg(det)) s_fail = 1;
+                    s_neg[k2 >> 1] = neg(a) || neg(det) ? 1 : 0;
                 }
             } else {
                 const double inv = rcp_rn_int(a);
                 if (lane == 0) {
                     Rb[k2][k2] = a;
                     s_inv[k2] = inv;
-                    if (neg(a)) s_fail = 1;
+                    s_neg[k2 >> 1] = neg(a) ? 1 : 0;
                 }
             }
         };
         if (warp == 0) block_params(0, nb > 1, Db[0][0], nb > 1 ? Db[0][1] : 0.0, nb > 1 ? Db[1][1] : 0.0);
         __syncthreads();
+        bool failed = false;          // the same in every thread and CTA
         for (int k = 0; k < nb; k += 2) {
-            if (s_fail) break;
+            if (s_neg[k >> 1]) {
+                failed = true;
+                break;
+            }
             const bool pair = k + 1 < nb;
             if (warp == 0) {
                 const int k2 = k + 2;
@@ -2603,10 +2651,10 @@ __device__ __forceinline__ void chol_body(const Dev& P, const double* __restrict
                                  nc = __shfl_sync(0xffffffffu, e, 2);
                     block_params(k2, pair2, na, nbv, nc);
                 }
-            } else if (warp != 4) {
+            } else if (upd) {
                 if (pair) {
                     const double p = s_inv[k], r = s_inv[k + 1], q = s_q[k];
-                    // a thread per (row, column) of the multipliers: warps 1-3, one per sub-partition
+                    // a thread per (row, column) of the multipliers
                     const int nd = nb - 2 - k;                 // block columns k+2 .. nb-1
                     const int o = ut & 1, cix = ut >> 1;
                     const double ca = o ? q : p, cb = o ? r : q;
@@ -2642,7 +2690,7 @@ __device__ __forceinline__ void chol_body(const Dev& P, const double* __restrict
             }
             __syncthreads();
         }
-        if (s_fail) {   // identical decision in every CTA: all leave together
+        if (failed) {   // identical decision in every CTA: all leave together
             if (bid == 0 && tid == 0) {
                 *P.status = -4;
                 if (record) *P.round_ctr += 1;
@@ -2650,17 +2698,14 @@ __device__ __forceinline__ void chol_body(const Dev& P, const double* __restrict
             return;
         }
         if (bid == 0) {
-            for (int t = tid; t < nb * nb; t += blockDim.x) {
-                int i = t % nb, j = t / nb;
-                if (i <= j) A[up_pos(c0 + i, c0 + j)] = Rb[i][j];
-            }
+            for (int j = warp; j < nb; j += kCoopThreads / 32)
+                if (lane <= j) A[up_pos(c0 + lane, c0 + j)] = Rb[lane][j];
             for (int t = tid; t < nb; t += blockDim.x) P.rinv[c0 + t] = s_inv[t];
         }
-        for (int t = tid; t < nb * ns; t += blockDim.x) {
-            const int i = t % nb, sl = t / nb;
-            const int j = c1 + (int)bid + sl * (int)G;
-            A[up_pos(c0 + i, j)] = SR[i][sl];
-            W[(size_t)i * D + j] = Sb[i][sl];
+        if (warp < ns && lane < nb) {          // an own column a warp
+            const int j = c1 + (int)bid + warp * (int)G;
+            A[up_pos(c0 + lane, j)] = SR[lane][warp];
+            W[(size_t)lane * D + j] = Sb[lane][warp];
         }
         // panel columns beyond the slab (very large d only): one column per warp, same blocks
         {
@@ -2693,27 +2738,44 @@ __device__ __forceinline__ void chol_body(const Dev& P, const double* __restrict
         }
         if (c1 >= d) break;
         if (!gs.sync()) goto timeout;
-        // trailing update, entries (i, j) with c1 <= i <= j < D (column d carries y)
+        // trailing update, entries (i, j) with c1 <= i <= j < D (column d carries y), in tiles of 8 x 8: two
+        // warps a tile, its 8 columns of multipliers (i) and of unscaled rows (j) in shared memory (the
+        // panel's buffers), four tiles a CTA at once, the tiles spread over the CTAs first.  Bound by the
+        // entry's 32 dependent operations and a trip to L2.  With each thread loading its 64 operands a
+        // panel's update took 5.2-7.0 k cycles at d = 301, now 4.2-5.7 k.
         {
-            const int m = D - c1;
-            const int T = m * (m + 1) / 2;
-            for (int e = gtid; e < T; e += gthreads) {
-                int ii, jj;
-                upper_ij(e, ii, jj);
-                const int i = c1 + ii, j = c1 + jj;
-                const double* ci = A + up_pos(0, i);
-                const double* wj = W + j;
-                double u[kCholNB], w[kCholNB];     // multipliers l_ki, unscaled a_kj, loaded ahead
+            const int m = D - c1, nt = (m + 7) / 8, ntiles = nt * (nt + 1) / 2;
+            const int half = tid >> 6, ht = tid & 63, iu = ht & 7, ju = ht >> 3;
+            double* U = &Db[0][0] + half * (kCholNB * 8);      // [32][8] of this half-pair's tile
+            double* V = &Rb[0][0] + half * (kCholNB * 8);
+            for (int t0 = (int)bid; t0 < ntiles; t0 += 4 * (int)G) {
+                const int tile = t0 + half * (int)G;
+                int ti = 0, tj = 0;
+                const bool on = tile < ntiles;
+                if (on) upper_ij(tile, ti, tj);
+                const int i0 = c1 + 8 * ti, j0 = c1 + 8 * tj, i = i0 + iu, j = j0 + ju;
+                const bool live = on && i <= j && j < D;
+                double u4[4], v4[4], a = 0.0;
 #pragma unroll
-                for (int k = 0; k < kCholNB; ++k) {
-                    u[k] = k < nb ? ci[c0 + k] : 0.0;
-                    w[k] = k < nb ? wj[(size_t)k * D] : 0.0;
+                for (int q = 0; q < 4; ++q) {       // element (row k, column c): U from A's columns, V from W's rows
+                    const int ku = ht & 31, cu = (ht >> 5) + 2 * q, kv = (ht >> 3) + 8 * q, cv = ht & 7;
+                    u4[q] = on && i0 + cu < d ? A[up_pos(c0 + ku, i0 + cu)] : 0.0;
+                    v4[q] = on && j0 + cv < D ? W[(size_t)kv * D + j0 + cv] : 0.0;
                 }
-                double a = A[up_pos(i, j)];
+                if (live) a = A[up_pos(i, j)];
+                __syncthreads();
 #pragma unroll
-                for (int k = 0; k < kCholNB; ++k)
-                    if (k < nb) a = fma(-u[k], w[k], a);
-                A[up_pos(i, j)] = a;
+                for (int q = 0; q < 4; ++q) {
+                    const int ku = ht & 31, cu = (ht >> 5) + 2 * q, kv = (ht >> 3) + 8 * q, cv = ht & 7;
+                    U[ku * 8 + cu] = u4[q];
+                    V[kv * 8 + cv] = v4[q];
+                }
+                __syncthreads();
+                if (live && i < d) {
+#pragma unroll
+                    for (int k = 0; k < kCholNB; ++k) a = fma(-U[k * 8 + iu], V[k * 8 + ju], a);
+                    A[up_pos(i, j)] = a;
+                }
             }
         }
         if (!gs.sync()) goto timeout;
@@ -2771,6 +2833,9 @@ __device__ __forceinline__ void chol_body(const Dev& P, const double* __restrict
         }
         for (int blk = 0; blk < nblocks; ++blk) {
             const int b1 = d - 32 * blk, b0 = max(0, b1 - 32), nbk = b1 - b0;
+            const int n0 = max(0, b0 - 32);                 // next block: rows [n0, b0)
+            const int ut = (warp < 4 ? warp - 1 : warp - 2) * 32 + lane;      // warps 1-3 and 5-7
+            double av1[32];
             if (tid < 32) {
                 double ar[32];
 #pragma unroll
@@ -2790,9 +2855,11 @@ __device__ __forceinline__ void chol_body(const Dev& P, const double* __restrict
             } else if (warp == 4) {
                 asm volatile("bar.sync 3, 64;" ::: "memory");
                 if (blk + 1 < nblocks) stage_t(blk + 1);
+            } else if (ut < n0) {      // the first row's entries, while warp 0 solves the block
+#pragma unroll
+                for (int s = 0; s < 32; ++s) av1[s] = (s < nbk) ? A[up_pos(ut, b0 + s)] : 0.0;
             }
             __syncthreads();
-            const int n0 = max(0, b0 - 32);                 // next block: rows [n0, b0)
             if (tid < 32) {
                 double av[32];
 #pragma unroll
@@ -2810,16 +2877,17 @@ __device__ __forceinline__ void chol_body(const Dev& P, const double* __restrict
                 asm volatile("bar.sync 2, 64;" ::: "memory");
                 if (blk + 1 < nblocks) stage_r(blk + 1);
             } else {
-                const int ut = (warp < 4 ? warp - 1 : warp - 2) * 32 + lane;
                 for (int i = ut; i < n0; i += blockDim.x - 64) {
-                    double av[32];
-#pragma unroll
-                    for (int s = 0; s < 32; ++s) av[s] = (s < nbk) ? A[up_pos(i, b0 + s)] : 0.0;
                     double w = y[i];
 #pragma unroll
                     for (int s = 31; s >= 0; --s)
-                        if (s < nbk) w = fma(-av[s], s_yb[blk & 1][s], w);
+                        if (s < nbk) w = fma(-av1[s], s_yb[blk & 1][s], w);
                     y[i] = w;
+                    if (i + (int)blockDim.x - 64 < n0) {
+#pragma unroll
+                        for (int s = 0; s < 32; ++s)
+                            av1[s] = (s < nbk) ? A[up_pos(i + blockDim.x - 64, b0 + s)] : 0.0;
+                    }
                 }
             }
         }
