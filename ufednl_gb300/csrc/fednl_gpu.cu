@@ -587,6 +587,20 @@ int mark(fednl_handle h, Marks* m, const char* name)
 // intercept's sums
 int client_threads(int d) { return std::min(1024, std::max(128, (2 * d + 31) / 32 * 32 + 32)); }
 
+// The client oracle of {0,1} features in the fixed order runs as one kernel, a CTA per client, as long as
+// all CTAs are resident at once; past that its short-lived CTAs queue, and the margins go to a thread per
+// sample over all clients and the sums to k_grad_binary (same operations, same values).  A FedNL-PP round
+// at d = 69, one kernel against two: 2048 clients of 6 samples 149 / 141 us, of 16 164 / 156, of 32
+// 182 / 186, of 48 215 / 209, of 100 270 / 262; 512 clients of 6 113 / 119, of 64 145 / 147; 128 clients
+// of 6 108 / 115; d = 301, 142 clients of 20 414 / 424.
+bool one_client_kernel(fednl_handle h)
+{
+    int dev = 0, sms = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return h->binary && !h->dev.ref && (long long)h->nc * client_threads(h->d) <= sms * 2048ll;
+}
+
 // dynamic shared memory of k_client_binary: the weights and the intercept's word sums
 size_t client_smem(fednl_handle h) { return (size_t)h->maxn * 16 + (size_t)((h->maxn + 63) / 64) * 16; }
 
@@ -697,19 +711,25 @@ int launch_round(fednl_handle h, Marks* M = nullptr, bool client_phase_only = fa
         }
         return FEDNL_OK;
     };
-    if (fork) {
+    // FedNL-PP: the branch samples the round's clients and makes their draws beside the client oracle (which
+    // takes every client), then forms the true gradient and its norm beside the rest of the round
+    const bool pfork = !M && h->side && h->pp;
+    if (fork || pfork) {
         CK(cudaEventRecord(h->fork_ev, st));
         CK(cudaStreamWaitEvent(h->side, h->fork_ev, 0));
-        int rc = draw(h->side);
-        if (rc) return rc;
     }
     if (h->pp) {
         MARK("k_pp_sample");
-        k_pp_sample<<<1, kPPThreads, shuffle_smem(h->tau), st>>>(
+        k_pp_sample<<<1, kPPThreads, shuffle_smem(h->tau), pfork ? h->side : st>>>(
             h->nc, h->tau, P.sampler, shuffle_smem(h->tau) ? nullptr : P.shuf, (int*)P.act, P.is_sel, P.needs);
         CKL();
     }
-    if (h->binary && !P.ref) {       // the client oracle in one launch
+    if (fork || pfork) {
+        int rc = draw(h->side);
+        if (rc) return rc;
+    }
+    if (pfork) CK(cudaEventRecord(h->join_ev, h->side));
+    if (one_client_kernel(h)) {      // the client oracle in one launch
         MARK("k_client_binary");
         k_client_binary<<<h->nc, client_threads(h->d), client_smem(h), st>>>(P);
         CKL();
@@ -730,12 +750,20 @@ int launch_round(fednl_handle h, Marks* M = nullptr, bool client_phase_only = fa
         CKL();
     }
     if (h->pp) {
+        cudaStream_t s2 = st;
+        if (pfork) {
+            CK(cudaStreamWaitEvent(st, h->join_ev, 0));
+            CK(cudaEventRecord(h->fork_ev, st));
+            CK(cudaStreamWaitEvent(h->side, h->fork_ev, 0));
+            s2 = h->side;
+        }
         MARK("k_pp_truegrad");
-        k_pp_truegrad<<<(h->d + 3) / 4, 128, 0, st>>>(P);
+        k_pp_truegrad<<<(h->d + 3) / 4, 128, 0, s2>>>(P);
         CKL();
         MARK("k_pp_norm");
-        k_pp_norm<<<1, 32, 0, st>>>(P);
+        k_pp_norm<<<1, 32, 0, s2>>>(P);
         CKL();
+        if (pfork) CK(cudaEventRecord(h->join_ev, h->side));
     }
     // the master merge runs in the solve's first phase (FP64 order, not FedNL-PP, not when the
     // solve is left to a batched launch)
@@ -793,7 +821,7 @@ int launch_round(fednl_handle h, Marks* M = nullptr, bool client_phase_only = fa
         CKL();
     } else if (fork) {
         CK(cudaStreamWaitEvent(st, h->join_ev, 0));     // the draws and the aggregation
-    } else {
+    } else if (!pfork) {
         int rc = draw(st);
         if (rc) return rc;
     }
@@ -807,14 +835,15 @@ int launch_round(fednl_handle h, Marks* M = nullptr, bool client_phase_only = fa
         k_pp_lkpart<<<dim3(h->nfpart, na), kHessThreads, 0, st>>>(P);
         CKL();
         MARK("k_pp_dir");
-        k_pp_dir<<<na, 128, 0, st>>>(P);
+        k_pp_dir<<<na, std::min(1024, 32 + (h->d + 31) / 32 * 32), 0, st>>>(P);     // + the warp for Lk
         CKL();
         MARK("k_pp_aggregate");
-        k_pp_aggregate<<<(h->d + 127) / 128, 128, 0, st>>>(P);
+        k_pp_aggregate<<<(h->d + 31) / 32 + 1, 32, 0, st>>>(P);      // + the block for l
         CKL();
         MARK("k_chol_coop");     // x = (H + l I)^-1 g (bin_fednl_local_pp TrainLoop.h:1560-1600)
         CK(cudaMemsetAsync(P.bar, 0, 4 * sizeof(unsigned), st));   // barrier words and error flag start at zero
         CK(launch_chol(P, h->chol_grid, st, P.H, 0, P.stats + 1, 0.0, P.g, P.x, nullptr, 0));
+        if (pfork) CK(cudaStreamWaitEvent(st, h->join_ev, 0));
         MARK("end");
         return FEDNL_OK;
     }
@@ -837,7 +866,7 @@ int launch_round(fednl_handle h, Marks* M = nullptr, bool client_phase_only = fa
     const fednl_problem_desc& D = h->desc;
     const double* lptr = D.option_a ? nullptr : P.stats + 1;      // Option A: H + lambda I
     // barrier words and error flag start at zero (the binary client oracle zeroes them at the round's start)
-    if (!(h->binary && !P.ref)) CK(cudaMemsetAsync(P.bar, 0, 4 * sizeof(unsigned), st));
+    if (!one_client_kernel(h)) CK(cudaMemsetAsync(P.bar, 0, 4 * sizeof(unsigned), st));
     if (P.ref) {
         MARK("k_chol_ref");
         CK(launch_chol_ref(P, h->ref_grid, st, lptr, P.lambda, P.dx, D.line_search ? nullptr : P.x, 1));
