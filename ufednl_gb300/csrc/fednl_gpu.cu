@@ -339,7 +339,11 @@ size_t chol32c_smem(int d, int* resident)
     }
     const size_t rb = c32c_smem_bytes(d, true);
     *resident = (d + 31) / 32 <= kC32ResBlocks && rb + stat + 1024 <= (size_t)optin ? 1 : 0;
-    return *resident ? rb : c32c_smem_bytes(d, false);
+    if (*resident) return rb;
+    // with room for the solves on two clusters of 16, where that fits
+    const size_t need = std::max(c32c_cluster_blocks(d, 16, true, false), c32c_cluster_blocks(d, 16, false, true));
+    const size_t pb = c32c_smem_bytes(d, false), cb = (size_t)(c32c_head_floats(d) - 1024 + need * 1024) * 4;
+    return cb + stat + 1024 <= (size_t)optin ? std::max(pb, cb) : pb;
 }
 
 // resident CTAs of k_chol32c for dimension d (the cooperative launch's upper bound)
@@ -354,16 +358,15 @@ int chol32c_cap(int d)
     return std::min(sms, sms * bps);
 }
 
-// whether one cluster of n CTAs of k_chol32c can be resident for dimension d
-bool chol32c_cluster_ok(int d, int n)
+// how many clusters of n CTAs of k_chol32c can be resident for dimension d
+int chol32c_clusters(int d, int n)
 {
     static std::mutex mu;
-    static std::map<std::pair<int, int>, bool> cache;
+    static std::map<std::pair<int, int>, int> cache;
     std::lock_guard<std::mutex> g(mu);
     auto it = cache.find({d, n});
     if (it != cache.end()) return it->second;
-    bool ok = false;
-    int res = 0;
+    int clusters = 0, res = 0;
     const size_t smem = chol32c_smem(d, &res);
     if (fednl_raise_dyn_smem((const void*)k_chol32c, smem) == cudaSuccess &&
         (n <= 8 || cudaFuncSetAttribute(k_chol32c, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess)) {
@@ -378,13 +381,13 @@ bool chol32c_cluster_ok(int d, int n)
         at[0].val.clusterDim.z = 1;
         cfg.attrs = at;
         cfg.numAttrs = 1;
-        int clusters = 0;
-        ok = cudaOccupancyMaxActiveClusters(&clusters, k_chol32c, &cfg) == cudaSuccess && clusters >= 1;
+        if (cudaOccupancyMaxActiveClusters(&clusters, k_chol32c, &cfg) != cudaSuccess) clusters = 0;
     }
     cudaGetLastError();
-    cache[{d, n}] = ok;
-    return ok;
+    cache[{d, n}] = clusters;
+    return clusters;
 }
+bool chol32c_cluster_ok(int d, int n) { return chol32c_clusters(d, n) >= 1; }
 
 // default launch: one cluster of 16 CTAs while the trailing updates are small (d up to 512), else
 // one CTA per 32 x 32 tile of the first trailing update within the resident limit (a negative
@@ -433,25 +436,44 @@ int fednl_device_optionb_solve32(const FednlSolveDesc& S, const FednlSolve32& E,
     const bool cl = grid < 0;
     if (cl && !chol32c_cluster_ok(S.d, -grid)) return FEDNL_EINVAL;
     grid = cl ? -grid : std::min(grid, cap);
+    // The solves run on clusters when CTA 0 does not keep the factor and their blocks fit: on the one
+    // cluster of the launch, or on two clusters of 16 of a cooperative grid
+    const int slots = ((int)(smem / 4) - (c32c_head_floats(S.d) - 1024)) / 1024;
+    int ncl = 0;
+    if (!res && cl) {
+        const int need = c32c_cluster_blocks(S.d, grid, true, true);
+        if (need > 0 && need <= slots) ncl = grid;
+    } else if (!res && grid >= 32) {
+        const int need = std::max(c32c_cluster_blocks(S.d, 16, true, false), c32c_cluster_blocks(S.d, 16, false, true));
+        const int most = chol32c_clusters(S.d, 16);
+        if (need > 0 && need <= slots && most >= 2) {
+            ncl = 16;
+            grid = 16 * std::min(most, grid / 16);
+        }
+    }
     Chol32c C{E.a,  E.diag0, E.linv, E.r,     E.acc,   E.accp, E.hh, E.hl,         E.rh,
-              E.rl, E.flag,  c32c_ld(S.d), E.refine, E.tol, res,    (int)(smem / 4), cl ? 1 : 0};
+              E.rl, E.flag,  c32c_ld(S.d), E.refine, E.tol, res,    (int)(smem / 4), cl ? 1 : 0, ncl};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kCoopThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    if (cl) {
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = grid;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-    } else {
-        attr[0].id = cudaLaunchAttributeCooperative;
-        attr[0].val.cooperative = 1;
+    cudaLaunchAttribute attr[2];
+    int na = 0;
+    if (cl || ncl) {
+        attr[na].id = cudaLaunchAttributeClusterDimension;
+        attr[na].val.clusterDim.x = cl ? grid : ncl;
+        attr[na].val.clusterDim.y = 1;
+        attr[na].val.clusterDim.z = 1;
+        ++na;
+    }
+    if (!cl) {
+        attr[na].id = cudaLaunchAttributeCooperative;
+        attr[na].val.cooperative = 1;
+        ++na;
     }
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = na;
     CK(cudaLaunchKernelEx(&cfg, k_chol32c, P, C, S.H, S.lptr, S.g, S.dx, S.xupd, S.record));
     return FEDNL_OK;
 }
