@@ -322,54 +322,21 @@ int fednl_device_optionb_solve(const double* H, int d, const double* lptr, const
 // ---- the FP32 cooperative solve of the mixed-precision form (fednl_chol32c.cuh) ---------------
 namespace {
 
-// dynamic shared memory of k_chol32c for dimension d, and whether CTA 0 keeps the factor resident
-// (when it fits beside the kernel's static shared memory)
-size_t chol32c_smem(int d, int* resident)
-{
-    static int optin = -1;
-    static size_t stat = 0;
-    if (optin < 0) {
-        int dev = 0, o = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&o, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-        cudaFuncAttributes fa{};
-        cudaFuncGetAttributes(&fa, k_chol32c);
-        stat = fa.sharedSizeBytes;
-        optin = o;
-    }
-    const size_t rb = c32c_smem_bytes(d, true);
-    *resident = (d + 31) / 32 <= kC32ResBlocks && rb + stat + 1024 <= (size_t)optin ? 1 : 0;
-    if (*resident) return rb;
-    // with room for the solves on two clusters of 16, where that fits
-    const size_t need = std::max(c32c_cluster_blocks(d, 16, true, false), c32c_cluster_blocks(d, 16, false, true));
-    const size_t pb = c32c_smem_bytes(d, false), cb = (size_t)(c32c_head_floats(d) - 1024 + need * 1024) * 4;
-    return cb + stat + 1024 <= (size_t)optin ? std::max(pb, cb) : pb;
-}
+// What a launch of k_chol32c for dimension d can use, found once per dimension and device (the
+// occupancy queries cost more than a small launch).
+struct C32Plan {
+    int res = 0;              // CTA 0 keeps the factor resident (when it fits beside the static shared memory)
+    size_t smem = 0;          // dynamic shared memory
+    int cap = 0;              // resident CTAs: the cooperative launch's upper bound
+    int slots = 0;            // blocks of 32 x 32 that the solves on clusters have room for
+    int two = 0;              // ... and need in the fullest CTA of two clusters of 16 (0: too many rows for a CTA)
+    std::map<int, int> clusters;     // resident clusters of n CTAs
+};
 
-// resident CTAs of k_chol32c for dimension d (the cooperative launch's upper bound)
-int chol32c_cap(int d)
+int chol32c_count_clusters(size_t smem, int n)
 {
-    int dev = 0, sms = 1, bps = 0, res = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const size_t smem = chol32c_smem(d, &res);
-    if (fednl_raise_dyn_smem((const void*)k_chol32c, smem) != cudaSuccess) return 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_chol32c, kCoopThreads, smem);
-    return std::min(sms, sms * bps);
-}
-
-// how many clusters of n CTAs of k_chol32c can be resident for dimension d
-int chol32c_clusters(int d, int n)
-{
-    static std::mutex mu;
-    static std::map<std::pair<int, int>, int> cache;
-    std::lock_guard<std::mutex> g(mu);
-    auto it = cache.find({d, n});
-    if (it != cache.end()) return it->second;
-    int clusters = 0, res = 0;
-    const size_t smem = chol32c_smem(d, &res);
-    if (fednl_raise_dyn_smem((const void*)k_chol32c, smem) == cudaSuccess &&
-        (n <= 8 || cudaFuncSetAttribute(k_chol32c, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess)) {
+    int clusters = 0;
+    if (n <= 8 || cudaFuncSetAttribute(k_chol32c, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(n);
         cfg.blockDim = dim3(kCoopThreads);
@@ -384,10 +351,52 @@ int chol32c_clusters(int d, int n)
         if (cudaOccupancyMaxActiveClusters(&clusters, k_chol32c, &cfg) != cudaSuccess) clusters = 0;
     }
     cudaGetLastError();
-    cache[{d, n}] = clusters;
     return clusters;
 }
-bool chol32c_cluster_ok(int d, int n) { return chol32c_clusters(d, n) >= 1; }
+
+// the plan for d, with the resident clusters of n CTAs counted (n > 0)
+C32Plan chol32c_plan(int d, int n)
+{
+    static std::mutex mu;
+    static std::map<std::pair<int, int>, C32Plan> cache;
+    std::lock_guard<std::mutex> g(mu);
+    int dev = 0;
+    cudaGetDevice(&dev);
+    C32Plan& p = cache[{dev, d}];
+    if (!p.smem) {
+        int optin = 0, sms = 1, bps = 0;
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        cudaFuncAttributes fa{};
+        cudaFuncGetAttributes(&fa, k_chol32c);
+        const size_t room = (size_t)optin - fa.sharedSizeBytes - 1024;
+        const size_t rb = c32c_smem_bytes(d, true);
+        p.res = (d + 31) / 32 <= kC32ResBlocks && rb <= room ? 1 : 0;
+        p.two = std::max(c32c_cluster_blocks(d, 16, true, false), c32c_cluster_blocks(d, 16, false, true));
+        // with room for the solves on two clusters of 16, where that fits
+        const size_t head = c32c_head_floats(d) - 1024, cb = (head + p.two * (size_t)1024) * 4;
+        const size_t smem = p.res ? rb : std::max(c32c_smem_bytes(d, false), cb <= room ? cb : 0);
+        p.slots = (int)((smem / 4 - head) / 1024);
+        if (fednl_raise_dyn_smem((const void*)k_chol32c, smem) != cudaSuccess) {
+            cudaGetLastError();
+            return C32Plan{};
+        }
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_chol32c, kCoopThreads, smem);
+        p.cap = std::min(sms, sms * bps);
+        p.smem = smem;
+    }
+    if (n > 0 && !p.clusters.count(n)) {
+        if (fednl_raise_dyn_smem((const void*)k_chol32c, p.smem) != cudaSuccess) cudaGetLastError();
+        p.clusters[n] = chol32c_count_clusters(p.smem, n);
+    }
+    return p;
+}
+
+// resident CTAs of k_chol32c for dimension d (the cooperative launch's upper bound)
+int chol32c_cap(int d) { return chol32c_plan(d, 0).cap; }
+
+// whether one cluster of n CTAs of k_chol32c can be resident for dimension d
+bool chol32c_cluster_ok(int d, int n) { return chol32c_plan(d, n).clusters[n] >= 1; }
 
 // default launch: one cluster of 16 CTAs while the trailing updates are small (d up to 512), else
 // one CTA per 32 x 32 tile of the first trailing update within the resident limit (a negative
@@ -428,28 +437,24 @@ int fednl_device_optionb_solve32(const FednlSolveDesc& S, const FednlSolve32& E,
     P.ls = S.ls;
     P.round_ctr = S.round_ctr;
     P.hist_cap = S.hist_cap;
-    int res = 0;
-    const size_t smem = chol32c_smem(S.d, &res);
-    const int cap = chol32c_cap(S.d);
-    if (cap < 1) return FEDNL_ECUDA;
     if (grid == 0) grid = chol32c_grid(S.d);
+    C32Plan plan = chol32c_plan(S.d, grid < 0 ? -grid : 16);
+    const size_t smem = plan.smem;
+    const int cap = plan.cap, res = plan.res;
+    if (cap < 1) return FEDNL_ECUDA;
+    CK(fednl_raise_dyn_smem((const void*)k_chol32c, smem));
     const bool cl = grid < 0;
-    if (cl && !chol32c_cluster_ok(S.d, -grid)) return FEDNL_EINVAL;
+    if (cl && plan.clusters[-grid] < 1) return FEDNL_EINVAL;
     grid = cl ? -grid : std::min(grid, cap);
     // The solves run on clusters when CTA 0 does not keep the factor and their blocks fit: on the one
     // cluster of the launch, or on two clusters of 16 of a cooperative grid
-    const int slots = ((int)(smem / 4) - (c32c_head_floats(S.d) - 1024)) / 1024;
     int ncl = 0;
     if (!res && cl) {
         const int need = c32c_cluster_blocks(S.d, grid, true, true);
-        if (need > 0 && need <= slots) ncl = grid;
-    } else if (!res && grid >= 32) {
-        const int need = std::max(c32c_cluster_blocks(S.d, 16, true, false), c32c_cluster_blocks(S.d, 16, false, true));
-        const int most = chol32c_clusters(S.d, 16);
-        if (need > 0 && need <= slots && most >= 2) {
-            ncl = 16;
-            grid = 16 * std::min(most, grid / 16);
-        }
+        if (need > 0 && need <= plan.slots) ncl = grid;
+    } else if (!res && grid >= 32 && plan.two > 0 && plan.two <= plan.slots && plan.clusters[16] >= 2) {
+        ncl = 16;
+        grid = 16 * std::min(plan.clusters[16], grid / 16);
     }
     Chol32c C{E.a,  E.diag0, E.linv, E.r,     E.acc,   E.accp, E.hh, E.hl,         E.rh,
               E.rl, E.flag,  c32c_ld(S.d), E.refine, E.tol, res,    (int)(smem / 4), cl ? 1 : 0, ncl};

@@ -202,6 +202,7 @@ int fednl_device_optionb_solve(const double* H, int d, const double* lptr, const
 struct fednl_mx_handle_s {
     fednl_problem_desc desc{};
     std::vector<int32_t> ns, soff;
+    bool margin_two = false;           // the margins take two samples a thread
     int d = 0, dp = 0, nc = 0, L = 0, U = 0, SW = 0, k = 0, S = 0, tiles = 0, comp = 0;
     long long Up = 0;
     cudaStream_t stream = nullptr;
@@ -282,6 +283,17 @@ FednlSolveDesc mx_solve_desc(fednl_mx_handle h)
     return S;
 }
 
+// Two samples a thread when blocks of 128 samples still cover the GPU three times (one sample / two, us:
+// d = 1024, 576 blocks 82 / 62, 216 blocks 41 / 41, 96 blocks 33 / 34; d = 301, 568 blocks 33 / 24, 304
+// blocks 17 / 16; d = 124, 320 blocks 12.3 / 13.9; d = 69, 96 blocks 9.2 / 8.6)
+void launch_margin(fednl_mx_handle h, const fednl_tc::MxDev& P, cudaStream_t st)
+{
+    const int per = h->margin_two ? 128 : 64;
+    const dim3 grid((h->L + per - 1) / per, h->nc), block(64, 4);
+    if (h->margin_two) fednl_tc::k_mx_margin<2><<<grid, block, 0, st>>>(P);
+    else fednl_tc::k_mx_margin<1><<<grid, block, 0, st>>>(P);
+}
+
 int mx_launch_round(fednl_mx_handle h, cudaEvent_t* ev = nullptr, bool client_phase_only = false)
 {
     using namespace fednl_tc;
@@ -309,13 +321,13 @@ int mx_launch_round(fednl_mx_handle h, cudaEvent_t* ev = nullptr, bool client_ph
     }
     k_mx_split_x<<<(h->d + 255) / 256, 256, 0, st>>>(P);
     mark();
-    k_mx_margin<<<dim3((h->L + 63) / 64, h->nc), dim3(64, 4), 0, st>>>(P);
+    launch_margin(h, P, st);
     mark();
     if (fork) {
         CKM(cudaEventRecord(h->ev_margin, st));
         CKM(cudaStreamWaitEvent(h->side, h->ev_margin, 0));
     }
-    k_mx_grad<<<(h->nc * h->d + 7) / 8, 256, 0, fork ? h->side : st>>>(P);
+    k_mx_grad<<<(h->nc * ((h->d + 1) / 2) + 7) / 8, 256, 0, fork ? h->side : st>>>(P);     // a warp per pair of features
     mark();
     if (randk) {
         if (fork) CKM(cudaStreamWaitEvent(st, h->ev_join, 0));
@@ -407,7 +419,10 @@ static int mx_create_impl(const fednl_problem_desc* desc, fednl_mx_handle* out, 
     h->tiles = (h->dp / fednl_tc::kBM) * (h->dp / fednl_tc::kBM + 1) / 2;
     h->ns.assign(D.n_samples, D.n_samples + D.n_clients);
     h->soff.assign(h->nc + 1, 0);
-    int maxn = 0;
+    int maxn = 0, dev = 0, sms = 1;
+    long long blocks = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     for (int c = 0; c < h->nc; ++c) {
         if (h->ns[c] < 1) {
             delete h;
@@ -415,7 +430,9 @@ static int mx_create_impl(const fednl_problem_desc* desc, fednl_mx_handle* out, 
         }
         h->soff[c + 1] = h->soff[c] + h->ns[c];
         maxn = std::max(maxn, h->ns[c]);
+        blocks += (h->ns[c] + 127) / 128;
     }
+    h->margin_two = blocks >= 3ll * sms;
     h->S = h->soff[h->nc];
     h->L = (maxn + 31) / 32 * 32;
     fednl_tc::MxDev& P = h->P;
@@ -639,7 +656,7 @@ int fednl_mx_init_shifts(fednl_mx_handle h, const double* x0)
     if (x0) CKM(cudaMemcpyAsync(P.x, x0, h->d * 8, cudaMemcpyHostToDevice, st));
     else CKM(cudaMemsetAsync(P.x, 0, h->d * 8, st));
     k_mx_split_x<<<(h->d + 255) / 256, 256, 0, st>>>(P);
-    k_mx_margin<<<dim3((h->L + 63) / 64, h->nc), dim3(64, 4), 0, st>>>(P);
+    launch_margin(h, P, st);
     GramJob J{h->dp, h->nc, h->L, h->dp / kBM, h->tiles, h->ns_dev, nullptr, P.Dw, h->err};
     EpiInitShift epi{P.shift, h->Up, (float)P.lambda, h->d};
     k_gram_tf32<EpiInitShift><<<h->nc * h->tiles, kThreads, smem_bytes(), st>>>(h->map, J, epi);

@@ -160,8 +160,9 @@ __device__ __forceinline__ void upper_tile(int t, int nb, int& mi, int& ni)
     ni = i + rem;
 }
 
-// Epilogue functor: operator()(client, row m, first column n0, 16 FP32 values, acc) for every row
-// of the tile (called by the 128 epilogue threads, 8 times each, acc a per-thread Epi::Acc), then
+// Epilogue functor: load(client, row m, first column n0, pre) fetches what operator()(client, row m, first
+// column n0, 16 FP32 values, pre, acc) needs, for every row of the tile (called by the 128 epilogue
+// threads, 8 times each, acc a per-thread Epi::Acc), then
 // finish(client, tile, thread 0..127, acc).
 template <class Epi>
 __global__ void __launch_bounds__(kThreads) k_gram_tf32(const __grid_constant__ CUtensorMap tmX, GramJob J, Epi epi)
@@ -269,18 +270,29 @@ __global__ void __launch_bounds__(kThreads) k_gram_tf32(const __grid_constant__ 
             mbar_arrive(&scaled[s]);
             wv = wn;
         }
-        // epilogue: the accumulator rows of this warp's TMEM lane quarter
+        // Epilogue: the accumulator rows of this warp's TMEM lane quarter, 16 columns at a time.  What the
+        // functor reads from memory is loaded two chunks ahead, the first two while the last MMAs run: a
+        // chunk's loads otherwise cost their latency eight times a tile (w8a-like, 3 x 3 tiles of 6 to 19
+        // slabs: 96 us, of which 57 the epilogue; with the loads ahead and the chunks told apart, see EpiDiff, 58; d = 1024: 290 -> 256).
+        const int quarter = warp & 3;
+        const int m = mi * kBM + quarter * 32 + lane;
+        typename Epi::Pre pre[2];
+        epi.load(c, m, ni * kBN, pre[0]);
+        epi.load(c, m, ni * kBN + 16, pre[1]);
         const bool ok = __all_sync(0xffffffffu, mbar_wait(done, 0u, abort_flag));   // warp-uniform for tcgen05.ld
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (ok) {
-            const int quarter = warp & 3;
-            const int m = mi * kBM + quarter * 32 + lane;
             typename Epi::Acc acc{};
 #pragma unroll 1
-            for (int j = 0; j < kBN / 16; ++j) {
-                float v[16];
-                tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(j * 16), v);
-                epi(c, m, ni * kBN + j * 16, v, acc);
+            for (int j = 0; j < kBN / 16; j += 2) {
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const int n0 = ni * kBN + (j + u) * 16;
+                    float v[16];
+                    tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((j + u) * 16), v);
+                    epi(c, m, n0, v, pre[u], acc);
+                    if (j + 2 < kBN / 16) epi.load(c, m, n0 + 32, pre[u]);
+                }
             }
             epi.finish(c, t, quarter * 32 + lane, acc);
         }
@@ -305,10 +317,12 @@ __global__ void __launch_bounds__(kThreads) k_gram_tf32(const __grid_constant__ 
 // matrix per client: out[c][m][n]
 struct EpiStore {
     struct Acc {};
+    struct Pre {};
     float* out;
     int d;
     float lambda;
-    __device__ __forceinline__ void operator()(int c, int m, int n0, const float* v, Acc&) const
+    __device__ __forceinline__ void load(int, int, int, Pre&) const {}
+    __device__ __forceinline__ void operator()(int c, int m, int n0, const float* v, const Pre&, Acc&) const
     {
         float* row = out + ((size_t)c * d + m) * d + n0;
 #pragma unroll
@@ -324,11 +338,13 @@ __device__ __forceinline__ long long upos(int m, int n) { return (long long)n * 
 // rows m, so for each column n they touch consecutive packed positions)
 struct EpiInitShift {
     struct Acc {};
+    struct Pre {};
     float* shift;          // [nc][Up]
     long long Up;
     float lambda;
     int d;                 // true dimension (rows and columns from d on are padding)
-    __device__ __forceinline__ void operator()(int c, int m, int n0, const float* v, Acc&) const
+    __device__ __forceinline__ void load(int, int, int, Pre&) const {}
+    __device__ __forceinline__ void operator()(int c, int m, int n0, const float* v, const Pre&, Acc&) const
     {
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
@@ -347,6 +363,10 @@ struct EpiDiff {
     struct Acc {
         float sq = 0.0f;
     };
+    struct Pre {           // shift values and selection words of 16 columns
+        float sh[16];
+        unsigned sw[16];
+    };
     const float* shift;    // [nc][Up]
     float* dsel;           // [nc][Up]
     const unsigned* sel;   // [nc][SW] or nullptr
@@ -355,31 +375,66 @@ struct EpiDiff {
     int SW, tiles;
     float lambda;
     int d;
-    __device__ __forceinline__ void operator()(int c, int m, int n0, const float* v, Acc& a) const
+    // A warp's 32 rows against 16 columns: nothing of the upper triangle (kNone), all of it and off the
+    // diagonal (kFull), or a part.  A lone warp issues an instruction every few cycles, so what bounds the
+    // epilogue is its instructions: whole chunks run without a test or a branch per value, and chunks
+    // outside of the triangle (d = 301 padded to 384: five of eight in the last tile column) are left out.
+    enum Kind { kNone, kPart, kFull };
+    __device__ __forceinline__ Kind kind(int m, int n0) const
     {
-        // all 16 shift values and selection words are loaded before the first store, so that the
-        // loads overlap instead of waiting one by one behind the stores to dsel
+        const int lo = m & ~31;
+        return n0 >= d || n0 + 15 < lo ? kNone : lo + 31 < n0 && n0 + 16 <= d ? kFull : kPart;
+    }
+    __device__ __forceinline__ void load(int c, int m, int n0, Pre& r) const
+    {
+        const Kind kd = kind(m, n0);
+        if (kd == kNone) return;
         const unsigned* sc = sel ? sel + (size_t)c * SW : nullptr;
         const float* shc = shift + (size_t)c * Up;
-        float sh[16];
-        unsigned sw[16];
+        int p = (int)upos(m, n0);                 // positions of a column's rows are consecutive
+        if (kd == kFull) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                r.sh[i] = __ldg(shc + p);
+                if (sc) r.sw[i] = __ldg(sc + (p >> 5));
+                p += n0 + i + 1;
+            }
+            return;
+        }
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
             const int n = n0 + i;
             const bool ok = m <= n && n < d;
-            const long long p = ok ? upos(m, n) : 0;
-            sh[i] = ok ? __ldg(shc + p) : 0.0f;
-            sw[i] = (ok && sc) ? __ldg(sc + (p >> 5)) : 0xffffffffu;
+            r.sh[i] = ok ? __ldg(shc + p) : 0.0f;
+            r.sw[i] = (ok && sc) ? __ldg(sc + (p >> 5)) : 0xffffffffu;
+            p += n + 1;
+        }
+    }
+    __device__ __forceinline__ void operator()(int c, int m, int n0, const float* v, const Pre& r, Acc& a) const
+    {
+        const Kind kd = kind(m, n0);
+        if (kd == kNone) return;
+        float* out = dsel + (size_t)c * Up;
+        int p = (int)upos(m, n0);
+        if (kd == kFull) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const float df = v[i] - r.sh[i];
+                a.sq = fmaf(2.0f * df, df, a.sq);
+                if (!sel || ((r.sw[i] >> (p & 31)) & 1u)) out[p] = df;
+                p += n0 + i + 1;
+            }
+            return;
         }
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
             const int n = n0 + i;
             if (m <= n && n < d) {
-                const long long p = upos(m, n);
-                const float df = (v[i] + (m == n ? lambda : 0.0f)) - sh[i];
+                const float df = (v[i] + (m == n ? lambda : 0.0f)) - r.sh[i];
                 a.sq = fmaf(m == n ? df : 2.0f * df, df, a.sq);
-                if ((sw[i] >> (p & 31)) & 1u) dsel[(size_t)c * Up + p] = df;
+                if ((r.sw[i] >> (p & 31)) & 1u) out[p] = df;
             }
+            p += n + 1;
         }
     }
     __device__ __forceinline__ void finish(int c, int t, int th, const Acc& a) const
@@ -456,110 +511,172 @@ __global__ void k_mx_split_x(MxDev P)
 // margin m_s = b_s a_s^T x, sigmoid (FP64), D_s (Gram weight, FP32) and b_s q_s (FP32 pair)
 __device__ __forceinline__ double mx_sigmoid(double m) { return 1.0 / (1.0 + exp(-m)); }
 
-// A block covers 64 samples; its four warp rows split each sample's features in quarters (eight
-// loads in flight each, two float-float accumulators), and the quarters are added in order.
+// A block covers 64 NS samples, NS per thread; its four warp rows split each sample's features in quarters
+// (eight loads in flight each, two float-float accumulators), and the quarters are added in order.  The
+// kernel is bound by issued instructions (12 of a float-float product per feature): two samples a thread
+// share the iterate's reads and halve the loads (d = 1024, 73728 samples: 92 -> 61 us; d = 301,
+// 56800 samples: 34 -> 25), as long as the blocks still fill the GPU (margin_two).
+template <int NS>
 __global__ void __launch_bounds__(256) k_mx_margin(MxDev P)
 {
-    __shared__ float s_xh[1024], s_xl[1024];
-    __shared__ float s_ph[4][64], s_pl[4][64];
+    __shared__ float2 s_x[1024];                  // the iterate's pairs
+    __shared__ float s_ph[4][64 * NS], s_pl[4][64 * NS];
+    __shared__ double s_inv;
     const int c = blockIdx.y, sx = threadIdx.x, q = threadIdx.y;
     const int tid = q * 64 + sx;
-    for (int i = tid; i < P.d && i < 1024; i += 256) {
-        s_xh[i] = P.xh[i];
-        s_xl[i] = P.xl[i];
-    }
-    __syncthreads();
     const int n = P.ns[c];
-    const int s = blockIdx.x * 64 + sx;
+    const int s0 = blockIdx.x * 64 * NS;
+    if (s0 >= n) return;
+    for (int i = tid; i < P.d && i < 1024; i += 256) s_x[i] = make_float2(P.xh[i], P.xl[i]);
+    if (tid == 0) s_inv = 1.0 / (double)n;        // one FP64 division per block
+    __syncthreads();
+    const int s = s0 + sx * NS;
     const int per = (P.d + 3) / 4, i0 = q * per, i1 = min(P.d, i0 + per);
-    float h0 = 0.0f, l0 = 0.0f, h1 = 0.0f, l1 = 0.0f;
-    if (s < n) {
+    float h0[NS], l0[NS], h1[NS], l1[NS];
+#pragma unroll
+    for (int t = 0; t < NS; ++t) h0[t] = l0[t] = h1[t] = l1[t] = 0.0f;
+    if (s < n) {                                  // (a second sample past n is padding, not used)
         const float* col = P.X + (size_t)c * P.dp * P.L + s;
+        auto load = [&](int i, float* x) {
+            const float* p = col + (size_t)i * P.L;
+            if constexpr (NS == 2) {
+                const float2 t = __ldg(reinterpret_cast<const float2*>(p));     // s and L are even
+                x[0] = t.x;
+                x[1] = t.y;
+            } else {
+                x[0] = __ldg(p);
+            }
+        };
+        auto pair = [&](int i) { return i < 1024 ? s_x[i] : make_float2(P.xh[i], P.xl[i]); };
         int i = i0;
         for (; i + 8 <= i1; i += 8) {
-            float xv[8];
+            float xv[8][NS];
+            float2 y[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) xv[u] = __ldg(col + (size_t)(i + u) * P.L);
+            for (int u = 0; u < 8; ++u) load(i + u, xv[u]);
+            if (i + 8 <= 1024) {
 #pragma unroll
-            for (int u = 0; u < 8; u += 2) {
-                const float yh0 = i + u < 1024 ? s_xh[i + u] : P.xh[i + u];
-                const float yl0 = i + u < 1024 ? s_xl[i + u] : P.xl[i + u];
-                const float yh1 = i + u + 1 < 1024 ? s_xh[i + u + 1] : P.xh[i + u + 1];
-                const float yl1 = i + u + 1 < 1024 ? s_xl[i + u + 1] : P.xl[i + u + 1];
-                ff_mac(h0, l0, xv[u], yh0, yl0);
-                ff_mac(h1, l1, xv[u + 1], yh1, yl1);
+                for (int u = 0; u < 8; ++u) y[u] = s_x[i + u];
+            } else {
+#pragma unroll
+                for (int u = 0; u < 8; ++u) y[u] = pair(i + u);
             }
+#pragma unroll
+            for (int u = 0; u < 8; u += 2)
+#pragma unroll
+                for (int t = 0; t < NS; ++t) {
+                    ff_mac(h0[t], l0[t], xv[u][t], y[u].x, y[u].y);
+                    ff_mac(h1[t], l1[t], xv[u + 1][t], y[u + 1].x, y[u + 1].y);
+                }
         }
         for (; i < i1; ++i) {
-            const float yh = i < 1024 ? s_xh[i] : P.xh[i], yl = i < 1024 ? s_xl[i] : P.xl[i];
-            ff_mac(h0, l0, __ldg(col + (size_t)i * P.L), yh, yl);
-        }
-        ff_add(h0, l0, h1, l1);
-    }
-    s_ph[q][sx] = h0;
-    s_pl[q][sx] = l0;
-    __syncthreads();
-    if (q != 0 || s >= n) return;
-    float hi = s_ph[0][sx], lo = s_pl[0][sx];
+            float xv[NS];
+            load(i, xv);
+            const float2 y = pair(i);
 #pragma unroll
-    for (int t = 1; t < 4; ++t) ff_add(hi, lo, s_ph[t][sx], s_pl[t][sx]);
-    const double b = P.lab[(size_t)c * P.L + s];
+            for (int t = 0; t < NS; ++t) ff_mac(h0[t], l0[t], xv[t], y.x, y.y);
+        }
+#pragma unroll
+        for (int t = 0; t < NS; ++t) ff_add(h0[t], l0[t], h1[t], l1[t]);
+    }
+#pragma unroll
+    for (int t = 0; t < NS; ++t) {
+        s_ph[q][sx * NS + t] = h0[t];
+        s_pl[q][sx * NS + t] = l0[t];
+    }
+    __syncthreads();
+    if (tid >= 64 * NS || s0 + tid >= n) return;
+    float hi = s_ph[0][tid], lo = s_pl[0][tid];
+#pragma unroll
+    for (int t = 1; t < 4; ++t) ff_add(hi, lo, s_ph[t][tid], s_pl[t][tid]);
+    const size_t o = (size_t)c * P.L + s0 + tid;
+    const double b = P.lab[o];
     const double m = b * ((double)hi + (double)lo);
     const double sig = mx_sigmoid(m);
-    const double inv_n = 1.0 / (double)n;
+    const double inv_n = s_inv;
     const double z1 = 1.0 - sig;
-    P.Dw[(size_t)c * P.L + s] = (float)(inv_n * (z1 * sig));
+    P.Dw[o] = (float)(inv_n * (z1 * sig));
     const double qv = b * (z1 * -inv_n);
-    split_ff(qv, P.qh[(size_t)c * P.L + s], P.ql[(size_t)c * P.L + s]);
+    split_ff(qv, P.qh[o], P.ql[o]);
 }
 
-// client gradients: one warp per (client, feature), lanes over the samples (eight in flight, the
-// last pass masked).  The warp reduces in float-float; eight lanes of the block then form the FP64
-// sums of its eight features, so the FP64 pipe sees one conversion and add per block, not per warp.
+// client gradients: one warp per (client, pair of features), lanes over the samples (eight in flight).  The
+// warp reduces in float-float; sixteen lanes of the block then form the FP64 sums of its features, so the
+// FP64 pipe sees one conversion and add per block, not per warp.  Bound by issued instructions: two
+// features share the weights' loads, whole batches carry no masks and the steps of 32 samples past the
+// client's last are left out (d = 1024, 73728 samples:
+// 69 -> 68 us; d = 301, 56800 samples: 29 -> 25).
 __global__ void __launch_bounds__(256) k_mx_grad(MxDev P)
 {
-    __shared__ float s_h[8], s_l[8];
+    __shared__ float s_h[16], s_l[16];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int wid = blockIdx.x * 8 + w, total = P.nc * P.d;
-    float hi = 0.0f, lo = 0.0f;
+    const int ppc = (P.d + 1) >> 1;                              // pairs per client
+    const int wid = blockIdx.x * 8 + w, total = P.nc * ppc;
+    float h[2][2] = {}, l[2][2] = {};                            // [feature][even or odd step]
     if (wid < total) {
-        const int c = wid / P.d, i = wid - c * P.d;
+        const int c = wid / ppc, i = 2 * (wid - c * ppc);
         const int n = P.ns[c];
-        const float* row = P.X + ((size_t)c * P.dp + i) * P.L;
+        const float* row0 = P.X + ((size_t)c * P.dp + i) * P.L;
+        const float* row1 = i + 1 < P.d ? row0 + P.L : row0;
         const float* qh = P.qh + (size_t)c * P.L;
         const float* ql = P.ql + (size_t)c * P.L;
-        float h1 = 0.0f, l1 = 0.0f;
-        for (int s = lane; s < n; s += 256) {
-            float x[8], a[8], b[8];
+        int s = 0;
+        for (; s + 256 <= n; s += 256) {
+            float x0[8], x1[8], a[8], b[8];
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
-                const int t = s + 32 * u;
+                const int t = s + 32 * u + lane;
+                x0[u] = __ldg(row0 + t);
+                x1[u] = __ldg(row1 + t);
+                a[u] = __ldg(qh + t);
+                b[u] = __ldg(ql + t);
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                ff_mac(h[0][u & 1], l[0][u & 1], x0[u], a[u], b[u]);
+                ff_mac(h[1][u & 1], l[1][u & 1], x1[u], a[u], b[u]);
+            }
+        }
+        if (s < n) {
+            float x0[8], x1[8], a[8], b[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int t = s + 32 * u + lane;
                 const bool in = t < n;
-                x[u] = in ? __ldg(row + t) : 0.0f;
+                x0[u] = in ? __ldg(row0 + t) : 0.0f;
+                x1[u] = in ? __ldg(row1 + t) : 0.0f;
                 a[u] = in ? __ldg(qh + t) : 0.0f;
                 b[u] = in ? __ldg(ql + t) : 0.0f;
             }
 #pragma unroll
-            for (int u = 0; u < 8; u += 2) {
-                ff_mac(hi, lo, x[u], a[u], b[u]);
-                ff_mac(h1, l1, x[u + 1], a[u + 1], b[u + 1]);
+            for (int u = 0; u < 8; ++u)
+                if (s + 32 * u < n) {
+                    ff_mac(h[0][u & 1], l[0][u & 1], x0[u], a[u], b[u]);
+                    ff_mac(h[1][u & 1], l[1][u & 1], x1[u], a[u], b[u]);
+                }
+        }
+#pragma unroll
+        for (int f = 0; f < 2; ++f) ff_add(h[f][0], l[f][0], h[f][1], l[f][1]);
+        for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+            for (int f = 0; f < 2; ++f) {
+                const float oh = __shfl_xor_sync(0xffffffffu, h[f][0], o), ol = __shfl_xor_sync(0xffffffffu, l[f][0], o);
+                ff_add(h[f][0], l[f][0], oh, ol);
             }
         }
-        ff_add(hi, lo, h1, l1);
-        for (int o = 16; o > 0; o >>= 1) {
-            const float oh = __shfl_xor_sync(0xffffffffu, hi, o), ol = __shfl_xor_sync(0xffffffffu, lo, o);
-            ff_add(hi, lo, oh, ol);
+    }
+    if (lane == 0) {                             // (the lanes' low parts differ in rounding)
+#pragma unroll
+        for (int f = 0; f < 2; ++f) {
+            s_h[2 * w + f] = h[f][0];
+            s_l[2 * w + f] = l[f][0];
         }
     }
-    if (lane == 0) {
-        s_h[w] = hi;
-        s_l[w] = lo;
-    }
     __syncthreads();
-    const int t = blockIdx.x * 8 + threadIdx.x;
-    if (threadIdx.x < 8 && t < total) {
-        const int c = t / P.d, i = t - c * P.d;
-        P.gc[(size_t)c * P.d + i] = ((double)s_h[threadIdx.x] + (double)s_l[threadIdx.x]) + P.lambda * P.x[i];
+    const int t = blockIdx.x * 8 + (threadIdx.x >> 1);
+    if (threadIdx.x < 16 && t < total) {
+        const int c = t / ppc, i = 2 * (t - c * ppc) + (threadIdx.x & 1);
+        if (i < P.d) P.gc[(size_t)c * P.d + i] = ((double)s_h[threadIdx.x] + (double)s_l[threadIdx.x]) + P.lambda * P.x[i];
     }
 }
 
@@ -647,16 +764,29 @@ __device__ __forceinline__ bool packed_is_diag(long long p)
     return p - j * (j + 1) / 2 == j;
 }
 
-// TopLEK's term of a kept-set entry (key << 32 | ~position) in fixed point: c v^2 2^sh (c = 1 on the
-// diagonal, 2 off it) for the FP32 magnitude v = m 2^(eb - 150) (biased exponent eb, significand m),
+// A kept-set entry is diagonal << 63 | key << 32 | ~position (keys have 31 bits).
+constexpr unsigned long long kSetDiag = 1ull << 63;
+__device__ __forceinline__ unsigned set_key(unsigned long long e) { return (unsigned)(e >> 32) & 0x7fffffffu; }
+
+// sum += v for a 64-bit sum in shared memory as two native 32-bit atomics, the low word's carry going to the
+// high one (a 64-bit shared atomicAdd is a compare-and-swap loop: over the few bins that the kept entries
+// share, 2408 of them took 37k cycles)
+__device__ __forceinline__ void add_u64(unsigned long long* sum, unsigned long long v)
+{
+    unsigned* w = reinterpret_cast<unsigned*>(sum);
+    const unsigned lo = (unsigned)v;
+    const unsigned old = atomicAdd(w, lo);
+    atomicAdd(w + 1, (unsigned)(v >> 32) + (old + lo < old ? 1u : 0u));
+}
+
+// TopLEK's term of a kept-set entry in fixed point: c v^2 2^sh (c = 1 on the diagonal, 2 off it) for the FP32 magnitude v = m 2^(eb - 150) (biased exponent eb, significand m),
 // i.e. m^2 2^(2 eb - 300 + sh), exact where the shift is not negative
 __device__ __forceinline__ unsigned long long lek_fixed(unsigned long long e, int sh)
 {
-    const unsigned key = (unsigned)(e >> 32);
+    const unsigned key = set_key(e);
     const int eb = (int)(key >> 23);
     const unsigned long long m = eb ? (unsigned long long)((key & 0x7fffffu) | 0x800000u) : (unsigned long long)(key & 0x7fffffu);
-    const long long q = (long long)(0xffffffffu - (unsigned)(e & 0xffffffffu));
-    const int s = 2 * (eb ? eb : 1) - 300 + sh + (packed_is_diag(q) ? 0 : 1);
+    const int s = 2 * (eb ? eb : 1) - 300 + sh + (e & kSetDiag ? 0 : 1);
     const unsigned long long m2 = m * m;
     return s >= 0 ? m2 << s : (s > -64 ? m2 >> -s : 0ull);
 }
@@ -689,7 +819,10 @@ __device__ __forceinline__ unsigned long long block_scan_u64(unsigned long long 
     return r;
 }
 
-// one CTA (1024 threads) per client: selection bitmap sel[c] from the differences dsel[c]
+// one CTA (1024 threads) per client: selection bitmap sel[c] from the differences dsel[c].  Its passes over
+// the differences are bound by the latency of their loads and by atomics on shared bins: eight loads in
+// flight per thread, the ties at the threshold only ordered where not all are kept, the kept entries'
+// values gathered by a thread per entry (d = 301, k = 8d, 142 clients: 74 -> 49 us).
 __global__ void __launch_bounds__(kSelThreads) k_mx_select(MxDev P, int k, int toplek, unsigned seed)
 {
     extern __shared__ unsigned long long s_set[];       // TopLEK: [max(Kp, 1024)] entries, [2048] masses
@@ -700,7 +833,7 @@ __global__ void __launch_bounds__(kSelThreads) k_mx_select(MxDev P, int k, int t
     __shared__ double s_win[3];                 // TopLEK: F, (1 - k/U) F, F/10
     __shared__ unsigned long long s_rx, s_above;
     __shared__ unsigned s_bin, s_need, s_cnt[32], s_nk, s_kmax, s_qstar;
-    __shared__ int s_istar;
+    __shared__ int s_istar, s_all;
     const int c = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int U = P.U;
     const float* v = P.dsel + (size_t)c * P.Up;
@@ -716,9 +849,17 @@ __global__ void __launch_bounds__(kSelThreads) k_mx_select(MxDev P, int k, int t
             const int sh = shs[pass], nb = 1 << nbits[pass];
             for (int b = tid; b < 2048; b += kSelThreads) hist[b] = 0u;
             __syncthreads();
-            for (int q = tid; q < U; q += kSelThreads) {
-                const unsigned key = mag_key(v[q]);
-                if ((key & mask) == prefix) atomicAdd(&hist[(key >> sh) & (unsigned)(nb - 1)], 1u);
+            for (int q0 = tid; q0 < U; q0 += 8 * kSelThreads) {
+                unsigned key[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const int q = q0 + u * kSelThreads;
+                    key[u] = q < U ? mag_key(v[q]) : 0xffffffffu;        // (no key has bit 31)
+                }
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if (key[u] != 0xffffffffu && (key[u] & mask) == prefix)
+                        atomicAdd(&hist[(key[u] >> sh) & (unsigned)(nb - 1)], 1u);
             }
             __syncthreads();
             // thread t owns bins nb-1-2t and nb-2-2t (descending keys)
@@ -730,9 +871,11 @@ __global__ void __launch_bounds__(kSelThreads) k_mx_select(MxDev P, int k, int t
                 if (excl + h0 >= need) {
                     s_bin = (unsigned)b0;
                     s_need = need - excl;
+                    s_all = h0 == need - excl;
                 } else {
                     s_bin = (unsigned)b1;
                     s_need = need - excl - h0;
+                    s_all = h1 == need - excl - h0;
                 }
             }
             __syncthreads();
@@ -744,13 +887,15 @@ __global__ void __launch_bounds__(kSelThreads) k_mx_select(MxDev P, int k, int t
         T = prefix;
     }
     // bitmap in position order: keys above T, and the first `need` keys equal to T.  Warp w owns a
-    // contiguous range of selection words (lane = bit); pass 1 counts its keys equal to T, one block
-    // scan orders the warps, pass 2 forms the words (loads of eight words in flight in each pass).
+    // contiguous range of selection words (lane = bit); unless all keys equal to T are kept, pass 1
+    // counts them, one block scan orders the warps; pass 2 forms the words (loads of eight words in
+    // flight in each pass).
     {
+        const bool all = K >= U || s_all != 0;      // (s_all of the last radix pass: the keys equal to T)
         const int SWn = (U + 31) >> 5, wpw = (SWn + 31) >> 5;
         const int w0 = warp * wpw, w1 = min(SWn, w0 + wpw);
         unsigned neq = 0;
-        for (int wd = w0; wd < w1; wd += 8) {
+        for (int wd = w0; wd < w1 && !all; wd += 8) {
             unsigned key[8];
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
@@ -763,7 +908,7 @@ __global__ void __launch_bounds__(kSelThreads) k_mx_select(MxDev P, int k, int t
         if (lane == 0) s_cnt[warp] = neq;
         __syncthreads();
         unsigned carry = 0;
-        for (int w = 0; w < warp; ++w) carry += s_cnt[w];
+        for (int w = 0; w < warp && !all; ++w) carry += s_cnt[w];
         for (int wd = w0; wd < w1; wd += 8) {
             unsigned key[8];
 #pragma unroll
@@ -816,18 +961,23 @@ __global__ void __launch_bounds__(kSelThreads) k_mx_select(MxDev P, int k, int t
                 const int b = __ffs(wd) - 1;
                 wd &= wd - 1u;
                 const unsigned q = (unsigned)w * 32u + (unsigned)b;
-                if (slot < (unsigned)Kp)
-                    s_set[slot] = ((unsigned long long)mag_key(v[q]) << 32) | (unsigned long long)(0xffffffffu - q);
+                if (slot < (unsigned)Kp) s_set[slot] = q;
                 ++slot;
             }
             base_cnt += tot;
         }
     }
     __syncthreads();
-    // the fixed-point scale from the largest key; F from the Gram epilogue's partial sums
+    // their values; the fixed-point scale from the largest key; F from the Gram epilogue's partial sums
     {
         unsigned km = 0u;
-        for (int m = tid; m < K; m += kSelThreads) km = max(km, (unsigned)(s_set[m] >> 32));
+#pragma unroll 4
+        for (int m = tid; m < K; m += kSelThreads) {
+            const unsigned q = (unsigned)s_set[m], key = mag_key(v[q]);
+            s_set[m] = (packed_is_diag(q) ? kSetDiag : 0ull) | (unsigned long long)key << 32 |
+                       (unsigned long long)(0xffffffffu - q);
+            km = max(km, key);
+        }
         km = __reduce_max_sync(0xffffffffu, km);
         if (lane == 0) atomicMax(&s_kmax, km);
     }
@@ -876,11 +1026,11 @@ __global__ void __launch_bounds__(kSelThreads) k_mx_select(MxDev P, int k, int t
             __syncthreads();
             for (int m = tid; m < K; m += kSelThreads) {
                 const unsigned long long e = s_set[m];
-                const unsigned key = (unsigned)(e >> 32);
+                const unsigned key = set_key(e);
                 if ((key & mask) == prefix) {
                     const unsigned b = (key >> sb) & (unsigned)(nb - 1);
                     atomicAdd(&hist[b], 1u);
-                    atomicAdd(&s_mass[b], lek_fixed(e, sh));
+                    add_u64(&s_mass[b], lek_fixed(e, sh));
                 }
             }
             __syncthreads();
@@ -918,7 +1068,7 @@ __global__ void __launch_bounds__(kSelThreads) k_mx_select(MxDev P, int k, int t
         unsigned tn = 0u;
         for (int m = m0; m < m0 + per && m < K; ++m) {
             const unsigned long long e = s_set[m];
-            if ((unsigned)(e >> 32) == prefix) {
+            if (set_key(e) == prefix) {
                 tm += lek_fixed(e, sh);
                 ++tn;
             }
@@ -929,7 +1079,7 @@ __global__ void __launch_bounds__(kSelThreads) k_mx_select(MxDev P, int k, int t
         unsigned idx = tni - tn;
         for (int m = m0; m < m0 + per && m < K; ++m) {
             const unsigned long long e = s_set[m];
-            if ((unsigned)(e >> 32) != prefix) continue;
+            if (set_key(e) != prefix) continue;
             const unsigned long long w = lek_fixed(e, sh);
             if (cum < rrem && rrem <= cum + w) {      // the boundary entry: j* = above_n + idx
                 const double scale = ldexp(1.0, -sh);
@@ -957,7 +1107,7 @@ __global__ void __launch_bounds__(kSelThreads) k_mx_select(MxDev P, int k, int t
         __syncthreads();
         for (int m = tid; m < K; m += kSelThreads) {
             const unsigned long long e = s_set[m];
-            const unsigned key = (unsigned)(e >> 32), q = 0xffffffffu - (unsigned)(e & 0xffffffffu);
+            const unsigned key = set_key(e), q = 0xffffffffu - (unsigned)(e & 0xffffffffu);
             if (key > kap || (key == kap && (q < qs || (inc && q == qs)))) atomicOr(&sc[q >> 5], 1u << (q & 31));
         }
     } else {
