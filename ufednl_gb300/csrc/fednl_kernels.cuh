@@ -2418,6 +2418,118 @@ struct GridSync {
     }
 };
 
+// ---- back substitution of the cooperative solve ----------------------------------------------------
+// Blocks of 32 rows from the bottom, a warp each (lane = row), kBackWarps consecutive blocks to a CTA.  A warp
+// takes the solutions y_t of the blocks below in descending t, v_i -= L_ti y_t, as they appear, and then
+// solves its own triangle, so that the chain is one shuffle and one FP64 operation per row (120 cycles in
+// a warp alone) and all other updates run beside it.  The SM's FP64 unit takes a warp's operation every 19
+// cycles, so kBackWarps warps keep pace (2 or 3 of them: the same within 5%).  Within a CTA y_t goes through shared memory (s_back), to
+// other CTAs through global memory (ybuf), read eight at a time; an entry holds kNotYet, a NaN that no
+// operation returns, until it is known, so that no flag or fence is on the chain.  Every wait is bounded.
+// With one warp solving and the others of one CTA updating all rows above, the back substitution took
+// 82k of 430k cycles at d = 301, 156k of 806k at 512 and 483k of 2492k at 1024; now 56k, 92k
+// and 186k (148 cycles a row of a triangle, a block's hand-over 370 within a CTA and 2.4k between CTAs).
+constexpr int kBackWarps = 4;
+constexpr int kBackStep = 4;                    // rows of a triangle between branches
+constexpr int kBackSpins = 1 << 25;               // about 100 cycles each, 2 s
+constexpr long long kNotYet = 0xfff8dead5eedbeefll;
+
+__device__ __forceinline__ bool is_not_yet(double v) { return __double2hiint(v) == (int)(kNotYet >> 32); }
+
+// `own`: the warp's block (0 is the bottom one); blocks from `first` on are this CTA's; false: a wait ran out
+__device__ __forceinline__ bool back_block(const double* A, int d, int own, int first,
+                                           double (*s_back)[32], volatile double* s_far, double* ybuf, double* dxout,
+                                           double* xupd)
+{
+    const int lane = threadIdx.x & 31;
+    const int b1 = d - 32 * own, b0 = max(0, b1 - 32), nbk = b1 - b0, row = b0 + lane;
+    const bool mine = lane < nbk;
+    // Entry (row, c0 + s) of block q's columns [c0, c0 + 32).  Lanes past the block and, in the own block,
+    // entries below the diagonal read other entries of A, which no kept value takes; columns past d - 1
+    // (a single block of fewer than 32 rows) are not read.
+    const double* Ar = A + (mine ? row : b0);
+    double v = mine ? Ar[(size_t)d * (d + 1) / 2] : 0.0;           // 0 on the lanes past the block
+    const double x = mine && xupd ? xupd[row] : 0.0;
+    double cur[32];
+    auto first_col = [&](int q) { return max(0, d - 32 * (q + 1)); };
+#pragma unroll
+    for (int s = 31; s >= 0; --s) cur[s] = first_col(0) + s < d ? Ar[up_pos(0, first_col(0) + s)] : 0.0;
+    bool ok = true;
+    auto remote = [&](int q) {                    // lane's value of another CTA's block, or kNotYet
+        double y;
+        asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=d"(y) : "l"(ybuf + first_col(q) + lane) : "memory");
+        return y;
+    };
+    double y = own > 0 && first > 0 ? remote(0) : 0.0;
+#pragma unroll 1
+    for (int q = 0; q < own; ++q) {
+        const bool far = q < first;
+        const volatile double* from = far ? s_far : s_back[q - first];
+        const int nc = first_col(q + 1);
+        const double* next = Ar + up_pos(0, nc + 31);
+#pragma unroll
+        for (int c = 24; c >= 0; c -= 8) {
+            if (far) {                            // eight values to the warp's own shared memory
+                for (int spin = 0; (__ballot_sync(0xffffffffu, !is_not_yet(y)) >> c & 255u) != 255u && ok; ++spin) {
+                    y = remote(q);
+                    ok = spin < kBackSpins;
+                }
+                s_far[lane] = y;
+                __syncwarp();
+                if (c) y = remote(q);
+                else if (q + 1 < first) y = remote(q + 1);
+            }
+            if (!far && q + 1 < own)              // only the next block's warp keeps pace value by value: all of
+                                                  // them at once would queue before the solving warp
+                for (int spin = 0; is_not_yet(from[c]) && ok; ++spin) ok = spin < kBackSpins;
+#pragma unroll
+            for (int s = c + 7; s >= c; --s) {
+                double t = from[s];
+                for (int spin = 0; is_not_yet(t) && ok; ++spin) {
+                    t = from[s];
+                    ok = spin < kBackSpins;
+                }
+                v = fma(-cur[s], t, v);
+                cur[s] = *next;                   // of the next block, beside the operations
+                next -= nc + s;
+            }
+            if (far) __syncwarp();
+        }
+    }
+    // the triangle; every lane stores the broadcast y_t for the CTA's other warps (a store by one lane is a
+    // divergent branch on the chain), and eight lanes at a time their own for other CTAs
+    const uint32_t near = (uint32_t)__cvta_generic_to_shared(&s_back[own - first][0]);
+    auto known = [](double a) { return is_not_yet(a) ? __longlong_as_double(0x7ff8000000000000ll) : a; };
+    auto publish = [&](int lo) {                  // rows lo .. lo + 7 of the block are final
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t"
+                     "@p st.relaxed.gpu.global.f64 [%0], %1;\n\t}" ::"l"(ybuf + row),
+                     "d"(known(v)), "r"((unsigned)(mine && lane >= lo && lane < lo + 8))
+                     : "memory");
+    };
+    if (nbk < 32) {                               // rows past the block: y = 0 on entries of 0
+#pragma unroll
+        for (int s = 0; s < 32; ++s)
+            if (s >= nbk) cur[s] = 0.0;
+    }
+#pragma unroll
+    for (int c = 32 - kBackStep; c >= 0; c -= kBackStep)
+        if (c < nbk) {                            // (a branch, so that the stores stay near their steps)
+#pragma unroll
+            for (int s = c + kBackStep - 1; s >= c; --s) {
+                const double yt = __shfl_sync(0xffffffffu, v, s);
+                if (s % 8 == 7 && s < 31) publish(s + 1);
+                if (lane < s) v = fma(-cur[s], yt, v);
+                asm volatile("st.volatile.shared.f64 [%0], %1;" ::"r"(near + 8 * s), "d"(known(yt)) : "memory");
+            }
+        }
+    publish(0);
+    if (mine) {
+        if (dxout) dxout[row] = v;
+        if (xupd) xupd[row] = __dsub_rn(x, v);
+    }
+    return ok;
+}
+
 // Hin is the packed upper triangle, or (hin_lda > 0) a column-major matrix with that leading
 // dimension of which the upper triangle is read.
 // The solve of one problem by a group of G cooperating CTAs (this CTA is number bid of the group);
@@ -2438,7 +2550,7 @@ __device__ __forceinline__ void chol_body(const Dev& P, const double* __restrict
     __shared__ double s_q[kCholNB];       // q of the pair starting at k
     __shared__ unsigned short s_ent[kCholNB * (kCholNB + 1) / 2];
     __shared__ int s_neg[kCholNB / 2];    // the block's a or det was negative
-    __shared__ double s_yb[2][32];
+    __shared__ double s_back[kBackWarps][32], s_far[kBackWarps][32];
     __shared__ double s_l;
     int ent_nb = -1;
     double l = (lptr && apply_first != 2) ? *lptr : lval;
@@ -2450,6 +2562,7 @@ __device__ __forceinline__ void chol_body(const Dev& P, const double* __restrict
     if (P.ls && bid == 0 && threadIdx.x == 0) P.ls[4] = 0.0;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int gtid = bid * blockDim.x + tid, gthreads = G * blockDim.x;
+    for (int i = gtid; i < d; i += gthreads) P.ybuf[i] = __longlong_as_double(kNotYet);
     if (apply_first) {
         const int U = d * (d + 1) / 2;
         const bool own_l = apply_first == 2;
@@ -2781,16 +2894,25 @@ __device__ __forceinline__ void chol_body(const Dev& P, const double* __restrict
         if (!gs.sync()) goto timeout;
     }
     if (!gs.sync()) goto timeout;
-    if (bid != 0) return;
     {
-        // L^T dx = z (z in column d), blocked by 32 rows (CTA 0)
-        double* y = P.ybuf;
-        double gs = 0.0;
-        for (int i = tid; i < d; i += blockDim.x) {
-            y[i] = A[up_pos(i, d)];
-            gs += gin[i] * gin[i];
+        // L^T dx = z (z in column d)
+        const int nblocks = (d + 31) / 32, ngroups = (nblocks + kBackWarps - 1) / kBackWarps;
+        const bool norm_here = bid == (G > (unsigned)ngroups ? (unsigned)ngroups : 0u);
+        bool lost = false;
+        for (int grp = (int)bid; grp < ngroups; grp += (int)G) {
+            if (tid < 32 * kBackWarps) s_back[warp][lane] = __longlong_as_double(kNotYet);
+            __syncthreads();
+            const int own = grp * kBackWarps + warp;
+            if (warp < kBackWarps && own < nblocks) {
+                lost |= !back_block(A, d, own, grp * kBackWarps, s_back, s_far[warp], P.ybuf, dxout, xupd);
+                if (P.ls && own == nblocks - 1 && lane == 0) P.ls[4] = lost ? 0.0 : 1.0;
+            }
+            __syncthreads();
         }
-        if (record) {   // ||g|| for the round statistics
+        if (lost && lane == 0) *P.status = -5;
+        if (record && norm_here) {   // ||g|| for the round statistics, in a CTA without rows if there is one
+            double gs = 0.0;
+            for (int i = tid; i < d; i += blockDim.x) gs += gin[i] * gin[i];
             for (int o = 16; o > 0; o >>= 1) gs += __shfl_down_sync(0xffffffffu, gs, o);
             __shared__ double s_gs[kCoopThreads / 32];
             if (lane == 0) s_gs[tid >> 5] = gs;
@@ -2799,110 +2921,11 @@ __device__ __forceinline__ void chol_body(const Dev& P, const double* __restrict
                 double t = 0.0;
                 for (int w = 0; w < kCoopThreads / 32; ++w) t += s_gs[w];
                 P.stats[0] = sqrt(t);
+                int r = *P.round_ctr;
+                if (r < P.hist_cap) P.hist[r] = P.stats[0];
+                *P.round_ctr = r + 1;
             }
         }
-        // Blocks of 32 rows from the bottom.  Warp 0 solves a block (lane = row, the block's
-        // triangle in registers), then applies the block's solution to the next block's rows, which
-        // it keeps in registers; meanwhile warps 1-3 and 5-7 apply it to all rows above.  Warp 4
-        // shares warp 0's sub-partition and runs no FP64 instruction: it stages the triangle (Db)
-        // and the rectangle of the update (Rb) of the block after the current one into shared
-        // memory, each as soon as warp 0 has taken the current one into registers (named barriers
-        // 3 and 2), so warp 0 reads no global memory.  A row receives its updates in descending t
-        // order whichever warp applies them.
-        const int nblocks = (d + 31) / 32;
-        auto stage_t = [&](int blk) {
-            const int b1 = d - 32 * blk, b0 = max(0, b1 - 32), nbk = b1 - b0;
-#pragma unroll 8
-            for (int s = 0; s < 32; ++s) Db[lane][s] = (lane < s && s < nbk) ? A[up_pos(b0 + lane, b0 + s)] : 0.0;
-        };
-        auto stage_r = [&](int blk) {
-            const int b1 = d - 32 * blk, b0 = max(0, b1 - 32), nbk = b1 - b0, n0 = max(0, b0 - 32);
-#pragma unroll 8
-            for (int s = 0; s < 32; ++s)
-                Rb[lane][s] = (s < nbk && n0 + lane < b0) ? A[up_pos(n0 + lane, b0 + s)] : 0.0;
-        };
-        if (warp == 4) {
-            stage_t(0);
-            stage_r(0);
-        }
-        __syncthreads();
-        double v = 0.0;
-        if (tid < 32) {
-            const int b1 = d, b0 = max(0, d - 32);
-            v = (lane < b1 - b0) ? y[b0 + lane] : 0.0;
-        }
-        for (int blk = 0; blk < nblocks; ++blk) {
-            const int b1 = d - 32 * blk, b0 = max(0, b1 - 32), nbk = b1 - b0;
-            const int n0 = max(0, b0 - 32);                 // next block: rows [n0, b0)
-            const int ut = (warp < 4 ? warp - 1 : warp - 2) * 32 + lane;      // warps 1-3 and 5-7
-            double av1[32];
-            if (tid < 32) {
-                double ar[32];
-#pragma unroll
-                for (int s = 0; s < 32; ++s) ar[s] = Db[lane][s];
-                asm volatile("bar.arrive 3, 64;" ::: "memory");   // warp 4 may refill Db
-#pragma unroll
-                for (int s = 31; s >= 0; --s) {
-                    if (s < nbk) {
-                        const double yt = __shfl_sync(0xffffffffu, v, s);
-                        if (lane < s) v = fma(-ar[s], yt, v);
-                    }
-                }
-                if (lane < nbk) {
-                    y[b0 + lane] = v;
-                    s_yb[blk & 1][lane] = v;
-                }
-            } else if (warp == 4) {
-                asm volatile("bar.sync 3, 64;" ::: "memory");
-                if (blk + 1 < nblocks) stage_t(blk + 1);
-            } else if (ut < n0) {      // the first row's entries, while warp 0 solves the block
-#pragma unroll
-                for (int s = 0; s < 32; ++s) av1[s] = (s < nbk) ? A[up_pos(ut, b0 + s)] : 0.0;
-            }
-            __syncthreads();
-            if (tid < 32) {
-                double av[32];
-#pragma unroll
-                for (int s = 0; s < 32; ++s) av[s] = Rb[lane][s];
-                asm volatile("bar.arrive 2, 64;" ::: "memory");   // warp 4 may refill Rb
-                if (b0 > 0) {
-                    const int i = n0 + lane;
-                    double w = (i < b0) ? y[i] : 0.0;
-#pragma unroll
-                    for (int s = 31; s >= 0; --s)
-                        if (s < nbk) w = fma(-av[s], s_yb[blk & 1][s], w);
-                    v = w;
-                }
-            } else if (warp == 4) {
-                asm volatile("bar.sync 2, 64;" ::: "memory");
-                if (blk + 1 < nblocks) stage_r(blk + 1);
-            } else {
-                for (int i = ut; i < n0; i += blockDim.x - 64) {
-                    double w = y[i];
-#pragma unroll
-                    for (int s = 31; s >= 0; --s)
-                        if (s < nbk) w = fma(-av1[s], s_yb[blk & 1][s], w);
-                    y[i] = w;
-                    if (i + (int)blockDim.x - 64 < n0) {
-#pragma unroll
-                        for (int s = 0; s < 32; ++s)
-                            av1[s] = (s < nbk) ? A[up_pos(i + blockDim.x - 64, b0 + s)] : 0.0;
-                    }
-                }
-            }
-        }
-        __syncthreads();
-        for (int i = tid; i < d; i += blockDim.x) {
-            const double dxi = y[i];
-            if (dxout) dxout[i] = dxi;
-            if (xupd) xupd[i] = __dsub_rn(xupd[i], dxi);
-        }
-        if (record && tid == 0) {
-            int r = *P.round_ctr;
-            if (r < P.hist_cap) P.hist[r] = P.stats[0];
-            *P.round_ctr = r + 1;
-        }
-        if (P.ls && tid == 0) P.ls[4] = 1.0;
     }
     return;
 timeout:
