@@ -118,9 +118,9 @@ cudaError_t raise_shuffle_smem(const void* kernel, int k)
     return shuffle_smem(k) > 48 * 1024 ? fednl_raise_dyn_smem(kernel, shuffle_smem(k)) : cudaSuccess;
 }
 
-// CTAs of the cooperative Cholesky, at most one per SM: two warps of the first trailing update each (its
-// entries' chains of 32 fused multiply-adds then run on sub-partitions of their own), which also leaves a
-// CTA few panel columns (d = 69: 3 CTAs of 13 columns 66 us, 12 of 3 60 us)
+// CTAs of the cooperative Cholesky, at most one per SM: two warps of the first trailing update each (the
+// SM's FP64 unit takes a warp's operation every 19 cycles, so the 64-cycle chains of three warps run side
+// by side), which also leaves a CTA few panel columns (d = 69: 3 CTAs of 13 columns 66 us, 12 of 3 60 us)
 int chol_grid(int d)
 {
     int dev = 0, sms = 1, bps = 1;

@@ -1384,7 +1384,7 @@ struct SelectDraws {
 
 // The difference's squared Frobenius norm in the fixed segment order (k_hess_binary's, the CPU
 // oracle's orc_frob_sym) and Lk = sqrt of it (TopK.h:74-78), formed by six of the selection kernel's
-// warps, two on each SM sub-partition that the heap's warp 0 is not on, while that walks the heap:
+// warps while warp 0 walks the heap:
 // segment seg holds 512 upper positions, lane l squares positions 32 q + l into fused multiply-adds
 // (diagonal and off-diagonal apart, loaded ahead) and gives a + 2 b to the segment's halving tree; warp 1
 // then adds the segment sums in order.
@@ -1442,9 +1442,9 @@ __device__ __forceinline__ void select_norms(const SelectDraws& dr, const double
 // kernel's warps beside the heap walk.  The ten running sums of the reference's loop are chains of
 // dependent FP64 adds (eight lane accumulators shared by all columns: column j, rows i < 8 floor(j/8) with
 // i mod 8 = lane; one scalar for rows 8 floor(j/8) .. j-1; one for the diagonal), and a dependent FP64 add
-// costs 64 cycles (320 while another warp issues FP64 instructions on the sub-partition), so everything
-// else is taken off them: warps 3, 6 and 7 square the coming columns into a ring (kFrobCols columns a
-// step, contiguous in the packed order, their loads a step ahead); warp 1, alone on its sub-partition, adds
+// costs 64 cycles alone (19 for each warp that uses the SM's FP64 unit, once these add up to more), so
+// everything else is taken off them: warps 3, 6 and 7 square the coming columns into a ring (kFrobCols columns a
+// step, contiguous in the packed order, their loads a step ahead); warp 1 adds
 // the eight lanes; warp 2 the two scalars.  d = 301: 5681 dependent adds at 86 cycles, 237 us beside the
 // walk, against 346 us for a kernel of its own before it (the round 1617 -> 1453 us).
 constexpr int kFrobCols = 4;
@@ -2686,7 +2686,7 @@ __device__ __forceinline__ void chol_body(const Dev& P, const double* __restrict
                 }
             }
 #pragma unroll
-            for (int q = 0; q < kSlotsS; ++q) {     // the first slab entries on warps 5-7, one per sub-partition
+            for (int q = 0; q < kSlotsS; ++q) {     // the first slab entries on warps 5-7
                 const int e = (ut + kUpd / 2) % kUpd + q * kUpd;
                 is_[q] = -1;
                 ss[q] = 0;

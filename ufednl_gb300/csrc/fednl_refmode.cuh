@@ -804,7 +804,7 @@ __global__ void __launch_bounds__(kRefCholThreads, 1) k_chol_ref(Dev P, const do
             rest[i] = sum;
         }
         // The products of a step, elements m >= 1: u = 8 m + q, row t - 1 - q, column t + 8 m, by warps 2, 3
-        // and 5-7 (warp 4 shares warp 0's sub-partition, whose FP64 pipe the chain needs).
+        // and 5-7.
         // R is loaded two steps ahead of the products' use (four a thread; more at large d in line).
         constexpr int kAhead = 4;
         double rv[kAhead];
