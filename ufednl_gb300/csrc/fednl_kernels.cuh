@@ -2935,7 +2935,7 @@ timeout:
     }
 }
 
-__global__ void __launch_bounds__(kCoopThreads) k_chol_coop(Dev P, const double* __restrict__ Hin, int hin_lda,
+__global__ void __launch_bounds__(kCoopThreads, 1) k_chol_coop(Dev P, const double* __restrict__ Hin, int hin_lda,
                                                             const double* lptr, double lval,
                                                             const double* __restrict__ gin, double* dxout,
                                                             double* xupd, int record, int apply_first)
@@ -2947,7 +2947,9 @@ __global__ void __launch_bounds__(kCoopThreads) k_chol_coop(Dev P, const double*
 
 // Several independent Option-B solves in one cooperative launch (the serving loop's tick): job j
 // owns CTAs [cta0, cta0 + ncta) and its own barrier words, so problems of different d proceed
-// side by side.
+// side by side.  Two CTAs an SM (128 registers): one problem's updates then run beside another's chains (a
+// serving tick 2885 -> 2805 us); k_chol_coop, with at most one, takes what it needs (16 RandK rounds
+// w8a-like 6248 -> 6114 us).
 struct CholJob {
     Dev P;
     const double* Hin;
@@ -2960,7 +2962,7 @@ struct CholJob {
     int record, cta0, ncta;
 };
 
-__global__ void __launch_bounds__(kCoopThreads) k_chol_batched(const CholJob* __restrict__ jobs, int njobs)
+__global__ void __launch_bounds__(kCoopThreads, 2) k_chol_batched(const CholJob* __restrict__ jobs, int njobs)
 {
     int j = 0;
     while (j + 1 < njobs && (int)blockIdx.x >= jobs[j + 1].cta0) ++j;
