@@ -41,10 +41,10 @@ def test_margins_one_and_two_samples_a_thread(gpu, d):
     assert abs(g[0] - g64) <= 1e-10 * g64
 
 
-@pytest.mark.parametrize("d,k", [(66, 300), (129, 1000), (130, 5000)])
+@pytest.mark.parametrize("d,k", [(66, 300), (129, 1000), (130, 5000), (258, 9000), (400, 3)])
 def test_topk_with_equal_differences(gpu, d, k):
     """Columns in equal triples: every difference off the blocks' diagonals appears several times, so the
-    threshold is shared; the lower positions are kept."""
+    threshold is shared; the lower positions are kept (one CTA a client, clusters of 2 and of 8)."""
     from ufednl_gb300 import datagen
 
     p = datagen.dense_problem_fp32(9, d, [70, 129], 1e-3)
@@ -58,5 +58,5 @@ def test_topk_with_equal_differences(gpu, d, k):
             order = np.lexsort((np.arange(len(mag)), -mag))
             np.testing.assert_array_equal(np.sort(order[:k]), sel)
             ties += mag[order[k - 1]] == mag[order[k]]
-    assert ties > 0
+    assert ties > 0 or k < 10
     mx.close()

@@ -220,6 +220,7 @@ struct fednl_mx_handle_s {
     bool ready = false;
     int rounds_done = 0;
     size_t select_smem = 0;
+    int select_ncl = 1;                // CTAs per client of the selection
     bool chol32 = false;               // the round solves with the FP32 factor + refinement
     bool chol32_ok = false;            // the system fits one CTA's shared memory
     bool coop32 = false;               // the round solves with the FP32 cooperative factor (fednl_chol32c.cuh)
@@ -294,6 +295,48 @@ void launch_margin(fednl_mx_handle h, const fednl_tc::MxDev& P, cudaStream_t st)
     else fednl_tc::k_mx_margin<1><<<grid, block, 0, st>>>(P);
 }
 
+cudaLaunchConfig_t mx_select_config(fednl_mx_handle h, int ncl, cudaLaunchAttribute* at)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(h->nc * ncl);
+    cfg.blockDim = dim3(fednl_tc::kSelThreads);
+    cfg.dynamicSmemBytes = h->select_smem;
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = ncl;
+    at->val.clusterDim.y = 1;
+    at->val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = ncl > 1 ? 1 : 0;
+    return cfg;
+}
+
+// CTAs per client of the selection: the largest cluster up to eight of which all clients' fit the GPU at
+// once (a second wave costs more than the cluster gains) and which leaves each thread four positions a
+// pass.  TopK, one CTA / a cluster, us: d = 1024, 24 clients 245 / 78 (four), 8 clients 219 / 53 (eight),
+// 16 clients 221 / 72 with four, 100 with eight, which take two waves; d = 700, 30 clients 109 / 45; d = 512, 60 clients
+// 66 / 45; d = 301, 24 clients 28 / 23; d = 200, 16 clients 18.8 / 18.7.
+int mx_select_cluster(fednl_mx_handle h)
+{
+    for (int ncl = 8; ncl > 1; ncl /= 2) {
+        if (h->U / ncl < 4 * fednl_tc::kSelThreads) continue;
+        cudaLaunchAttribute at;
+        const cudaLaunchConfig_t cfg = mx_select_config(h, ncl, &at);
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, fednl_tc::k_mx_select, &cfg) == cudaSuccess && clusters >= h->nc)
+            return ncl;
+        cudaGetLastError();
+    }
+    return 1;
+}
+
+cudaError_t launch_mx_select(fednl_mx_handle h, const fednl_tc::MxDev& P, int toplek, cudaStream_t st)
+{
+    cudaLaunchAttribute at;
+    cudaLaunchConfig_t cfg = mx_select_config(h, h->select_ncl, &at);
+    cfg.stream = st;
+    return cudaLaunchKernelEx(&cfg, fednl_tc::k_mx_select, P, h->k, toplek, (unsigned)h->desc.toplek_seed, h->select_ncl);
+}
+
 int mx_launch_round(fednl_mx_handle h, cudaEvent_t* ev = nullptr, bool client_phase_only = false)
 {
     using namespace fednl_tc;
@@ -348,7 +391,7 @@ int mx_launch_round(fednl_mx_handle h, cudaEvent_t* ev = nullptr, bool client_ph
     }
     if (!randk) {
         const int toplek = h->comp == FEDNL_TOPLEK;
-        k_mx_select<<<h->nc, kSelThreads, h->select_smem, st>>>(P, h->k, toplek, h->desc.toplek_seed);
+        CKM(launch_mx_select(h, P, toplek, st));
         mark();
     }
     k_mx_apply<<<(h->U + 255) / 256, 256, 0, st>>>(P);
@@ -578,6 +621,7 @@ static int mx_create_impl(const fednl_problem_desc* desc, fednl_mx_handle* out, 
             return fail_m(FEDNL_ECUDA, "shared-memory attribute refused");
         }
     }
+    if (h->comp != FEDNL_RANDK_PHILOX && h->k < h->U) h->select_ncl = mx_select_cluster(h);
     *out = h;
     return FEDNL_OK;
 }

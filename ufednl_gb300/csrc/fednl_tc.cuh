@@ -779,8 +779,9 @@ __device__ __forceinline__ void add_u64(unsigned long long* sum, unsigned long l
     atomicAdd(w + 1, (unsigned)(v >> 32) + (old + lo < old ? 1u : 0u));
 }
 
-// TopLEK's term of a kept-set entry in fixed point: c v^2 2^sh (c = 1 on the diagonal, 2 off it) for the FP32 magnitude v = m 2^(eb - 150) (biased exponent eb, significand m),
-// i.e. m^2 2^(2 eb - 300 + sh), exact where the shift is not negative
+// TopLEK's term of a kept-set entry in fixed point: c v^2 2^sh (c = 1 on the diagonal, 2 off it) for the
+// FP32 magnitude v = m 2^(eb - 150) (biased exponent eb, significand m), i.e. m^2 2^(2 eb - 300 + sh),
+// exact where the shift is not negative
 __device__ __forceinline__ unsigned long long lek_fixed(unsigned long long e, int sh)
 {
     const unsigned key = set_key(e);
@@ -819,11 +820,26 @@ __device__ __forceinline__ unsigned long long block_scan_u64(unsigned long long 
     return r;
 }
 
-// one CTA (1024 threads) per client: selection bitmap sel[c] from the differences dsel[c].  Its passes over
+__device__ __forceinline__ unsigned cluster_u32(const unsigned* at, int rank)
+{
+    uint32_t a;
+    unsigned v;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(at)), "r"(rank));
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// one CTA (1024 threads), or a cluster, per client: selection bitmap sel[c] from the differences dsel[c].  Its passes over
 // the differences are bound by the latency of their loads and by atomics on shared bins: eight loads in
 // flight per thread, the ties at the threshold only ordered where not all are kept, the kept entries'
-// values gathered by a thread per entry (d = 301, k = 8d, 142 clients: 74 -> 49 us).
-__global__ void __launch_bounds__(kSelThreads) k_mx_select(MxDev P, int k, int toplek, unsigned seed)
+// values gathered by a thread per entry (d = 301, k = 8d, 142 clients: 74 -> 49 us).  With few clients a
+// cluster of ncl CTAs per client shares the passes (one SM reads L2 at about 20 bytes a cycle), each a
+// range of the selection words, the histograms summed over the cluster; CTA 0 runs TopLEK's rule.
+__global__ void __launch_bounds__(kSelThreads) k_mx_select(MxDev P, int k, int toplek, unsigned seed, int ncl)
 {
     extern __shared__ unsigned long long s_set[];       // TopLEK: [max(Kp, 1024)] entries, [2048] masses
     __shared__ unsigned hist[2048];
@@ -834,11 +850,14 @@ __global__ void __launch_bounds__(kSelThreads) k_mx_select(MxDev P, int k, int t
     __shared__ unsigned long long s_rx, s_above;
     __shared__ unsigned s_bin, s_need, s_cnt[32], s_nk, s_kmax, s_qstar;
     __shared__ int s_istar, s_all;
-    const int c = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    __shared__ unsigned s_ties;
+    const int c = blockIdx.x / ncl, rank = blockIdx.x % ncl, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int U = P.U;
     const float* v = P.dsel + (size_t)c * P.Up;
     unsigned* sc = P.sel + (size_t)c * P.SW;
     const int K = k < U ? k : U;
+    const int SWn = (U + 31) >> 5, wpc = (SWn + ncl - 1) / ncl;      // this CTA's selection words
+    const int wa = min(SWn, rank * wpc), wb = min(SWn, wa + wpc), qb = min(U, 32 * wb);
     unsigned T = 0, need = 0;
     if (K < U) {
         // radix select of the K-th largest key: 11 + 11 + 9 bits from the top
@@ -849,12 +868,12 @@ __global__ void __launch_bounds__(kSelThreads) k_mx_select(MxDev P, int k, int t
             const int sh = shs[pass], nb = 1 << nbits[pass];
             for (int b = tid; b < 2048; b += kSelThreads) hist[b] = 0u;
             __syncthreads();
-            for (int q0 = tid; q0 < U; q0 += 8 * kSelThreads) {
+            for (int q0 = 32 * wa + tid; q0 < qb; q0 += 8 * kSelThreads) {
                 unsigned key[8];
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
                     const int q = q0 + u * kSelThreads;
-                    key[u] = q < U ? mag_key(v[q]) : 0xffffffffu;        // (no key has bit 31)
+                    key[u] = q < qb ? mag_key(v[q]) : 0xffffffffu;       // (no key has bit 31)
                 }
 #pragma unroll
                 for (int u = 0; u < 8; ++u)
@@ -864,7 +883,16 @@ __global__ void __launch_bounds__(kSelThreads) k_mx_select(MxDev P, int k, int t
             __syncthreads();
             // thread t owns bins nb-1-2t and nb-2-2t (descending keys)
             const int b0 = nb - 1 - 2 * tid, b1 = b0 - 1;
-            const unsigned h0 = b0 >= 0 ? hist[b0] : 0u, h1 = b1 >= 0 ? hist[b1] : 0u;
+            unsigned h0 = b0 >= 0 ? hist[b0] : 0u, h1 = b1 >= 0 ? hist[b1] : 0u;
+            if (ncl > 1) {
+                cluster_sync();
+                for (int r = 0; r < ncl; ++r)
+                    if (r != rank) {
+                        if (b0 >= 0) h0 += cluster_u32(hist + b0, r);
+                        if (b1 >= 0) h1 += cluster_u32(hist + b1, r);
+                    }
+                cluster_sync();                   // the histograms may be cleared for the next pass
+            }
             const unsigned incl = block_scan_u32(h0 + h1, s_wu, nullptr);
             const unsigned excl = incl - h0 - h1;
             if (excl < need && need <= incl) {
@@ -892,8 +920,8 @@ __global__ void __launch_bounds__(kSelThreads) k_mx_select(MxDev P, int k, int t
     // flight in each pass).
     {
         const bool all = K >= U || s_all != 0;      // (s_all of the last radix pass: the keys equal to T)
-        const int SWn = (U + 31) >> 5, wpw = (SWn + 31) >> 5;
-        const int w0 = warp * wpw, w1 = min(SWn, w0 + wpw);
+        const int wpw = (wb - wa + 31) >> 5;
+        const int w0 = min(wb, wa + warp * wpw), w1 = min(wb, w0 + wpw);
         unsigned neq = 0;
         for (int wd = w0; wd < w1 && !all; wd += 8) {
             unsigned key[8];
@@ -909,6 +937,11 @@ __global__ void __launch_bounds__(kSelThreads) k_mx_select(MxDev P, int k, int t
         __syncthreads();
         unsigned carry = 0;
         for (int w = 0; w < warp && !all; ++w) carry += s_cnt[w];
+        if (ncl > 1 && !all) {                    // the ties in the CTAs before this one
+            if (tid == kSelThreads - 1) s_ties = carry + s_cnt[31];
+            cluster_sync();
+            for (int r = 0; r < rank; ++r) carry += cluster_u32(&s_ties, r);
+        }
         for (int wd = w0; wd < w1; wd += 8) {
             unsigned key[8];
 #pragma unroll
@@ -930,6 +963,8 @@ __global__ void __launch_bounds__(kSelThreads) k_mx_select(MxDev P, int k, int t
         }
         __syncthreads();
     }
+    if (ncl > 1) cluster_sync();                  // every CTA's words are written, and its counts read
+    if (rank != 0) return;
     if (!toplek || K >= U) {
         if (tid == 0) P.cnt[c] = K;
         return;
