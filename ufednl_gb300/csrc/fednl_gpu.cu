@@ -628,6 +628,19 @@ bool one_client_kernel(fednl_handle h)
     return h->binary && !h->dev.ref && (long long)h->nc * client_threads(h->d) <= sms * 2048ll;
 }
 
+// CTAs of the round's solve: the factorization's, but no more than four selection words a CTA in its merge,
+// as far as the SMs go, so that a word's FP64 chain over the clients has the SM's unit nearly to itself (d =
+// 25, 126 clients, RandK k = 25: one CTA 57 us, three 38, Natural 115 and 64; d = 60, seven CTAs 65, fifteen
+// 55; above d = 110 the factorization takes as many)
+int round_grid(fednl_handle h)
+{
+    int dev = 0, sms = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int g = chol_grid(h->d), words = (h->U + 31) / 32;
+    return h->pp ? g : std::max(g, std::min(sms, (words + 3) / 4));
+}
+
 // dynamic shared memory of k_client_binary: the weights and the intercept's word sums
 size_t client_smem(fednl_handle h) { return (size_t)h->maxn * 16 + (size_t)((h->maxn + 63) / 64) * 16; }
 
@@ -715,7 +728,7 @@ int launch_round(fednl_handle h, Marks* M = nullptr, bool client_phase_only = fa
     const int na = P.n_act, comp = h->comp;
     // The master's aggregation needs only the gradients and Lk.  With TopK / TopLEK it runs in the
     // selection kernel's idle warps; otherwise, in a graph, on a branch beside the shift update, and
-    // the compressor's draws, which read nothing of the round, run there from its start (all kept in
+    // the compressor's draws, which read nothing of the round, run there beside the Hessian (all kept in
     // line when the round is profiled kernel by kernel)
     const bool agg_in_select = !h->pp && (comp == FEDNL_TOPK || comp == FEDNL_TOPLEK);
     const bool fork = !M && h->side && !h->pp && !agg_in_select;
@@ -741,7 +754,7 @@ int launch_round(fednl_handle h, Marks* M = nullptr, bool client_phase_only = fa
     // FedNL-PP: the branch samples the round's clients and makes their draws beside the client oracle (which
     // takes every client), then forms the true gradient and its norm beside the rest of the round
     const bool pfork = !M && h->side && h->pp;
-    if (fork || pfork) {
+    if (pfork) {
         CK(cudaEventRecord(h->fork_ev, st));
         CK(cudaStreamWaitEvent(h->side, h->fork_ev, 0));
     }
@@ -751,11 +764,11 @@ int launch_round(fednl_handle h, Marks* M = nullptr, bool client_phase_only = fa
             h->nc, h->tau, P.sampler, shuffle_smem(h->tau) ? nullptr : P.shuf, (int*)P.act, P.is_sel, P.needs);
         CKL();
     }
-    if (fork || pfork) {
+    if (pfork) {
         int rc = draw(h->side);
         if (rc) return rc;
+        CK(cudaEventRecord(h->join_ev, h->side));
     }
-    if (pfork) CK(cudaEventRecord(h->join_ev, h->side));
     if (one_client_kernel(h)) {      // the client oracle in one launch
         MARK("k_client_binary");
         k_client_binary<<<h->nc, client_threads(h->d), client_smem(h), st>>>(P);
@@ -775,6 +788,15 @@ int launch_round(fednl_handle h, Marks* M = nullptr, bool client_phase_only = fa
         if (h->binary) k_grad_binary<<<gg, 128, (size_t)h->maxn * 16, st>>>(P);
         else k_grad_dense<<<gg, 128, 0, st>>>(P);
         CKL();
+    }
+    // the draws run beside the Hessian: beside the client oracle their CTAs crowd its own, one a client, onto
+    // the SMs left over, and FP64 work does not share an SM well (d = 25, 126 clients of up to 660
+    // samples, k = 100: a round of 192 us so)
+    if (fork) {
+        CK(cudaEventRecord(h->fork_ev, st));
+        CK(cudaStreamWaitEvent(h->side, h->fork_ev, 0));
+        int rc = draw(h->side);
+        if (rc) return rc;
     }
     if (h->pp) {
         cudaStream_t s2 = st;
@@ -1147,7 +1169,7 @@ static int create_impl(const fednl_problem_desc* desc, fednl_handle* out, int64_
         fednl_gpu_destroy(h);
         return fail(FEDNL_ECUDA, "shared-memory attribute refused");
     }
-    h->chol_grid = chol_grid(h->d);
+    h->chol_grid = round_grid(h);
     if (P.ref) {
         h->ref_grid = ref_grid(h->d);
         if (fednl_raise_dyn_smem((const void*)k_chol_ref, ref_chol_smem(h->d, h->ref_grid)) != cudaSuccess) {
