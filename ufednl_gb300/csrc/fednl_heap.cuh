@@ -238,4 +238,31 @@ __device__ __forceinline__ bool extract_chunk(HeapS& h, HeapTop& top, bool live,
     return false;
 }
 
+// Two warps share TopLEK's extraction, step q = 1 .. nch: one extracts chunk q while the other tests the
+// window of chunk q - 1, then they meet (a barrier of the two).  Step q's verdict stands in hit[q & 1], both
+// zero before.  The word is written again in step q + 2, behind the meeting of step q + 1, which the
+// extracting warp joins only after it has read it.  In a single word step q + 1's verdict could overtake a
+// late read of step q's: the extracting warp would leave and the other wait for it for ever.
+template <class Extract, class Meet>
+__device__ __forceinline__ void extract_steps(int nch, const int* hit, Extract extract, Meet meet)
+{
+    for (int q = 1;; ++q) {
+        if (q < nch) extract(q);
+        meet();
+        if (hit[q & 1] || q == nch) break;
+    }
+}
+
+// window(q): whether chunk q holds a hit, the same in every lane; one lane writes
+template <class Window, class Meet>
+__device__ __forceinline__ void window_steps(int nch, int* hit, bool writer, Window window, Meet meet)
+{
+    for (int q = 1;; ++q) {
+        const bool found = q > 1 && window(q - 1);
+        if (writer) hit[q & 1] = found;
+        meet();
+        if (found || q == nch) break;
+    }
+}
+
 }  // namespace fednl

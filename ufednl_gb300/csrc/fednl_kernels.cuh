@@ -135,6 +135,13 @@ __device__ __forceinline__ void row_bound(unsigned* word, int left, int lane, do
     if (lane == 0) *word = m;
 }
 
+// Named barrier kId of kThreads threads, whole warps
+template <int kId, int kThreads>
+__device__ __forceinline__ void named_sync()
+{
+    asm volatile("bar.sync %0, %1;" ::"n"(kId), "n"(kThreads) : "memory");
+}
+
 __device__ __forceinline__ bool upper_is_diag(int p)
 {
     int i, j;
@@ -1392,7 +1399,7 @@ __global__ void __launch_bounds__(kSelThreads, 1) k_select(const double* __restr
     __shared__ __align__(8) unsigned long long s_bar[2];
     __shared__ __align__(16) unsigned s_gm[2 * (kSelStage / 32)];
     __shared__ HeapMins s_mins;
-    __shared__ int s_keep, s_fail, s_more, s_hit;
+    __shared__ int s_keep, s_fail, s_more, s_hit[2];
     __shared__ double s_win[5];
     const int c = act ? act[blockIdx.x] : blockIdx.x;
     const double* v = vals + (size_t)c * ustr;
@@ -1591,7 +1598,7 @@ __global__ void __launch_bounds__(kSelThreads, 1) k_select(const double* __restr
             }
             if (lane == 0) {
                 s_more = more;
-                s_hit = 0;
+                s_hit[0] = s_hit[1] = 0;
                 s_win[0] = omd;
                 s_win[1] = eps;
                 s_win[2] = hi;
@@ -1603,15 +1610,14 @@ __global__ void __launch_bounds__(kSelThreads, 1) k_select(const double* __restr
         if (s_more) {
             // Warp 0 extracts chunk q while warp 1 forms the window of chunk q - 1, whose places no longer
             // change; a hit is seen a chunk late, which only reorders the places below it.
+            auto meet = [] { named_sync<2, 64>(); };
             if (warp == 0) {
                 HeapTop top;
                 bool live = k - 32 > 21;
                 if (lane == 0 && live) top.load(h, mins);
-                for (int q = 1;; ++q) {
-                    if (q < nch && lane == 0) live = extract_chunk(h, top, live, k - 32 * q, max(k - 32 * (q + 1), 1));
-                    asm volatile("bar.sync 2, 64;" ::: "memory");
-                    if (s_hit || q == nch) break;
-                }
+                extract_steps(nch, s_hit, [&](int q) {
+                    if (lane == 0) live = extract_chunk(h, top, live, k - 32 * q, max(k - 32 * (q + 1), 1));
+                }, meet);
                 if (lane == 0 && live) top.store(h);
             } else if (warp == 1) {
                 omd = s_win[0];
@@ -1619,15 +1625,10 @@ __global__ void __launch_bounds__(kSelThreads, 1) k_select(const double* __restr
                 hi = s_win[2];
                 carry = s_win[3];
                 prev_last = s_win[4];
-                for (int q = 1;; ++q) {
-                    if (q > 1) {
-                        const int m = (q - 1) * 32 + lane;
-                        const bool hit = window(q - 1, m < k ? term_of(h.key[k - 1 - m], h.hid[k - 1 - m]) : 0.0);
-                        if (lane == 0) s_hit = hit;
-                    }
-                    asm volatile("bar.sync 2, 64;" ::: "memory");
-                    if (s_hit || q == nch) break;
-                }
+                window_steps(nch, s_hit, lane == 0, [&](int q) {
+                    const int m = q * 32 + lane;
+                    return window(q, m < k ? term_of(h.key[k - 1 - m], h.hid[k - 1 - m]) : 0.0);
+                }, meet);
             }
         }
         if (warp == (s_more ? 1 : 0) && lane == 0) {
