@@ -24,3 +24,12 @@ def test_extraction_and_windows_leave_together(host, nch, hit_at):
     met_x, met_w, stuck = map(int, host("steps", nch, hit_at).split())
     last = min(hit_at + 1, nch)
     assert (met_x, met_w, stuck) == (last, last, 0)
+
+
+@pytest.mark.parametrize("reverse", [0, 1])
+@pytest.mark.parametrize("k,values", [(21, 1000), (22, 5), (85, 1000), (300, 1 << 20), (341, 12)])
+def test_lanes_that_run_apart_keep_one_heap(host, k, values, reverse):
+    """A warp replaces the root together: each lane in turn runs as far ahead of the others as the code's own
+    meetings let it, and the heap and every lane's registers end as one thread's."""
+    bad, meetings = map(int, host("lanes", k, 200, values, reverse).split())
+    assert bad == 0 and meetings > 0

@@ -18,6 +18,10 @@ struct HeapS {
 // node start on a 32-byte boundary (two 16-byte loads), the id array so that they start on a
 // 16-byte boundary.  The path moves up one node and (ck, ci) is written where the walk stops,
 // which equals the reference's chain of swaps.
+//
+// kWarp: a whole warp makes the same call, every lane with the same values and the same stores.  Lanes may run
+// apart, and a level's stores replace what that level's loads read, so the lanes meet in between.
+template <bool kWarp = false>
 __device__ __forceinline__ void heap_descend(HeapS& h, int i, int n, unsigned long long lv,
                                              unsigned long long ck, unsigned ci)
 {
@@ -46,8 +50,10 @@ __device__ __forceinline__ void heap_descend(HeapS& h, int i, int n, unsigned lo
             }
         }
         if (!(lv > m)) break;
+        const unsigned hl = h.hid[lo];
+        if (kWarp) __syncwarp();
         h.key[i] = m;
-        h.hid[i] = h.hid[lo];
+        h.hid[i] = hl;
         i = lo;
         lv = m;
     }
@@ -161,7 +167,8 @@ struct HeapTop {
     // The entry (ck, ci) enters at the root of a heap of n >= 21 entries with its own key as the
     // comparison value (MinHeap.h:78-85 and :125-141: heap_descend(h, 0, n, ck, ck, ci)), in two steps:
     // the new root, true if the entry goes below it; then its place below.  below() returns true if
-    // entries in shared memory moved.
+    // entries in shared memory moved.  kWarp as for heap_descend: the lanes meet once all have read what the
+    // entry replaces (its node's id by the last ahead(), the entry that moves up).
     __device__ __forceinline__ bool root(unsigned long long ck, unsigned ci)
     {
         const bool gt = ck > s1;
@@ -169,6 +176,7 @@ struct HeapTop {
         I0 = gt ? i1 : ci;
         return gt;
     }
+    template <bool kWarp = false>
     __device__ __forceinline__ bool below(HeapS& h, int n, unsigned long long ck, unsigned ci)
     {
         const unsigned nd = t1 & 7u;
@@ -178,7 +186,10 @@ struct HeapTop {
         if (deeper) {       // level 2: the least child of the node is below the value that moved up
             x = m1;
             xi = h.hid[g1];
-            heap_descend(h, g1, n, m1, ck, ci);
+        }
+        if (kWarp) __syncwarp();
+        if (deeper) {
+            heap_descend<kWarp>(h, g1, n, m1, ck, ci);
             xm = children(h, nd);
         }
         h.hid[nd] = xi;

@@ -1340,7 +1340,7 @@ __device__ __forceinline__ bool select_scan(HeapS& h, int k, const double* v, co
     if (REGS) top.load(h, mins);
     for (int q = 0; q < n_chunks; ++q) {
         const int b = q & 1;
-        if (!mbar_wait(&s_bar[b], (unsigned)(q >> 1) & 1u)) return false;
+        if (!__all_sync(0xffffffffu, mbar_wait(&s_bar[b], (unsigned)(q >> 1) & 1u))) return false;
         const int st = s0 + q * kSelStage;
         const int len = min(kSelStage, U - st);
         const double* buf = stage + b * kSelStage;
@@ -1370,7 +1370,7 @@ __device__ __forceinline__ bool select_scan(HeapS& h, int k, const double* v, co
                     }
                     l = (int)__reduce_min_sync(0xffffffffu, (mine > root && lane > l) ? (unsigned)lane : 32u);
                     const unsigned long long nc = __shfl_sync(0xffffffffu, mine, l & 31);
-                    if (REGS && gt) top.below(h, k, cand, p);
+                    if (REGS && gt) top.below<true>(h, k, cand, p);
                     cand = nc;
                 }
             }
