@@ -33,3 +33,12 @@ def test_lanes_that_run_apart_keep_one_heap(host, k, values, reverse):
     meetings let it, and the heap and every lane's registers end as one thread's."""
     bad, meetings = map(int, host("lanes", k, 200, values, reverse).split())
     assert bad == 0 and meetings > 0
+
+
+def test_named_barriers_are_reached_by_whole_warps():
+    """bar.sync and bar.arrive are undefined on a warp whose lanes are apart: each stands behind __syncwarp()."""
+    lines = [(f, t) for f in sorted(os.listdir(CSRC)) for t in open(os.path.join(CSRC, f)).read().splitlines()]
+    at = [n for n, (_, t) in enumerate(lines) if 'asm volatile("bar.sync' in t or 'asm volatile("bar.arrive' in t]
+    assert at
+    for n in at:
+        assert lines[n - 1][1].strip() == "__syncwarp();", lines[n]

@@ -135,11 +135,19 @@ __device__ __forceinline__ void row_bound(unsigned* word, int left, int lane, do
     if (lane == 0) *word = m;
 }
 
-// Named barrier kId of kThreads threads, whole warps
-template <int kId, int kThreads>
-__device__ __forceinline__ void named_sync()
+// Named barrier of kThreads threads, whole warps.  bar.sync and bar.arrive are the aligned forms, undefined on a
+// warp whose lanes are apart (behind one lane's work, say), so the lanes meet first.
+template <int kThreads>
+__device__ __forceinline__ void named_sync(int id)
 {
-    asm volatile("bar.sync %0, %1;" ::"n"(kId), "n"(kThreads) : "memory");
+    __syncwarp();
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kThreads) : "memory");
+}
+template <int kThreads>
+__device__ __forceinline__ void named_arrive(int id)
+{
+    __syncwarp();
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(kThreads) : "memory");
 }
 
 __device__ __forceinline__ bool upper_is_diag(int p)
@@ -1186,7 +1194,7 @@ __device__ __forceinline__ void select_norms(const SelectDraws& dr, const double
         const double cs = chunk_tree(segment_value(fa, fb2));
         if (lane == 0) fp[seg] = cs;
     }
-    asm volatile("bar.sync 1, 192;" ::: "memory");
+    named_sync<192>(1);
     if (warp == 1) {
         double f = 0.0;
         for (int q0 = 0; q0 < dr.nseg; q0 += 32) {
@@ -1249,7 +1257,7 @@ __device__ __forceinline__ void select_frob_ref(double* ring, const double* __re
                     buf += j + 1;
                 }
             }
-            asm volatile("bar.sync 3, 160;" ::: "memory");
+            named_sync<160>(3);
         }
     } else {
         const int st = (warp == 3 ? 0 : warp - 5) * 32 + lane;
@@ -1274,11 +1282,11 @@ __device__ __forceinline__ void select_frob_ref(double* ring, const double* __re
                     buf[i] = __dmul_rn(v[o + i], v[o + i]);
                 fetch(s + 1);
             }
-            asm volatile("bar.sync 3, 160;" ::: "memory");
+            named_sync<160>(3);
         }
     }
     if (warp == 2 && lane < 2) s_two[lane] = acc;
-    asm volatile("bar.sync 3, 160;" ::: "memory");
+    named_sync<160>(3);
     if (warp == 1) {
         double c8[8];
 #pragma unroll
@@ -1610,7 +1618,7 @@ __global__ void __launch_bounds__(kSelThreads, 1) k_select(const double* __restr
         if (s_more) {
             // Warp 0 extracts chunk q while warp 1 forms the window of chunk q - 1, whose places no longer
             // change; a hit is seen a chunk late, which only reorders the places below it.
-            auto meet = [] { named_sync<2, 64>(); };
+            auto meet = [] { named_sync<64>(2); };
             if (warp == 0) {
                 HeapTop top;
                 bool live = k - 32 > 21;
@@ -2536,7 +2544,7 @@ __device__ __forceinline__ void chol_body(const Dev& P, const double* __restrict
                         const int sl = cix - nd;
                         SR[k + o][sl] = fma(ca, Sb[k][sl], __dmul_rn(cb, Sb[k + 1][sl]));
                     }
-                    asm volatile("bar.sync 1, 192;" ::: "memory");
+                    named_sync<192>(1);
 #pragma unroll
                     for (int q2 = 0; q2 < kSlotsB; ++q2) {
                         const int i = ib[q2], j = jb[q2];

@@ -562,7 +562,7 @@ __global__ void __launch_bounds__(kRefCholThreads, 1) k_chol_ref(Dev P, const do
                     };
                     double inv = pivot(0, Lr[0][r0]);
                     for (int k = 0; k < nr; ++k) {
-                        asm volatile("bar.sync 1, 64;" ::: "memory");      // row k's pivot, warp 1's exports
+                        named_sync<64>(1);      // row k's pivot, warp 1's exports
                         if (s_neg[k]) break;
                         if (k + 1 < nr) {
                             const double rk = __dmul_rn(inv, s_num1[k]);
@@ -599,9 +599,9 @@ __global__ void __launch_bounds__(kRefCholThreads, 1) k_chol_ref(Dev P, const do
                         s_tl[0] = 0.0;
                     }
                     for (int k = 0; k < nr; ++k) {
-                        asm volatile("bar.sync 1, 64;" ::: "memory");      // row k's pivot
+                        named_sync<64>(1);      // row k's pivot
                         if (s_neg[k]) {
-                            asm volatile("bar.arrive %0, 192;" ::"r"(3 + k) : "memory");
+                            named_arrive<192>(3 + k);
                             break;
                         }
                         const double inv = s_inv[r0 + k];
@@ -613,8 +613,7 @@ __global__ void __launch_bounds__(kRefCholThreads, 1) k_chol_ref(Dev P, const do
                             if (on && j == k) RB[r0 + k][r0 + i] = i == k ? s_r[r0 + k] : r;
                         }
                         __threadfence_block();
-                        __syncwarp();
-                        asm volatile("bar.arrive %0, 192;" ::"r"(3 + k) : "memory");
+                        named_arrive<192>(3 + k);
                         if (k + 1 < nr) {
                             const bool later = on && j > k;
                             const double rj = later ? RB[r0 + k][r0 + j] : 0.0, ri = later ? RB[r0 + k][r0 + i] : 0.0;
@@ -639,7 +638,7 @@ __global__ void __launch_bounds__(kRefCholThreads, 1) k_chol_ref(Dev P, const do
 #pragma unroll
                     for (int k = 0; k < 8; ++k) {
                         if (k >= nr) break;
-                        asm volatile("bar.sync %0, 192;" ::"r"(3 + k) : "memory");
+                        named_sync<192>(3 + k);
                         if (s_neg[k]) break;
                         if (m <= 0) continue;
                         const double r = __dmul_rn(s_inv[r0 + k], num);
@@ -658,7 +657,7 @@ __global__ void __launch_bounds__(kRefCholThreads, 1) k_chol_ref(Dev P, const do
                     const bool any = (s & ~3) < ns;              // the warp has columns
                     double tail = 0.0, num = __dsub_rn(h, L);
                     for (int k = 0; k < nr; ++k) {
-                        asm volatile("bar.sync %0, 192;" ::"r"(3 + k) : "memory");
+                        named_sync<192>(3 + k);
                         if (s_neg[k]) break;
                         if (!any) continue;
                         double r = __dmul_rn(s_inv[r0 + k], num);
