@@ -263,6 +263,12 @@ int fednl_gpu_optionb_solve32(const double* H, int32_t d, int32_t lda, double l,
  * from the hardware sqrt and 1.0 / x. */
 int fednl_gpu_selftest_rn(int64_t n, uint64_t seed, int64_t* sqrt_mismatches, int64_t* rcp_mismatches);
 
+/* Self-test of a solve whose wait for another CTA's values runs out: (I + I) dx = 1, x -= dx with every such
+ * wait cut to `limit` (0: the kernels' own bounds, about a second; < 0: at once), by the FP64 cooperative solve
+ * or (fp32 != 0) the FP32 one, whose waits keep their bounds.  The launch's status (FEDNL_OK or FEDNL_ETIMEOUT) and how many entries of x
+ * changed: all of them, or none. */
+int fednl_gpu_selftest_lost_wait(int32_t d, int32_t fp32, int32_t limit, int32_t* status, int32_t* changed);
+
 /* Measurement of this GPU's FP64 pipe (no counterpart in the reference; the denominator of the FP64
  * kernels' roofline): lane operations per second of dependent FP64 fma and add chains with all SMs
  * full of warps (8 chains a thread), in G op/s, and the clock cycles of one dependent FP64 add in a

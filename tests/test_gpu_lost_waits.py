@@ -1,0 +1,25 @@
+"""A wait inside a solve that runs out gives FEDNL_ETIMEOUT and leaves the iterate as it was: the FP64 back
+substitution with its blocks in one CTA and over several.  The waits are cut to nothing; every one still ends by itself."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def gpu():
+    from ufednl_gb300 import build, fednl
+    build.build()
+    fednl.load()
+    return fednl
+
+
+@pytest.mark.parametrize("fp32,d", [(False, 64), (False, 129), (False, 301), (False, 1024)])
+def test_x_stays_when_a_wait_runs_out(gpu, fp32, d):
+    for _ in range(3):
+        assert gpu.selftest_lost_wait(d, fp32, -1) == (-5, 0)
+        assert gpu.selftest_lost_wait(d, fp32, 0) == (0, d)
+
+
+@pytest.mark.parametrize("fp32,d", [(False, 1), (False, 31)])
+def test_solves_without_such_waits(gpu, fp32, d):
+    assert gpu.selftest_lost_wait(d, fp32, -1) == (0, d)

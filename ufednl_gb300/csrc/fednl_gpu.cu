@@ -248,6 +248,7 @@ int fednl_solve_batch_launch(const FednlSolveDesc* descs, int n, void* stream)
             J.P.ls = S.ls;
             J.P.round_ctr = S.round_ctr;
             J.P.hist_cap = S.hist_cap;
+            J.P.wait_limit = S.wait_limit;
             J.Hin = S.H;
             J.hin_lda = 0;
             J.lptr = S.lptr;
@@ -437,6 +438,7 @@ int fednl_device_optionb_solve32(const FednlSolveDesc& S, const FednlSolve32& E,
     P.ls = S.ls;
     P.round_ctr = S.round_ctr;
     P.hist_cap = S.hist_cap;
+    P.wait_limit = S.wait_limit;
     if (grid == 0) grid = chol32c_grid(S.d);
     C32Plan plan = chol32c_plan(S.d, grid < 0 ? -grid : 16);
     const size_t smem = plan.smem;
@@ -3017,6 +3019,82 @@ int fednl_gpu_selftest_rn(int64_t n, uint64_t seed, int64_t* sqrt_mismatches, in
     if (e != cudaSuccess) return fail(FEDNL_ECUDA, "self-test kernel failed: %s", cudaGetErrorString(e));
     *sqrt_mismatches = (int64_t)h[0];
     *rcp_mismatches = (int64_t)h[1];
+    return FEDNL_OK;
+}
+
+// ---- self-test of the solves' lost waits -------------------------------------------------------
+// (I + I) dx = 1 with x = 1, 2, ..: a wait that ran out must leave x as it was
+int fednl_gpu_selftest_lost_wait(int32_t d, int32_t fp32, int32_t limit, int32_t* status, int32_t* changed)
+{
+    int rc = ensure_device();
+    if (rc) return rc;
+    if (d < 1 || d > kC32MaxD || !status || !changed) return fail(FEDNL_EINVAL, "bad argument");
+    const size_t U = (size_t)d * (d + 1) / 2, ld = (size_t)c32c_ld(d);
+    Scratch s;
+    CK(cudaStreamCreateWithFlags(&s.st, cudaStreamNonBlocking));
+    FednlSolveDesc S{};
+    FednlSolve32 E{};
+    double *H, *g, *l;
+    float *hh, *hl, *rh, *rl;
+    s.a.want(&H, U);
+    s.a.want(&g, d);
+    s.a.want(&l, 1);
+    s.a.want(&S.dx, d);
+    s.a.want(&S.xupd, d);
+    s.a.want(&S.work, fednl_chol_work_elems(d));
+    s.a.want(&S.ybuf, d);
+    s.a.want(&S.rinv, d);
+    s.a.want(&S.bar, 4);
+    s.a.want(&S.status, 1);
+    s.a.want(&S.stats, 4);
+    s.a.want(&E.a, ld * ld);
+    s.a.want(&E.diag0, d);
+    s.a.want(&E.linv, ld * 32);
+    s.a.want(&E.r, d);
+    s.a.want(&E.acc, d);
+    s.a.want(&E.accp, 2 * (size_t)d);
+    s.a.want(&E.flag, 1);
+    s.a.want(&hh, U);
+    s.a.want(&hl, U);
+    s.a.want(&rh, U);
+    s.a.want(&rl, U);
+    rc = s.a.commit();
+    if (rc) return rc;
+    std::vector<double> hH(U, 0.0), x0(d), x1(d), ones(d, 1.0);
+    for (int j = 0; j < d; ++j) {
+        hH[(size_t)j * (j + 1) / 2 + j] = 1.0;
+        x0[j] = j + 1.0;
+    }
+    CK(cudaMemcpyAsync(H, hH.data(), U * 8, cudaMemcpyHostToDevice, s.st));
+    CK(cudaMemcpyAsync(g, ones.data(), d * 8, cudaMemcpyHostToDevice, s.st));
+    CK(cudaMemcpyAsync(l, ones.data(), 8, cudaMemcpyHostToDevice, s.st));
+    CK(cudaMemcpyAsync(S.xupd, x0.data(), d * 8, cudaMemcpyHostToDevice, s.st));
+    CK(cudaMemsetAsync(S.bar, 0, 16, s.st));
+    CK(cudaMemsetAsync(S.status, 0, 4, s.st));
+    S.H = H;
+    S.d = d;
+    S.lptr = l;
+    S.g = g;
+    S.wait_limit = limit;
+    if (fp32) {
+        k_split_pairs<<<(unsigned)((U + 255) / 256), 256, 0, s.st>>>(H, d, hh, hl, rh, rl);
+        CKL();
+        E.hh = hh;
+        E.hl = hl;
+        E.rh = rh;
+        E.rl = rl;
+        E.refine = 2;
+        E.tol = 0x1p-30f;
+        rc = fednl_device_optionb_solve32(S, E, s.st, 0);
+    } else {
+        rc = fednl_solve_batch_launch(&S, 1, s.st);
+    }
+    if (rc) return fail(rc, "solve launch failed");
+    CK(cudaStreamSynchronize(s.st));
+    CK(cudaMemcpy(status, S.status, 4, cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(x1.data(), S.xupd, d * 8, cudaMemcpyDeviceToHost));
+    *changed = 0;
+    for (int j = 0; j < d; ++j) *changed += x1[j] != x0[j];
     return FEDNL_OK;
 }
 

@@ -76,6 +76,7 @@ struct Dev {
     int* status;            // [1]
     double* stats;          // [2] ||g||, l
     int hist_cap;
+    int wait_limit;         // polls after which a solve's wait for another CTA's value runs out; 0: the built-in bound, < 0: at once
     unsigned* bar;          // [4] grid barrier: arrival count with error flag, finished CTAs (two spare)
     // FedNL-PP (bin_fednl_local_pp); act == nullptr: every client takes part (plain FedNL)
     int pp, n_act;          // n_act: clients processed this round (tau, or nc without PP)
@@ -2202,10 +2203,12 @@ constexpr long long kNotYet = 0xfff8dead5eedbeefll;
 
 __device__ __forceinline__ bool is_not_yet(double v) { return __double2hiint(v) == (int)(kNotYet >> 32); }
 
-// `own`: the warp's block (0 is the bottom one); blocks from `first` on are this CTA's; false: a wait ran out
+// `own`: the warp's block (0 is the bottom one); blocks from `first` on are this CTA's.  False: a wait ran out (of
+// `spins` polls), and the block hands nothing on, so that the blocks above it fail as well: the top block
+// succeeds only if all do.
 __device__ __forceinline__ bool back_block(const double* A, int d, int own, int first,
                                            double (*s_back)[32], volatile double* s_far, double* ybuf, double* dxout,
-                                           double* xupd)
+                                           int spins)
 {
     const int lane = threadIdx.x & 31;
     const int b1 = d - 32 * own, b0 = max(0, b1 - 32), nbk = b1 - b0, row = b0 + lane;
@@ -2215,7 +2218,6 @@ __device__ __forceinline__ bool back_block(const double* A, int d, int own, int 
     // (a single block of fewer than 32 rows) are not read.
     const double* Ar = A + (mine ? row : b0);
     double v = mine ? Ar[(size_t)d * (d + 1) / 2] : 0.0;           // 0 on the lanes past the block
-    const double x = mine && xupd ? xupd[row] : 0.0;
     double cur[32];
     auto first_col = [&](int q) { return max(0, d - 32 * (q + 1)); };
 #pragma unroll
@@ -2238,7 +2240,7 @@ __device__ __forceinline__ bool back_block(const double* A, int d, int own, int 
             if (far) {                            // eight values to the warp's own shared memory
                 for (int spin = 0; (__ballot_sync(0xffffffffu, !is_not_yet(y)) >> c & 255u) != 255u && ok; ++spin) {
                     y = remote(q);
-                    ok = spin < kBackSpins;
+                    ok = spin < spins;
                 }
                 s_far[lane] = y;
                 __syncwarp();
@@ -2247,13 +2249,13 @@ __device__ __forceinline__ bool back_block(const double* A, int d, int own, int 
             }
             if (!far && q + 1 < own)              // only the next block's warp keeps pace value by value: all of
                                                   // them at once would queue before the solving warp
-                for (int spin = 0; is_not_yet(from[c]) && ok; ++spin) ok = spin < kBackSpins;
+                for (int spin = 0; is_not_yet(from[c]) && ok; ++spin) ok = spin < spins;
 #pragma unroll
             for (int s = c + 7; s >= c; --s) {
                 double t = from[s];
                 for (int spin = 0; is_not_yet(t) && ok; ++spin) {
                     t = from[s];
-                    ok = spin < kBackSpins;
+                    ok = spin < spins;
                 }
                 v = fma(-cur[s], t, v);
                 cur[s] = *next;                   // of the next block, beside the operations
@@ -2262,6 +2264,7 @@ __device__ __forceinline__ bool back_block(const double* A, int d, int own, int 
             if (far) __syncwarp();
         }
     }
+    if (!__all_sync(0xffffffffu, ok)) return false;
     // the triangle; every lane stores the broadcast y_t for the CTA's other warps (a store by one lane is a
     // divergent branch on the chain), and eight lanes at a time their own for other CTAs
     const uint32_t near = (uint32_t)__cvta_generic_to_shared(&s_back[own - first][0]);
@@ -2289,11 +2292,8 @@ __device__ __forceinline__ bool back_block(const double* A, int d, int own, int 
             }
         }
     publish(0);
-    if (mine) {
-        if (dxout) dxout[row] = v;
-        if (xupd) xupd[row] = __dsub_rn(x, v);
-    }
-    return ok;
+    if (mine && dxout) dxout[row] = v;
+    return true;
 }
 
 // Hin is the packed upper triangle, or (hin_lda > 0) a column-major matrix with that leading
@@ -2664,18 +2664,30 @@ __device__ __forceinline__ void chol_body(const Dev& P, const double* __restrict
         // L^T dx = z (z in column d)
         const int nblocks = (d + 31) / 32, ngroups = (nblocks + kBackWarps - 1) / kBackWarps;
         const bool norm_here = bid == (G > (unsigned)ngroups ? (unsigned)ngroups : 0u);
-        bool lost = false;
+        __shared__ int s_lost;
+        if (tid == 0) s_lost = 0;
         for (int grp = (int)bid; grp < ngroups; grp += (int)G) {
             if (tid < 32 * kBackWarps) s_back[warp][lane] = __longlong_as_double(kNotYet);
             __syncthreads();
             const int own = grp * kBackWarps + warp;
-            if (warp < kBackWarps && own < nblocks) {
-                lost |= !back_block(A, d, own, grp * kBackWarps, s_back, s_far[warp], P.ybuf, dxout, xupd);
-                if (P.ls && own == nblocks - 1 && lane == 0) P.ls[4] = lost ? 0.0 : 1.0;
+            if (warp < kBackWarps && own < nblocks &&
+                !back_block(A, d, own, grp * kBackWarps, s_back, s_far[warp], P.ybuf, dxout,
+                            P.wait_limit ? P.wait_limit : kBackSpins) && lane == 0) {
+                s_lost = 1;
+                *P.status = -5;
             }
             __syncthreads();
         }
-        if (lost && lane == 0) *P.status = -5;
+        // The top block's CTA has seen every value.  x -= dx there, all of it or, when a wait ran out, none
+        if ((int)bid == (ngroups - 1) % (int)G && !s_lost) {
+            if (P.ls && tid == 0) P.ls[4] = 1.0;
+            if (xupd)
+                for (int i = tid; i < d; i += blockDim.x) {
+                    double y;
+                    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=d"(y) : "l"(P.ybuf + i) : "memory");
+                    xupd[i] = __dsub_rn(xupd[i], y);
+                }
+        }
         if (record && norm_here) {   // ||g|| for the round statistics, in a CTA without rows if there is one
             double gs = 0.0;
             for (int i = tid; i < d; i += blockDim.x) gs += gin[i] * gin[i];

@@ -31,6 +31,8 @@ struct FednlSolveDesc {
     int* round_ctr;
     int hist_cap;
     int record;
+    int wait_limit;        // polls after which a wait inside the FP64 solve runs out;
+                           // 0: the kernel's own bound (about a second), < 0: at once (the self-test)
 };
 
 // fednl_gpu.cu
