@@ -2204,8 +2204,8 @@ constexpr long long kNotYet = 0xfff8dead5eedbeefll;
 __device__ __forceinline__ bool is_not_yet(double v) { return __double2hiint(v) == (int)(kNotYet >> 32); }
 
 // `own`: the warp's block (0 is the bottom one); blocks from `first` on are this CTA's.  False: a wait ran out (of
-// `spins` polls), and the block hands nothing on, so that the blocks above it fail as well: the top block
-// succeeds only if all do.
+// `spins` polls), and the block hands nothing on but kNotYet, so that the blocks above it fail as well: the top
+// block succeeds only if all do.  (A return there instead: the solve of a round at d = 301 242 -> 246 us.)
 __device__ __forceinline__ bool back_block(const double* A, int d, int own, int first,
                                            double (*s_back)[32], volatile double* s_far, double* ybuf, double* dxout,
                                            int spins)
@@ -2264,11 +2264,13 @@ __device__ __forceinline__ bool back_block(const double* A, int d, int own, int 
             if (far) __syncwarp();
         }
     }
-    if (!__all_sync(0xffffffffu, ok)) return false;
+    ok = __all_sync(0xffffffffu, ok);
     // the triangle; every lane stores the broadcast y_t for the CTA's other warps (a store by one lane is a
     // divergent branch on the chain), and eight lanes at a time their own for other CTAs
     const uint32_t near = (uint32_t)__cvta_generic_to_shared(&s_back[own - first][0]);
-    auto known = [](double a) { return is_not_yet(a) ? __longlong_as_double(0x7ff8000000000000ll) : a; };
+    auto known = [&](double a) {
+        return !ok ? __longlong_as_double(kNotYet) : is_not_yet(a) ? __longlong_as_double(0x7ff8000000000000ll) : a;
+    };
     auto publish = [&](int lo) {                  // rows lo .. lo + 7 of the block are final
         asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t"
                      "@p st.relaxed.gpu.global.f64 [%0], %1;\n\t}" ::"l"(ybuf + row),
@@ -2292,8 +2294,8 @@ __device__ __forceinline__ bool back_block(const double* A, int d, int own, int 
             }
         }
     publish(0);
-    if (mine && dxout) dxout[row] = v;
-    return true;
+    if (mine && ok && dxout) dxout[row] = v;
+    return ok;
 }
 
 // Hin is the packed upper triangle, or (hin_lda > 0) a column-major matrix with that leading
@@ -2664,27 +2666,25 @@ __device__ __forceinline__ void chol_body(const Dev& P, const double* __restrict
         // L^T dx = z (z in column d)
         const int nblocks = (d + 31) / 32, ngroups = (nblocks + kBackWarps - 1) / kBackWarps;
         const bool norm_here = bid == (G > (unsigned)ngroups ? (unsigned)ngroups : 0u);
-        __shared__ int s_lost;
-        if (tid == 0) s_lost = 0;
+        bool lost = false;
         for (int grp = (int)bid; grp < ngroups; grp += (int)G) {
             if (tid < 32 * kBackWarps) s_back[warp][lane] = __longlong_as_double(kNotYet);
             __syncthreads();
             const int own = grp * kBackWarps + warp;
-            if (warp < kBackWarps && own < nblocks &&
-                !back_block(A, d, own, grp * kBackWarps, s_back, s_far[warp], P.ybuf, dxout,
-                            P.wait_limit ? P.wait_limit : kBackSpins) && lane == 0) {
-                s_lost = 1;
-                *P.status = -5;
-            }
+            if (warp < kBackWarps && own < nblocks)
+                lost |= !back_block(A, d, own, grp * kBackWarps, s_back, s_far[warp], P.ybuf, dxout,
+                                    P.wait_limit ? P.wait_limit : kBackSpins);
+            if (warp < kBackWarps && own == nblocks - 1 && P.ls && lane == 0) P.ls[4] = lost ? 0.0 : 1.0;
             __syncthreads();
         }
-        // The top block's CTA has seen every value.  x -= dx there, all of it or, when a wait ran out, none
-        if ((int)bid == (ngroups - 1) % (int)G && !s_lost) {
-            if (P.ls && tid == 0) P.ls[4] = 1.0;
+        if (lost && lane == 0) *P.status = -5;
+        // The top block's CTA has seen every value: x -= dx there, all of it or, when a wait ran out, none (at
+        // d = 301 0.7 us more than each block for its own rows, which nothing could take back)
+        if ((int)bid == (ngroups - 1) % (int)G && !__syncthreads_or(lost)) {
             if (xupd)
-                for (int i = tid; i < d; i += blockDim.x) {
+                for (int i = tid; i < d; i += kCoopThreads) {
                     double y;
-                    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=d"(y) : "l"(P.ybuf + i) : "memory");
+                    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=d"(y) : "l"(P.ybuf + i));
                     xupd[i] = __dsub_rn(xupd[i], y);
                 }
         }
