@@ -1,5 +1,6 @@
 """A wait inside a solve that runs out gives FEDNL_ETIMEOUT and leaves the iterate as it was: the FP64 back
-substitution with its blocks in one CTA and over several.  The waits are cut to nothing; every one still ends by itself."""
+substitution with its blocks in one CTA and over several, and the FP32 solves on one cluster (d up to 512) and
+on two of a grid.  The waits are cut to nothing; every one still ends by itself."""
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -13,13 +14,14 @@ def gpu():
     return fednl
 
 
-@pytest.mark.parametrize("fp32,d", [(False, 64), (False, 129), (False, 301), (False, 1024)])
+@pytest.mark.parametrize("fp32,d", [(False, 64), (False, 129), (False, 301), (False, 1024),
+                                    (True, 350), (True, 512), (True, 640), (True, 1024)])
 def test_x_stays_when_a_wait_runs_out(gpu, fp32, d):
     for _ in range(3):
         assert gpu.selftest_lost_wait(d, fp32, -1) == (-5, 0)
         assert gpu.selftest_lost_wait(d, fp32, 0) == (0, d)
 
 
-@pytest.mark.parametrize("fp32,d", [(False, 1), (False, 31)])
+@pytest.mark.parametrize("fp32,d", [(False, 1), (False, 31), (True, 31), (True, 301)])
 def test_solves_without_such_waits(gpu, fp32, d):
     assert gpu.selftest_lost_wait(d, fp32, -1) == (0, d)

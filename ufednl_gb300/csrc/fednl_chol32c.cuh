@@ -48,6 +48,7 @@ struct Chol32c {
     int smem_floats;   // dynamic shared memory of the launch, in floats
     int cluster;       // the launch is one thread-block cluster (cluster barriers)
     int solve_cluster; // CTAs of the clusters that run the solves (0: CTA 0 runs them)
+    long long wait_cycles;  // bound of a wait for a block (< 0: none is waited for)
 };
 
 __host__ __device__ inline int c32c_ld(int d) { return (d + 31) & ~31; }
@@ -300,11 +301,13 @@ struct C32Cluster {
     int n, rank;                  // CTAs of the cluster, this one
     int own[kC32Own];             // its blocks, ascending (past the last: nblk)
     uint64_t* mb;                 // [nblk] one per block: 128 bytes arrive a solve
-    bool lost;                    // a wait ran out (its data are not valid; the caller reports it)
+    bool lost;                    // a wait of this thread ran out (its data are not valid; the caller reports it)
+    long long limit;              // cycles a wait takes at most
 
-    __device__ void init(int nblk, int n_, bool last_first, uint64_t* bars)
+    __device__ void init(int nblk, int n_, bool last_first, uint64_t* bars, long long limit_)
     {
         n = n_;
+        limit = limit_;
         rank = (int)c32c_cluster_rank();
         mb = bars;
         lost = false;
@@ -345,9 +348,19 @@ struct C32Cluster {
     }
     __device__ void wait(int b, int phase)
     {
-        if (lost) return;
-        const uint32_t a = (uint32_t)__cvta_generic_to_shared(mb + b);
+        if (!lost) lost = limit < 0 || !arrived(b, phase, clock64(), limit);
+    }
+    // After a lost wait the others' blocks are still on their way: no next solve and no exit before they are
+    // here (or the bound has passed)
+    __device__ void drain(int nblk, int phase)
+    {
+        if (!lost) return;
         const long long t0 = clock64();
+        for (int b = 0; b < nblk; ++b) arrived(b, phase, t0, kC32WaitCycles);
+    }
+    __device__ bool arrived(int b, int phase, long long t0, long long cycles)
+    {
+        const uint32_t a = (uint32_t)__cvta_generic_to_shared(mb + b);
         for (;;) {
             uint32_t done;
             asm volatile("{\n\t.reg .pred p;\n\t"
@@ -356,11 +369,8 @@ struct C32Cluster {
                          : "=r"(done)
                          : "r"(a), "r"(phase)
                          : "memory");
-            if (done) return;
-            if (clock64() - t0 > kC32WaitCycles) {
-                lost = true;
-                return;
-            }
+            if (done) return true;
+            if (clock64() - t0 > cycles) return false;
         }
     }
 };
@@ -446,6 +456,7 @@ __device__ __forceinline__ void c32c_forward_cl(C32Cluster& K, int phase, const 
             s[n] = fmaf(a4.w, v4.w, s[n]);
         }
     }
+    K.drain(nblk, phase);
     K.arm(nblk);
 }
 
@@ -554,6 +565,7 @@ __device__ __forceinline__ void c32c_backward_cl(C32Cluster& K, int phase, const
         }
         K.wait(m, phase);
     }
+    K.drain(nblk, phase);
     K.arm(nblk);
     __syncthreads();
 }
@@ -936,14 +948,14 @@ __device__ __forceinline__ void chol32c_body(const Dev& P, const Chol32c& C, con
     if (n_cl) {
         const int nblk = (d + 31) / 32;
         if (my_cl == fwd_cl) {
-            KF.init(nblk, (int)n_cl, true, s_mb[0]);
+            KF.init(nblk, (int)n_cl, true, s_mb[0], C.wait_cycles);
             c32c_load_rows(C, KF, nblk, s_pre);
             if (!bwd_cl)
 #pragma unroll
                 for (int n = 0; n < kC32Own; ++n) cols += KF.own[n] < nblk ? (KF.own[n] + 1) * 1024 : 0;
         }
         if (my_cl == bwd_cl) {
-            KB.init(nblk, (int)n_cl, !bwd_cl, s_mb[1]);
+            KB.init(nblk, (int)n_cl, !bwd_cl, s_mb[1], C.wait_cycles);
             c32c_load_cols(C, KB, nblk, cols);
         }
         c32c_wait<0>();
@@ -955,12 +967,12 @@ __device__ __forceinline__ void chol32c_body(const Dev& P, const Chol32c& C, con
                 c32c_forward_cl(
                     KF, it & 1, s_pre, v, d, s_t, [&](int row) { return (float)(it == 0 ? g[row] : __ldcg(C.r + row)); },
                     C.accp);
-                if (KF.lost) *P.status = -5;
+                if (KF.lost) gs.give_up();
             }
             if (!gs.sync()) return c32c_timeout(P, C, bid, record);
             if (my_cl == bwd_cl) {
                 c32c_backward_cl(KB, it & 1, cols, v, d, s_part, s_t, C.accp);
-                if (KB.lost) *P.status = -5;
+                if (KB.lost) gs.give_up();
             }
         }
         if (bid == leader) {
@@ -1046,6 +1058,15 @@ __device__ __forceinline__ void chol32c_body(const Dev& P, const Chol32c& C, con
     }
     if (n_cl) c32c_cluster_sync();          // no CTA leaves while another of its cluster may write to it
     if (bid != leader) return;
+    if (n_cl && gs.given_up()) {            // a wait of the solves ran out: x stays
+        __syncthreads();
+        if (tid == 0) {
+            *P.status = -5;
+            if (record) *P.round_ctr += 1;
+            if (gs.cluster) atomicExch(gs.bar, 0u);      // (else finish() does)
+        }
+        return;
+    }
     __syncthreads();
     double gn = 0.0;
     for (int i = tid; i < d; i += kCoopThreads) {

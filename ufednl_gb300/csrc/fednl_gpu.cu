@@ -459,7 +459,8 @@ int fednl_device_optionb_solve32(const FednlSolveDesc& S, const FednlSolve32& E,
         grid = 16 * std::min(plan.clusters[16], grid / 16);
     }
     Chol32c C{E.a,  E.diag0, E.linv, E.r,     E.acc,   E.accp, E.hh, E.hl,         E.rh,
-              E.rl, E.flag,  c32c_ld(S.d), E.refine, E.tol, res,    (int)(smem / 4), cl ? 1 : 0, ncl};
+              E.rl, E.flag,  c32c_ld(S.d), E.refine, E.tol, res,    (int)(smem / 4), cl ? 1 : 0, ncl,
+              S.wait_limit ? S.wait_limit : kC32WaitCycles};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kCoopThreads);

@@ -2174,6 +2174,11 @@ struct GridSync {
         return s_ok != 0;
     }
 
+    // A wait other than the barrier's ran out: every later sync() fails, and given_up() holds in whoever is
+    // ordered behind the call (the cluster's barrier itself, which carries no flag, goes on).
+    __device__ void give_up() { atomicOr(bar, kBarrierError); }
+    __device__ bool given_up() const { return (*(volatile unsigned*)bar & kBarrierError) != 0u; }
+
     __device__ void finish()
     {
         if (cluster) return;

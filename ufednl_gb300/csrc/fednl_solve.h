@@ -31,8 +31,8 @@ struct FednlSolveDesc {
     int* round_ctr;
     int hist_cap;
     int record;
-    int wait_limit;        // polls after which a wait inside the FP64 solve runs out;
-                           // 0: the kernel's own bound (about a second), < 0: at once (the self-test)
+    int wait_limit;        // polls (FP64) or cycles (FP32) after which a wait inside the solve runs out;
+                           // 0: the kernels' own bounds (about a second), < 0: at once (the self-test)
 };
 
 // fednl_gpu.cu
