@@ -580,6 +580,7 @@ struct fednl_handle_s {
     int hess_nt = kHessThreads;        // chosen: threads per block
     size_t hess_smem_sm = 0, hess_smem_gl = 0;   // bytes with the masks staged (0: they do not fit) / read from global
     bool hits_ready = false;           // common-sample lists built at upload (k_hess_hits)
+    bool one_client = false;           // the client oracle is one kernel (k_client_binary)
     int hits_maxrec = 0;               // most multi-sample records in one segment
     double hess_ms = 0.0;              // tuned shape's measured launch time (0: not tuned)
     int chol_grid = 1;
@@ -617,20 +618,6 @@ int mark(fednl_handle h, Marks* m, const char* name)
 // intercept's sums
 int client_threads(int d) { return std::min(1024, std::max(128, (2 * d + 31) / 32 * 32 + 32)); }
 
-// The client oracle of {0,1} features in the fixed order runs as one kernel, a CTA per client, as long as
-// all CTAs are resident at once; past that its short-lived CTAs queue, and the margins go to a thread per
-// sample over all clients and the sums to k_grad_binary (same operations, same values).  A FedNL-PP round
-// at d = 69, one kernel against two: 2048 clients of 6 samples 149 / 141 us, of 16 164 / 156, of 32
-// 182 / 186, of 48 215 / 209, of 100 270 / 262; 512 clients of 6 113 / 119, of 64 145 / 147; 128 clients
-// of 6 108 / 115; d = 301, 142 clients of 20 414 / 424.
-bool one_client_kernel(fednl_handle h)
-{
-    int dev = 0, sms = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return h->binary && !h->dev.ref && (long long)h->nc * client_threads(h->d) <= sms * 2048ll;
-}
-
 // CTAs of the round's solve: the factorization's, but no more than four selection words a CTA in its merge,
 // as far as the SMs go, so that a word's FP64 chain over the clients has the SM's unit nearly to itself (d =
 // 25, 126 clients, RandK k = 25: one CTA 57 us, three 38, Natural 115 and 64; d = 60, seven CTAs 65, fifteen
@@ -646,6 +633,26 @@ int round_grid(fednl_handle h)
 
 // dynamic shared memory of k_client_binary: the weights and the intercept's word sums
 size_t client_smem(fednl_handle h) { return (size_t)h->maxn * 16 + (size_t)((h->maxn + 63) / 64) * 16; }
+
+// Whether the client oracle of {0,1} features in the fixed order runs as one kernel, a CTA per client, or as
+// two: the margins a thread per sample over all clients, then the sums (k_grad_binary; the same operations and
+// values).  Two pay where more clients than CTAs are resident at once (10 CTAs an SM at d = 24, 7 at 69, 4 at
+// 124) have few samples: a CTA is then mostly its start-up, and the CTAs queue.  A FedNL-PP round, us, one / two:
+// d = 69, 1100 clients of 6 samples 128 / 123, 1800 135 / 131, 2048 143 / 133, 4500 199 / 174, 2048 of 16
+// 147 / 139, of 32 164 / 162, of 64 201 / 201; d = 24, 4500 of 6 139 / 119, of 32 154 / 156; d = 124, 2048 of 16
+// 205 / 192, of 32 223 / 217.  With more samples a client's word-parallel sums win: d = 69, 1800 of 32 154 / 160,
+// of 128 231 / 252, of 400 420 / 493, of 600 569 / 686; d = 24, 2500 of 256 258 / 315; d = 124, 1200 of 400
+// 427 / 477 (from 65 to 100 samples, a second word of 64 hardly begun, two may be up to 10 % ahead).  While all
+// clients are resident one is: d = 69, 700 of 6 108 / 115, 512 of 400 381 / 405; d = 301, 304 of 400 1434 / 1482.
+int choose_client_kernel(fednl_handle h, bool* one)
+{
+    int dev = 0, sms = 1, bps = 1;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_client_binary, client_threads(h->d), client_smem(h)));
+    *one = !h->dev.ref && ((long long)h->nc <= (long long)sms * bps || h->S > 16ll * h->nc);
+    return FEDNL_OK;
+}
 
 // The binary Hessian's kernels: attribute masks intersected every round (staged in shared memory
 // or read from global memory), or the common-sample lists built at upload.
@@ -772,7 +779,7 @@ int launch_round(fednl_handle h, Marks* M = nullptr, bool client_phase_only = fa
         if (rc) return rc;
         CK(cudaEventRecord(h->join_ev, h->side));
     }
-    if (one_client_kernel(h)) {      // the client oracle in one launch
+    if (h->one_client) {             // the client oracle in one launch
         MARK("k_client_binary");
         k_client_binary<<<h->nc, client_threads(h->d), client_smem(h), st>>>(P);
         CKL();
@@ -918,7 +925,7 @@ int launch_round(fednl_handle h, Marks* M = nullptr, bool client_phase_only = fa
     const fednl_problem_desc& D = h->desc;
     const double* lptr = D.option_a ? nullptr : P.stats + 1;      // Option A: H + lambda I
     // barrier words and error flag start at zero (the binary client oracle zeroes them at the round's start)
-    if (!one_client_kernel(h)) CK(cudaMemsetAsync(P.bar, 0, 4 * sizeof(unsigned), st));
+    if (!h->one_client) CK(cudaMemsetAsync(P.bar, 0, 4 * sizeof(unsigned), st));
     if (P.ref) {
         MARK("k_chol_ref");
         CK(launch_chol_ref(P, h->ref_grid, st, lptr, P.lambda, P.dx, D.line_search ? nullptr : P.x, 1));
@@ -1558,6 +1565,8 @@ static int install_binary(fednl_handle h, const std::vector<int>& rowptr, const 
     CK(raise_hess_smem(h));
     if ((size_t)h->maxn * 16 > 48 * 1024) CK(fednl_raise_dyn_smem((const void*)k_grad_binary, (size_t)h->maxn * 16));
     if (client_smem(h) > 48 * 1024) CK(fednl_raise_dyn_smem((const void*)k_client_binary, client_smem(h)));
+    rc = choose_client_kernel(h, &h->one_client);
+    if (rc) return rc;
     h->binary = 1;
     return FEDNL_OK;
 }
@@ -1577,6 +1586,7 @@ static void clear_client_data(fednl_handle h)
     P.hrec = nullptr;
     P.hhits = nullptr;
     h->hits_ready = false;
+    h->one_client = false;
 }
 
 // after either upload: labels, readiness, and the captured round (its launch shapes may change)
