@@ -1221,7 +1221,10 @@ __device__ __forceinline__ void select_norms(const SelectDraws& dr, const double
 // the eight lanes; warp 2 the two scalars.  d = 301: 5681 dependent adds at 86 cycles, 237 us beside the
 // walk, against 346 us for a kernel of its own before it (the round 1617 -> 1453 us).
 constexpr int kFrobCols = 4;
-constexpr int kFrobAhead = 13;       // loads of a staging thread kept a step ahead (4 d entries over 96 threads)
+// Loads of a staging thread kept a step ahead, the columns' others in line.  The adders' chains hide either at
+// any d: depths of 2 to 24 differ by 1 % or less from d = 124 to 1024 (d = 301 400-407 us a launch, 400 557-565,
+// 1024 2543-2554; the norm in a kernel of its own 563, 797 and 3346), so no more registers than four.
+constexpr int kFrobAhead = 4;
 constexpr int kFrobStagers = 96;
 
 __device__ __forceinline__ void select_frob_ref(double* ring, const double* __restrict__ v, int d, int c, double* F,
