@@ -2221,11 +2221,10 @@ __device__ __forceinline__ bool back_block(const double* A, int d, int own, int 
     const int lane = threadIdx.x & 31;
     const int b1 = d - 32 * own, b0 = max(0, b1 - 32), nbk = b1 - b0, row = b0 + lane;
     const bool mine = lane < nbk;
-    // Entry (row, c0 + s) of block q's columns [c0, c0 + 32).  Lanes past the block and, in the own block,
-    // entries below the diagonal read other entries of A, which no kept value takes; columns past d - 1
-    // (a single block of fewer than 32 rows) are not read.
+    // Entry (row, c0 + s) of block q's columns [c0, c0 + 32).  Lanes past the block go along on row b0's entries;
+    // columns past d - 1 (a single block of fewer than 32 rows) are not read.
     const double* Ar = A + (mine ? row : b0);
-    double v = mine ? Ar[(size_t)d * (d + 1) / 2] : 0.0;           // 0 on the lanes past the block
+    double v = mine ? Ar[(size_t)d * (d + 1) / 2] : 0.0;
     double cur[32];
     auto first_col = [&](int q) { return max(0, d - 32 * (q + 1)); };
 #pragma unroll
@@ -2285,7 +2284,9 @@ __device__ __forceinline__ bool back_block(const double* A, int d, int own, int 
                      "d"(known(v)), "r"((unsigned)(mine && lane >= lo && lane < lo + 8))
                      : "memory");
     };
-    if (nbk < 32) {                               // rows past the block: y = 0 on entries of 0
+    if (nbk < 32) {                               // rows past the block: y = 0 on entries of 0 (their v is of
+                                                  // row b0's entries so far, and 0 would not cancel an infinity)
+        v = mine ? v : 0.0;
 #pragma unroll
         for (int s = 0; s < 32; ++s)
             if (s >= nbk) cur[s] = 0.0;
