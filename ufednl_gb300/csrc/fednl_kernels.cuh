@@ -663,8 +663,8 @@ __global__ void __launch_bounds__(NT) k_hess_binary(Dev P, int mode)
             // Per 32 mask words: pass 1, without branches, finds the words holding samples with
             // both attributes set; pass 2 sums over those words only, in sample order.  The sum's
             // first term is 0 + D_s = D_s exactly (D_s >= 0), so it costs no FP64 add: on this part
-            // a warp's FP64 instruction takes the pipe for ~64 cycles however few lanes are active,
-            // and most entries have at most one sample with both attributes set
+            // an FP64 instruction takes a warp 64 cycles and the SM's unit 19, however few lanes are
+            // active, and most entries have at most one sample with both attributes set
             h = 0.0;
             bool first = true;
             for (int w0 = 0; w0 < W; w0 += 32) {
@@ -1140,17 +1140,17 @@ __device__ __forceinline__ void master_l(const MasterAgg& A, int lane)
 // Work fused into k_select.  TopLEK's rounding draws: the launch's last CTA to finish (counted on
 // ctr, which it returns to zero) makes every worker's draws (k_toplek_rng's work) once all clients'
 // window flags are written; ctr == nullptr: no draws in this launch.  The master's aggregation
-// (agg.gc != nullptr): CTA 0's three other warps form l and g while its first warp walks the heap.
+// (agg.gc != nullptr): CTA 0's seven other warps form l and g while its first warp walks the heap.
 struct SelectDraws {
     unsigned* ctr;
     int n_mat, W;
     unsigned* wstate;
     MasterAgg agg;
-    // norms != 0: warps 1-3 form the client's ||diff||_F^2 (F, its segment sums in fpart) and Lk
+    // norms != 0: six warps form the client's ||diff||_F^2 (F, its segment sums in fpart) and Lk (select_norms)
     int norms, nseg;
     double* fpart;     // [n_mat][nseg]
     double* lk;        // [n_mat]
-    // frob != 0: these warps form the reference order's ||diff||_F^2 and Lk instead (select_frob_ref), in
+    // frob != 0: five warps form the reference order's ||diff||_F^2 and Lk instead (select_frob_ref), in
     // a ring of 2 kFrobCols columns of `frob` = d entries at the end of the dynamic shared memory
     int frob;
 };
@@ -1966,20 +1966,20 @@ __device__ __forceinline__ size_t up_pos(int i, int j) { return (size_t)j * (j +
 //   1. every CTA factors the kCholNB x kCholNB diagonal block redundantly in shared memory (no
 //      barrier needed; CTA 0 writes it back) and, in the same column loop, the panel rows of its
 //      own share of the columns right of the block (l_kj = a_kj (1 / d_k), then
-//      a_ij = fma(-l_ki, a_kj, a_ij) with a_kj unscaled); on GB300 a warp's FP64 instructions
-//      issue about once per 64 cycles and the correctly rounded reciprocal takes ~300 cycles, so
-//      the loop keeps the pivot chain short (two CTA barriers per column) and spreads the updates
-//      over all warps;
+//      a_ij = fma(-l_ki, a_kj, a_ij) with a_kj unscaled); on GB300 an FP64 operation takes a warp
+//      64 cycles (the SM's unit takes one every 19) and the correctly rounded reciprocal ~300, so
+//      one warp runs the pivots' chain, two columns a step and a step ahead, and the updates are
+//      spread over six others (one CTA barrier and one of the six a step);
 //   2. the panel's multipliers go to the packed factor and its unscaled rows right of the block to
-//      the work array's panel buffer; grid barrier, then all threads apply the panel to the
-//      trailing triangle entry by entry (a_ij = fma(-l_ki, a_kj, a_ij), k over the panel in
-//      order); grid barrier.
+//      the work array's panel buffer; grid barrier, then the CTAs apply the panel to the trailing
+//      triangle in tiles of 8 x 8 entries staged in shared memory (a_ij = fma(-l_ki, a_kj, a_ij), k
+//      over the panel in order); grid barrier.
 // Every entry undergoes exactly the operation sequence of the unblocked right-looking algorithm,
 // so the factor equals the CPU oracle's factor bit for bit.  g is appended as column d of the
 // packed matrix: the strips and trailing updates then carry out the forward substitution L y = g
 // (y_i = fma(-l_ti, y_t, y_i)), and the scaling of row t leaves z_t = y_t (1 / d_t) in column d.
-// The backward substitution L^T x = z (unit diagonal) runs in CTA 0, blocked by 32 rows, same
-// order as the oracle's.
+// The backward substitution L^T x = z (unit diagonal) streams over blocks of 32 rows, a warp each, on
+// as many CTAs as that takes (back_block), in the oracle's order.
 constexpr int kCholNB = 32;
 constexpr int kCholSlab = 8;                          // panel columns per CTA kept in shared memory
 constexpr int kCoopThreads = 256;
@@ -1987,8 +1987,8 @@ static_assert(kCholSlab == kCoopThreads / 32, "a warp loads one own column");
 constexpr long long kBarrierCycles = 4000000000ll;   // ~2 s at 2 GHz, then ETIMEOUT
 
 // ---- correctly rounded square root and reciprocal without the FP64 pipe ----------------------
-// On this part a warp's FP64 instructions (and 64-bit integer <-> float conversions) issue about once
-// per 64 cycles, and the hardware sequences for sqrt and 1/x cost about 720 and 355 cycles on the
+// On this part an FP64 instruction (or a conversion between 64-bit integers and floats) takes a warp 64
+// cycles, the next one waiting for it, and the hardware sequences for sqrt and 1/x cost about 720 and 355 cycles on the
 // Cholesky's pivot chain.  These give the same correctly rounded results from integer arithmetic:
 // an FP32 estimate, Newton steps whose residuals are computed exactly in 64-bit integers (converted
 // to FP32 through 32-bit integers only), and a final exact remainder test that decides the rounding.

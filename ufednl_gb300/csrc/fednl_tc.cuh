@@ -446,7 +446,7 @@ struct EpiDiff {
 
 // ---- mixed-precision round kernels (dense FP32 features, feature-major [nc][d][L]) ------------
 // Margins and gradients need FP64-grade sums (the final ||grad|| is ~1e-9 of terms of order 1), and
-// GB300 issues a warp's FP64 instruction about once per 64 cycles; both are therefore formed with
+// on GB300 an FP64 instruction takes a warp 64 cycles and the SM's unit 19; both are therefore formed with
 // FP32 pairs ("float-float"): each product x * (y_hi + y_lo) as an exact two-product plus the small
 // cross term, accumulated with two-sum (Dekker / Knuth) -- roughly 2^-44 relative, at the FP32 rate.
 __device__ __forceinline__ void ff_add(float& hi, float& lo, float p, float e)
