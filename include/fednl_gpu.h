@@ -265,8 +265,8 @@ int fednl_gpu_selftest_rn(int64_t n, uint64_t seed, int64_t* sqrt_mismatches, in
 
 /* Self-test of a solve whose wait for another CTA's values runs out: (I + I) dx = 1, x -= dx with every such
  * wait cut to `limit` (0: the kernels' own bounds, about a second; < 0: at once), by the FP64 cooperative solve
- * or (fp32 != 0) the FP32 one.  The launch's status (FEDNL_OK or FEDNL_ETIMEOUT) and how many entries of x
- * changed: all of them, or none. */
+ * (fp32 0), the FP32 one (1) or, d above 512, the FP32 one's grid launched without its clusters (2).  The
+ * launch's status (FEDNL_OK or FEDNL_ETIMEOUT) and how many entries of x changed: all of them, or none. */
 int fednl_gpu_selftest_lost_wait(int32_t d, int32_t fp32, int32_t limit, int32_t* status, int32_t* changed);
 
 /* Measurement of this GPU's FP64 pipe (no counterpart in the reference; the denominator of the FP64

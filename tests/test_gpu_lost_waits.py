@@ -22,6 +22,12 @@ def test_x_stays_when_a_wait_runs_out(gpu, fp32, d):
         assert gpu.selftest_lost_wait(d, fp32, 0) == (0, d)
 
 
+@pytest.mark.parametrize("d", [640, 1024])
+def test_a_grid_that_got_no_clusters_solves_without(gpu, d):
+    """As a profiler may replay it: no store into another CTA of a cluster, and no wait for one."""
+    assert gpu.selftest_lost_wait(d, 2, -1) == (0, d)
+
+
 @pytest.mark.parametrize("fp32,d", [(False, 1), (False, 31), (True, 31), (True, 301)])
 def test_solves_without_such_waits(gpu, fp32, d):
     assert gpu.selftest_lost_wait(d, fp32, -1) == (0, d)

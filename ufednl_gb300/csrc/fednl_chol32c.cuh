@@ -292,6 +292,12 @@ __device__ __forceinline__ uint32_t c32c_cluster_rank()
     asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
 }
+__device__ __forceinline__ uint32_t c32c_cluster_size()
+{
+    uint32_t n;
+    asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(n));
+    return n;
+}
 __device__ __forceinline__ void c32c_cluster_sync()
 {
     asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
@@ -939,8 +945,10 @@ __device__ __forceinline__ void chol32c_body(const Dev& P, const Chol32c& C, con
     __shared__ double s_red[2][kCoopThreads / 32];
     double en_prev = 0.0;
     // the solves run in CTA 0, or in a cluster each (in one, when the launch is one cluster); the leader
-    // has the solution at the end and keeps its sum
-    const unsigned n_cl = (unsigned)C.solve_cluster, fwd_cl = 0, bwd_cl = n_cl && G > n_cl ? 1 : 0;
+    // has the solution at the end and keeps its sum.  A launch that was to have clusters and got none (a
+    // profiler that replays it as a plain cooperative one) solves in CTA 0: a store into another CTA of a
+    // cluster that is not there faults.
+    const unsigned n_cl = c32c_cluster_size() == (uint32_t)C.solve_cluster ? C.solve_cluster : 0, fwd_cl = 0, bwd_cl = n_cl && G > n_cl ? 1 : 0;
     const unsigned my_cl = n_cl ? bid / n_cl : 0, leader = bwd_cl * n_cl;
     __shared__ __align__(8) uint64_t s_mb[2][kC32MaxBlocks];
     C32Cluster KF, KB;

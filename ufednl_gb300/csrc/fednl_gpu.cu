@@ -468,7 +468,7 @@ int fednl_device_optionb_solve32(const FednlSolveDesc& S, const FednlSolve32& E,
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
     int na = 0;
-    if (cl || ncl) {
+    if (cl || (ncl && !S.no_clusters)) {
         attr[na].id = cudaLaunchAttributeClusterDimension;
         attr[na].val.clusterDim.x = cl ? grid : ncl;
         attr[na].val.clusterDim.y = 1;
@@ -3087,6 +3087,7 @@ int fednl_gpu_selftest_lost_wait(int32_t d, int32_t fp32, int32_t limit, int32_t
     S.lptr = l;
     S.g = g;
     S.wait_limit = limit;
+    S.no_clusters = fp32 == 2;
     if (fp32) {
         k_split_pairs<<<(unsigned)((U + 255) / 256), 256, 0, s.st>>>(H, d, hh, hl, rh, rl);
         CKL();

@@ -315,8 +315,9 @@ def selftest_rn(n: int, seed: int = 1) -> tuple:
     return a.value, b.value
 
 
-def selftest_lost_wait(d: int, fp32: bool = False, limit: int = -1) -> tuple:
-    """(status, entries of x that changed) of a solve whose waits between CTAs run out after `limit`."""
+def selftest_lost_wait(d: int, fp32: int = 0, limit: int = -1) -> tuple:
+    """(status, entries of x that changed) of a solve whose waits between CTAs run out after `limit`; fp32: 1 the
+    FP32 solve, 2 the same without its clusters."""
     status, changed = C.c_int32(0), C.c_int32(0)
     _check(load().fednl_gpu_selftest_lost_wait(int(d), int(fp32), int(limit), C.byref(status), C.byref(changed)))
     return status.value, changed.value
