@@ -19,5 +19,13 @@ def oracle():
     return pyoracle
 
 
+@pytest.fixture(scope="session")
+def gpu():
+    from ufednl_gb300 import build, fednl
+    build.build()
+    fednl.load()
+    return fednl
+
+
 def golden_path(name: str) -> str:
     return os.path.join(REPO, "tests", "golden", name)

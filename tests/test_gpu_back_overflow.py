@@ -6,14 +6,6 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.fixture(scope="module")
-def gpu():
-    from ufednl_gb300 import build, fednl
-    build.build()
-    fednl.load()
-    return fednl
-
-
 @pytest.mark.parametrize("d", [3, 33, 34, 35, 36, 38, 63, 64, 66, 131, 301])
 def test_an_infinite_first_component(gpu, oracle, d):
     H = np.eye(d)

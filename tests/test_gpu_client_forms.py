@@ -9,14 +9,6 @@ from ufednl_gb300 import datagen
 pytestmark = pytest.mark.gpu
 
 
-@pytest.fixture(scope="module")
-def gpu():
-    from ufednl_gb300 import build, fednl
-    build.build()
-    fednl.load()
-    return fednl
-
-
 LARGE = [63, 64, 65, 128, 129, 200, 300]      # beside clients of few samples
 
 

@@ -9,14 +9,6 @@ from ufednl_gb300 import datagen
 pytestmark = pytest.mark.gpu
 
 
-@pytest.fixture(scope="module")
-def gpu():
-    from ufednl_gb300 import build, fednl
-    build.build()
-    fednl.load()
-    return fednl
-
-
 @pytest.mark.parametrize("d,k,comp,own_kernel", [
     (97, 194, "toplek", False), (130, 520, "topk", False), (400, 1600, "toplek", False),
     (301, 9000, "toplek", True), (301, 9000, "topk", True), (403, 8500, "toplek", True),
