@@ -265,8 +265,9 @@ int fednl_gpu_selftest_rn(int64_t n, uint64_t seed, int64_t* sqrt_mismatches, in
 
 /* Self-test of a solve whose wait for another CTA's values runs out: (I + I) dx = 1, x -= dx with every such
  * wait cut to `limit` (0: the kernels' own bounds, about a second; < 0: at once), by the FP64 cooperative solve
- * (fp32 0), the FP32 one (1) or, d above 512, the FP32 one's grid launched without its clusters (2).  The
- * launch's status (FEDNL_OK or FEDNL_ETIMEOUT) and how many entries of x changed: all of them, or none. */
+ * (fp32 0; -1: x = dx, as in FedNL-PP), the FP32 one (1) or, d above 512, the FP32 one's grid launched without
+ * its clusters (2).  The launch's status (FEDNL_OK or FEDNL_ETIMEOUT) and how many entries of x changed: all of
+ * them, or none. */
 int fednl_gpu_selftest_lost_wait(int32_t d, int32_t fp32, int32_t limit, int32_t* status, int32_t* changed);
 
 /* Measurement of this GPU's FP64 pipe (no counterpart in the reference; the denominator of the FP64
@@ -284,7 +285,7 @@ int fednl_gpu_fp64_rate(int64_t iters, double* fma_gops, double* add_gops, doubl
  *   - H (column-major d x lda, upper triangle read), g and dx are DEVICE pointers the caller owns;
  *   - the call runs on `stream` (a cudaStream_t, NULL = the default stream) and waits for that
  *     stream to finish the solve before it returns the status (FEDNL_OK, FEDNL_ENOTPD,
- *     FEDNL_ETIMEOUT);
+ *     FEDNL_ETIMEOUT, with which dx may be partly written);
  *   - its scratch is one fixed device array of the library, about 1 MB, which every device that
  *     loads the library holds until the process exits; so d is at most 512, and a larger d returns
  *     FEDNL_EINVAL with a message naming the limit;

@@ -6,16 +6,8 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.fixture(scope="module")
-def gpu():
-    from ufednl_gb300 import build, fednl
-    build.build()
-    fednl.load()
-    return fednl
-
-
-@pytest.mark.parametrize("fp32,d", [(False, 64), (False, 129), (False, 301), (False, 1024),
-                                    (True, 350), (True, 512), (True, 640), (True, 1024)])
+@pytest.mark.parametrize("fp32,d", [(0, 64), (0, 129), (0, 301), (0, 1024), (-1, 69), (-1, 301),
+                                    (1, 350), (1, 512), (1, 640), (1, 1024)])
 def test_x_stays_when_a_wait_runs_out(gpu, fp32, d):
     for _ in range(3):
         assert gpu.selftest_lost_wait(d, fp32, -1) == (-5, 0)
@@ -28,6 +20,6 @@ def test_a_grid_that_got_no_clusters_solves_without(gpu, d):
     assert gpu.selftest_lost_wait(d, 2, -1) == (0, d)
 
 
-@pytest.mark.parametrize("fp32,d", [(False, 1), (False, 31), (True, 31), (True, 301)])
+@pytest.mark.parametrize("fp32,d", [(0, 1), (0, 31), (-1, 20), (1, 31), (1, 301)])
 def test_solves_without_such_waits(gpu, fp32, d):
     assert gpu.selftest_lost_wait(d, fp32, -1) == (0, d)

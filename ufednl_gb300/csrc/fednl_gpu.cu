@@ -249,6 +249,7 @@ int fednl_solve_batch_launch(const FednlSolveDesc* descs, int n, void* stream)
             J.P.round_ctr = S.round_ctr;
             J.P.hist_cap = S.hist_cap;
             J.P.wait_limit = S.wait_limit;
+            J.P.pp = S.set_x;
             J.Hin = S.H;
             J.hin_lda = 0;
             J.lptr = S.lptr;
@@ -901,7 +902,7 @@ int launch_round(fednl_handle h, Marks* M = nullptr, bool client_phase_only = fa
         CKL();
         MARK("k_chol_coop");     // x = (H + l I)^-1 g (bin_fednl_local_pp TrainLoop.h:1560-1600)
         CK(cudaMemsetAsync(P.bar, 0, 4 * sizeof(unsigned), st));   // barrier words and error flag start at zero
-        CK(launch_chol(P, h->chol_grid, st, P.H, 0, P.stats + 1, 0.0, P.g, P.x, nullptr, 0));
+        CK(launch_chol(P, h->chol_grid, st, P.H, 0, P.stats + 1, 0.0, P.g, nullptr, P.x, 0));
         if (pfork) CK(cudaStreamWaitEvent(st, h->join_ev, 0));
         MARK("end");
         return FEDNL_OK;
@@ -3088,7 +3089,8 @@ int fednl_gpu_selftest_lost_wait(int32_t d, int32_t fp32, int32_t limit, int32_t
     S.g = g;
     S.wait_limit = limit;
     S.no_clusters = fp32 == 2;
-    if (fp32) {
+    S.set_x = fp32 < 0;
+    if (fp32 > 0) {
         k_split_pairs<<<(unsigned)((U + 255) / 256), 256, 0, s.st>>>(H, d, hh, hl, rh, rl);
         CKL();
         E.hh = hh;

@@ -2694,7 +2694,7 @@ __device__ __forceinline__ void chol_body(const Dev& P, const double* __restrict
                 for (int i = tid; i < d; i += kCoopThreads) {
                     double y;
                     asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=d"(y) : "l"(P.ybuf + i));
-                    xupd[i] = __dsub_rn(xupd[i], y);
+                    xupd[i] = P.pp ? y : __dsub_rn(xupd[i], y);      // FedNL-PP: x = dx
                 }
         }
         if (record && norm_here) {   // ||g|| for the round statistics, in a CTA without rows if there is one

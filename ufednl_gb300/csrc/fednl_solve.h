@@ -33,6 +33,7 @@ struct FednlSolveDesc {
     int record;
     int wait_limit;        // polls (FP64) or cycles (FP32) after which a wait inside the solve runs out;
                            // 0: the kernels' own bounds (about a second), < 0: at once (the self-test)
+    int set_x;             // 1: x = dx instead of x -= dx (FP64)
     int no_clusters;       // 1: the FP32 solve's grid is launched without its clusters (the self-test)
 };
 

@@ -316,8 +316,8 @@ def selftest_rn(n: int, seed: int = 1) -> tuple:
 
 
 def selftest_lost_wait(d: int, fp32: int = 0, limit: int = -1) -> tuple:
-    """(status, entries of x that changed) of a solve whose waits between CTAs run out after `limit`; fp32: 1 the
-    FP32 solve, 2 the same without its clusters."""
+    """(status, entries of x that changed) of a solve whose waits between CTAs run out after `limit`; fp32: 0 the
+    FP64 solve, -1 the same with x = dx, 1 the FP32 solve, 2 the same without its clusters."""
     status, changed = C.c_int32(0), C.c_int32(0)
     _check(load().fednl_gpu_selftest_lost_wait(int(d), int(fp32), int(limit), C.byref(status), C.byref(changed)))
     return status.value, changed.value
