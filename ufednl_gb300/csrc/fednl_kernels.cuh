@@ -847,8 +847,9 @@ __global__ void k_h_init(Dev P)
 // client, the launch as long as its slowest client.  Cycles of that client (w8a-like, d = 301, k = 2408):
 // first rounds 855 k, of which extraction 510 k, to 440 k (2387 extractions at 208 -> 100 cycles, windows
 // beside them); settled rounds 580 k to 377 k (713 replacements at 650 -> 440 cycles with their
-// searches, 1387 rows without an entry above the root at 37 -> 2).  k_select 376 -> 207 us; a9a-like
-// (d = 124, k = 992) 139 -> 95 us, dense d = 512, k = 4096 239 -> 137 us, reference order at w8a 696 -> 299.
+// searches, 1387 rows without an entry above the root at 37 -> 2).  k_select 376 -> 209 us; a9a-like
+// (d = 124, k = 992) 139 -> 97 us, dense d = 512, k = 4096 239 -> 141 us, reference order at w8a 696 -> 299
+// (2 % of each for the meetings of the scanning warp's lanes, see heap_descend).
 __device__ __forceinline__ unsigned long long abs_bits(double v)
 {
     return (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
