@@ -948,7 +948,8 @@ __device__ __forceinline__ void chol32c_body(const Dev& P, const Chol32c& C, con
     // has the solution at the end and keeps its sum.  A launch that was to have clusters and got none (a
     // profiler that replays it as a plain cooperative one) solves in CTA 0: a store into another CTA of a
     // cluster that is not there faults.
-    const unsigned n_cl = c32c_cluster_size() == (uint32_t)C.solve_cluster ? C.solve_cluster : 0, fwd_cl = 0, bwd_cl = n_cl && G > n_cl ? 1 : 0;
+    const unsigned n_cl = c32c_cluster_size() == (uint32_t)C.solve_cluster ? C.solve_cluster : 0;
+    const unsigned fwd_cl = 0, bwd_cl = n_cl && G > n_cl ? 1 : 0;
     const unsigned my_cl = n_cl ? bid / n_cl : 0, leader = bwd_cl * n_cl;
     __shared__ __align__(8) uint64_t s_mb[2][kC32MaxBlocks];
     C32Cluster KF, KB;

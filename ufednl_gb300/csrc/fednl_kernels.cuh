@@ -76,7 +76,8 @@ struct Dev {
     int* status;            // [1]
     double* stats;          // [2] ||g||, l
     int hist_cap;
-    int wait_limit;         // polls after which a solve's wait for another CTA's value runs out; 0: the built-in bound, < 0: at once
+    int wait_limit;         // polls after which the solve's wait for another CTA's value runs out (0: kBackSpins,
+                            // < 0: at once)
     unsigned* bar;          // [4] grid barrier: arrival count with error flag, finished CTAs (two spare)
     // FedNL-PP (bin_fednl_local_pp); act == nullptr: every client takes part (plain FedNL)
     int pp, n_act;          // n_act: clients processed this round (tau, or nc without PP)
